@@ -201,11 +201,10 @@ __global__ void __launch_bounds__(256) k_linear(uint32_t n, const float* __restr
     }
 }
 
-// dX (n x K) [+]= dY (n x NO) W (NO x K)
+// dX (n x K) += dY (n x NO) W (NO x K)
 template <int K, int NO>
 __global__ void __launch_bounds__(256) k_linear_bwd_data(uint32_t n, const float* __restrict__ dY,
-                                                         const __nv_bfloat16* __restrict__ W, float* __restrict__ dX,
-                                                         int accumulate)
+                                                         const __nv_bfloat16* __restrict__ W, float* __restrict__ dX)
 {
     constexpr int ROWS = kBwdRows, TPR = 256 / ROWS, CPT = K / TPR;
     __shared__ float Ws[NO][K + 1];
@@ -238,7 +237,7 @@ __global__ void __launch_bounds__(256) k_linear_bwd_data(uint32_t n, const float
         for (int c = 0; c < CPT; ++c)
         {
             const size_t idx = (size_t)(r0 + r) * K + cg + c * TPR;
-            dX[idx] = accumulate ? dX[idx] + acc[c] : acc[c];
+            dX[idx] += acc[c];
         }
 }
 
@@ -297,16 +296,39 @@ __global__ void __launch_bounds__(256) k_linear_bwd_weight(uint32_t n, uint32_t 
     if (threadIdx.x < NO) out[PAIRS + threadIdx.x] = bacc;
 }
 
-// out[j] (+)= sum over b of partial[b * stride + j], in block order
-__global__ void k_reduce_partials(uint32_t nblocks, uint32_t stride, uint32_t count, const float* __restrict__ partial,
-                                  float* __restrict__ out, int accumulate)
+// out[j] = sum over b of partial[b * stride + j].  32 columns a CTA, one warp
+// per residue of b: a load is a 128-byte line, 32 chains run side by side, and
+// the residues are added in their own order, so the sum depends on nothing but
+// nblocks.  (One thread a column walked all the partials in one chain of
+// dependent adds behind L2 loads: 9.2 ms of the 16.7 ms device time of a 512^2
+// step, with one partial for every 8 nodes.)
+constexpr int kReduceWarps = 32;
+
+__global__ void __launch_bounds__(32 * kReduceWarps) k_reduce_partials(uint32_t nblocks, uint32_t stride, uint32_t count,
+                                                                       const float* __restrict__ partial,
+                                                                       float* __restrict__ out)
 {
-    for (uint32_t j = blockIdx.x * blockDim.x + threadIdx.x; j < count; j += gridDim.x * blockDim.x)
+    __shared__ float sums[kReduceWarps][33];
+    const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5, j = blockIdx.x * 32u + lane;
+    float s = 0.f;
+    if (j < count)
+#pragma unroll 4
+        for (uint32_t b = warp; b < nblocks; b += kReduceWarps) s += partial[(size_t)b * stride + j];
+    sums[warp][lane] = s;
+    __syncthreads();
+    if (warp == 0 && j < count)
     {
-        float s = 0.f;
-        for (uint32_t b = 0; b < nblocks; ++b) s += partial[(size_t)b * stride + j];
-        out[j] = accumulate ? out[j] + s : s;
+        float t = 0.f;
+#pragma unroll
+        for (int w = 0; w < kReduceWarps; ++w) t += sums[w][lane];
+        out[j] = t;
     }
+}
+
+static void reduce_partials(b2s_ctx* ctx, uint32_t nblocks, uint32_t stride, uint32_t count, const float* partial,
+                            float* out)
+{
+    B2S_LAUNCH(ctx, k_reduce_partials, (count + 31) / 32, 32 * kReduceWarps, 0, nblocks, stride, count, partial, out);
 }
 
 // ------------------------------------------------------------ message passing
@@ -376,67 +398,111 @@ __global__ void __launch_bounds__(256) k_aggregate(uint32_t n, const uint32_t* _
 }
 
 // backward of k_aggregate for one layer.
-//   dpre = dHout * (pre > 0);  dHin = dHout (residual, written here);
+//   dpre = dHout * (pre > 0);  (the residual part of dHin is dHout itself)
 //   dSM[:, :64] = dpre;  dSM[j, 64:] = sum_{i in N(j)} invdeg_i g_ij dpre_i
 //   per-CTA partials of dW_g (64x4), db_g (64), db (64)
-__global__ void __launch_bounds__(256) k_aggregate_bwd(uint32_t n, const uint32_t* __restrict__ rp,
-                                                       const uint32_t* __restrict__ ci, const uint32_t* __restrict__ rev,
-                                                       const float* __restrict__ EF, const float* __restrict__ invdeg,
-                                                       const float* __restrict__ SM, const __nv_bfloat16* __restrict__ Wl,
-                                                       const float* __restrict__ pre, const float* __restrict__ dHout,
-                                                       float* __restrict__ dSM, float* __restrict__ dHin,
-                                                       float* __restrict__ partial)
+// One warp per node as in the forward kernel, grid-stride: a lane keeps its two
+// channels' gate gradients in registers over all its nodes, so a CTA writes one
+// 1.5 KB partial at its end instead of one for every 8 nodes, and a batch of
+// edges has all its gathers in flight before the gates are formed.  Bound by
+// the gathers' latency and the sigmoids (two an edge and channel): 512^2 in
+// 0.565 ms before (a node a warp and CTA lifetime, the partials summed in
+// shared memory).
+constexpr int kEdgeBatch = 4;
+
+__global__ void __launch_bounds__(256, 2) k_aggregate_bwd(uint32_t n, const uint32_t* __restrict__ rp,
+                                                          const uint32_t* __restrict__ ci,
+                                                          const uint32_t* __restrict__ rev,
+                                                          const float* __restrict__ EF,
+                                                          const float* __restrict__ invdeg,
+                                                          const float* __restrict__ SM,
+                                                          const __nv_bfloat16* __restrict__ Wl,
+                                                          const float* __restrict__ pre,
+                                                          const float* __restrict__ dHout, float* __restrict__ dSM,
+                                                          float* __restrict__ partial)
 {
-    __shared__ float wg[H][FE], bg[H];
     __shared__ float pw[8][H][FE + 2];  // per warp: dW_g (4), db_g, db
-    for (int t = threadIdx.x; t < H * FE; t += blockDim.x) wg[t / FE][t % FE] = __bfloat162float(Wl[L_WG + t]);
-    for (int t = threadIdx.x; t < H; t += blockDim.x) bg[t] = __bfloat162float(Wl[L_BG + t]);
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    for (int t = lane; t < H * (FE + 2); t += 32) pw[warp][t / (FE + 2)][t % (FE + 2)] = 0.f;
-    __syncthreads();
-    const uint32_t j = blockIdx.x * 8 + warp;
-    if (j < n)
+    float wg[2][FE], bg[2], acc[2][FE + 2];
+#pragma unroll
+    for (int h = 0; h < 2; ++h)
     {
+        const int c = lane + 32 * h;
+#pragma unroll
+        for (int f = 0; f < FE; ++f) wg[h][f] = __bfloat162float(Wl[L_WG + c * FE + f]);
+        bg[h] = __bfloat162float(Wl[L_BG + c]);
+#pragma unroll
+        for (int f = 0; f < FE + 2; ++f) acc[h][f] = 0.f;
+    }
+    auto gate = [&](int h, const float4& e) {
+        return sigm(bg[h] + wg[h][0] * e.x + wg[h][1] * e.y + wg[h][2] * e.z + wg[h][3] * e.w);
+    };
+    for (uint32_t j = blockIdx.x * 8 + warp; j < n; j += gridDim.x * 8)
+    {
+        float dp[2], dpj[2], dm[2] = {0.f, 0.f};
+        const float idj = invdeg[j];
+#pragma unroll
         for (int h = 0; h < 2; ++h)
         {
-            const int c = lane + 32 * h;
-            const float dp = pre[(size_t)j * H + c] > 0.f ? dHout[(size_t)j * H + c] : 0.f;
-            dSM[(size_t)j * 2 * H + c] = dp;
-            dHin[(size_t)j * H + c] = dHout[(size_t)j * H + c];
-            pw[warp][c][FE + 1] += dp;
-            // gather over neighbours i of j: edge (i, j) at rev[p] in row i
-            float dm = 0.f;
-            for (uint32_t p = rp[j]; p < rp[j + 1]; ++p)
+            const size_t o = (size_t)j * H + lane + 32 * h;
+            dp[h] = pre[o] > 0.f ? dHout[o] : 0.f;
+            dpj[h] = dp[h] * idj;
+            acc[h][FE + 1] += dp[h];
+        }
+        const uint32_t pa = rp[j], pe = rp[j + 1];
+        for (uint32_t pb = pa; pb < pe; pb += kEdgeBatch)
+        {
+            uint32_t ii[kEdgeBatch];
+            float4 eo[kEdgeBatch], ei[kEdgeBatch];  // features of (j, i) and of (i, j), listed in row i at rev[p]
+            float di[kEdgeBatch][2], mi[kEdgeBatch][2], idi[kEdgeBatch];
+#pragma unroll
+            for (int k = 0; k < kEdgeBatch; ++k) ii[k] = pb + k < pe ? ci[pb + k] : j;
+#pragma unroll
+            for (int k = 0; k < kEdgeBatch; ++k)
             {
-                const uint32_t i = ci[p];
-                if (i == j) continue;
-                const uint32_t q = rev[p];
-                const float* e = EF + (size_t)q * FE;
-                const float z = bg[c] + wg[c][0] * e[0] + wg[c][1] * e[1] + wg[c][2] * e[2] + wg[c][3] * e[3];
-                const float g = sigm(z);
-                const float dpi = pre[(size_t)i * H + c] > 0.f ? dHout[(size_t)i * H + c] : 0.f;
-                const float w = invdeg[i] * dpi;
-                dm += w * g;
+                const bool on = ii[k] != j;
+                const uint32_t q = on ? rev[pb + k] : 0u, i = on ? ii[k] : j;
+                const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+                eo[k] = on ? *reinterpret_cast<const float4*>(EF + (size_t)(pb + k) * FE) : zero;
+                ei[k] = on ? *reinterpret_cast<const float4*>(EF + (size_t)q * FE) : zero;
+                idi[k] = invdeg[i];
+#pragma unroll
+                for (int h = 0; h < 2; ++h)
+                {
+                    const size_t o = (size_t)i * H + lane + 32 * h;
+                    di[k][h] = pre[o] > 0.f ? dHout[o] : 0.f;
+                    mi[k][h] = SM[(size_t)i * 2 * H + H + lane + 32 * h];
+                }
             }
-            dSM[(size_t)j * 2 * H + H + c] = dm;
-            // gate gradient for the edges (j, k) of row j (owned by node j)
-            const float dpj = dp * invdeg[j];
-            for (uint32_t p = rp[j]; p < rp[j + 1]; ++p)
+#pragma unroll
+            for (int k = 0; k < kEdgeBatch; ++k)
             {
-                const uint32_t k = ci[p];
-                if (k == j) continue;
-                const float* e = EF + (size_t)p * FE;
-                const float z = bg[c] + wg[c][0] * e[0] + wg[c][1] * e[1] + wg[c][2] * e[2] + wg[c][3] * e[3];
-                const float g = sigm(z);
-                const float dz = dpj * SM[(size_t)k * 2 * H + H + c] * g * (1.f - g);
-                pw[warp][c][0] += dz * e[0];
-                pw[warp][c][1] += dz * e[1];
-                pw[warp][c][2] += dz * e[2];
-                pw[warp][c][3] += dz * e[3];
-                pw[warp][c][FE] += dz;
+                if (ii[k] == j) continue;  // the diagonal, or past the row's end: the whole warp
+#pragma unroll
+                for (int h = 0; h < 2; ++h)
+                {
+                    dm[h] += idi[k] * di[k][h] * gate(h, ei[k]);
+                    const float g = gate(h, eo[k]);
+                    const float dz = dpj[h] * mi[k][h] * g * (1.f - g);
+                    acc[h][0] += dz * eo[k].x;
+                    acc[h][1] += dz * eo[k].y;
+                    acc[h][2] += dz * eo[k].z;
+                    acc[h][3] += dz * eo[k].w;
+                    acc[h][FE] += dz;
+                }
             }
         }
+#pragma unroll
+        for (int h = 0; h < 2; ++h)
+        {
+            dSM[(size_t)j * 2 * H + lane + 32 * h] = dp[h];
+            dSM[(size_t)j * 2 * H + H + lane + 32 * h] = dm[h];
+        }
     }
+#pragma unroll
+    for (int h = 0; h < 2; ++h)
+#pragma unroll
+        for (int f = 0; f < FE + 2; ++f) pw[warp][lane + 32 * h][f] = acc[h][f];
     __syncthreads();
     // fixed-order sum over the 8 warps, then one partial per CTA
     float* out = partial + (size_t)blockIdx.x * (H * (FE + 2));
@@ -546,7 +612,9 @@ __global__ void k_head_dc(uint32_t nnz, const double* __restrict__ dL, const dou
 }
 
 // head backward: dH_i += sum_row dc_q u (+ dc_ii d) ; dH_j += sum_{col j} dc_q v ;
-// per-CTA partials of du, dv, dw, dbo, dd, dbd
+// per-CTA partials of du, dv, dw, dbo, dd, dbd.  A warp per node, grid-stride,
+// the parameter gradients in registers until the end (as k_aggregate_bwd; one
+// partial for every 8 nodes before: 0.214 ms on 512^2).
 __global__ void __launch_bounds__(256) k_head_bwd(uint32_t n, const uint32_t* __restrict__ Lrp,
                                                   const uint32_t* __restrict__ Lci, const uint32_t* __restrict__ Trp,
                                                   const uint32_t* __restrict__ Tpos, const uint32_t* __restrict__ Arp,
@@ -556,39 +624,70 @@ __global__ void __launch_bounds__(256) k_head_bwd(uint32_t n, const uint32_t* __
 {
     __shared__ float pw[8][O_SIZE];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    for (int t = lane; t < O_SIZE; t += 32) pw[warp][t] = 0.f;
-    __syncwarp();
-    const uint32_t i = blockIdx.x * 8 + warp;
-    if (i < n)
+    float pu[2], pv[2], pd[2], du[2] = {0.f, 0.f}, dv[2] = {0.f, 0.f}, dd[2] = {0.f, 0.f};
+    float dw = 0.f, dbo = 0.f, dbd = 0.f;  // dw: lane c < FE; dbo, dbd: the same in every lane
+#pragma unroll
+    for (int h = 0; h < 2; ++h)
     {
-        for (int h = 0; h < 2; ++h)
+        pu[h] = Pf[OFF_OUT + O_U + lane + 32 * h];
+        pv[h] = Pf[OFF_OUT + O_V + lane + 32 * h];
+        pd[h] = Pf[OFF_OUT + O_D + lane + 32 * h];
+    }
+    for (uint32_t i = blockIdx.x * 8 + warp; i < n; i += gridDim.x * 8)
+    {
+        float dh[2] = {0.f, 0.f}, hi[2];
+#pragma unroll
+        for (int h = 0; h < 2; ++h) hi[h] = Hf[(size_t)i * H + lane + 32 * h];
+        const uint32_t qa = Lrp[i], qe = Lrp[i + 1], ea = Arp[i];
+        for (uint32_t q = qa; q < qe; ++q)
         {
-            const int c = lane + 32 * h;
-            float dh = 0.f;
-            const float hic = Hf[(size_t)i * H + c];
-            for (uint32_t q = Lrp[i]; q < Lrp[i + 1]; ++q)
+            const uint32_t j = Lci[q];
+            const float d = dC[q];
+            if (j == i)
             {
-                const uint32_t j = Lci[q];
-                const float d = dC[q];
-                if (j == i)
+#pragma unroll
+                for (int h = 0; h < 2; ++h)
                 {
-                    dh += d * Pf[OFF_OUT + O_D + c];
-                    pw[warp][O_D + c] += d * hic;
-                    if (c == 0) pw[warp][O_BD] += d;
+                    dh[h] += d * pd[h];
+                    dd[h] += d * hi[h];
                 }
-                else
-                {
-                    dh += d * Pf[OFF_OUT + O_U + c];
-                    pw[warp][O_U + c] += d * hic;
-                    pw[warp][O_V + c] += d * Hf[(size_t)j * H + c];
-                    if (c < FE) pw[warp][O_W + c] += d * EF[(size_t)(Arp[i] + (q - Lrp[i])) * FE + c];
-                    if (c == 0) pw[warp][O_BO] += d;
-                }
+                dbd += d;
             }
-            // column part: entries (k, i) with k > i, listed in row i of L^T
-            for (uint32_t t = Trp[i]; t < Trp[i + 1]; ++t) dh += dC[Tpos[t]] * Pf[OFF_OUT + O_V + c];
-            dH[(size_t)i * H + c] = dh;
+            else
+            {
+#pragma unroll
+                for (int h = 0; h < 2; ++h)
+                {
+                    dh[h] += d * pu[h];
+                    du[h] += d * hi[h];
+                    dv[h] += d * Hf[(size_t)j * H + lane + 32 * h];
+                }
+                if (lane < FE) dw += d * EF[(size_t)(ea + (q - qa)) * FE + lane];
+                dbo += d;
+            }
         }
+        // column part: entries (k, i) with k > i, listed in row i of L^T
+        for (uint32_t t = Trp[i]; t < Trp[i + 1]; ++t)
+        {
+            const float d = dC[Tpos[t]];
+            dh[0] += d * pv[0];
+            dh[1] += d * pv[1];
+        }
+        dH[(size_t)i * H + lane] = dh[0];
+        dH[(size_t)i * H + lane + 32] = dh[1];
+    }
+#pragma unroll
+    for (int h = 0; h < 2; ++h)
+    {
+        pw[warp][O_U + lane + 32 * h] = du[h];
+        pw[warp][O_V + lane + 32 * h] = dv[h];
+        pw[warp][O_D + lane + 32 * h] = dd[h];
+    }
+    if (lane < FE) pw[warp][O_W + lane] = dw;
+    if (lane == 0)
+    {
+        pw[warp][O_BO] = dbo;
+        pw[warp][O_BD] = dbd;
     }
     __syncthreads();
     float* out = partial + (size_t)blockIdx.x * O_SIZE;
@@ -1334,13 +1433,15 @@ static void train_step(b2s_ctx* ctx, Gnn& net, const CsrDev& A, int nprobes, uin
     B2S_LAUNCH(ctx, k_head_dc, stream_grid(ctx, Lnnz), kThreads, 0, Lnnz, dL.p, Lv.p, L0.p, C.p, dC.p);
 
     // backward
-    const unsigned gw = (n + 7) / 8, g64 = (n + kBwdRows - 1) / kBwdRows;
+    const unsigned g64 = (n + kBwdRows - 1) / kBwdRows;
+    // node kernels: grid-stride, at most 4 CTAs an SM (one partial of the parameter gradients each)
+    const unsigned gw = std::min<unsigned>((n + 7) / 8, (unsigned)ctx->sm_count * 4);
     B2S_CUDA(cudaMemsetAsync(net.g.p, 0, net.g.bytes(), ctx->stream));
-    DBuf<float> dH(n * (size_t)H), dH2(n * (size_t)H), dSM(n * (size_t)2 * H), part;
+    DBuf<float> dH(n * (size_t)H), dSM(n * (size_t)2 * H), part;
     part.alloc((size_t)std::max<unsigned>(gw, 1) * (H * (FE + 2) > O_SIZE ? H * (FE + 2) : O_SIZE) + 16);
     B2S_LAUNCH(ctx, k_head_bwd, gw, 256, 0, n, Lrp.p, Lci.p, Trp.p, Tpos.p, A.rp.p, G.EF.p, G.Hs[NL].p, net.pr.p,
                dC.p, dH.p, part.p);
-    B2S_LAUNCH(ctx, k_reduce_partials, 1, 256, 0, gw, (uint32_t)O_SIZE, (uint32_t)O_SIZE, part.p, net.g.p + OFF_OUT, 0);
+    reduce_partials(ctx, gw, O_SIZE, O_SIZE, part.p, net.g.p + OFF_OUT);
     const uint32_t rows_per = 2048;
     const unsigned gwb = (n + rows_per - 1) / rows_per;
     DBuf<float> wpart((size_t)gwb * (2 * H * H + 2 * H) + 16), red(H * (FE + 2));
@@ -1348,26 +1449,22 @@ static void train_step(b2s_ctx* ctx, Gnn& net, const CsrDev& A, int nprobes, uin
     {
         const __nv_bfloat16* Wl = net.pb.p + LAYER0 + l * L_SIZE;
         float* gl = net.g.p + LAYER0 + l * L_SIZE;
-        // dH (wrt H_{l+1}) -> dpre, dSM, residual into dH2
+        // dH (wrt H_{l+1}) -> dpre, dSM
         B2S_LAUNCH(ctx, k_aggregate_bwd, gw, 256, 0, n, A.rp.p, A.ci.p, G.rev.p, G.EF.p, G.invdeg.p, G.SM[l].p, Wl,
-                   G.pre[l].p, dH.p, dSM.p, dH2.p, part.p);
+                   G.pre[l].p, dH.p, dSM.p, part.p);
         // per-CTA gate partials -> ordered sum -> layer layout
-        B2S_LAUNCH(ctx, k_reduce_partials, 2, 256, 0, gw, (uint32_t)(H * (FE + 2)), (uint32_t)(H * (FE + 2)), part.p,
-                   red.p, 0);
+        reduce_partials(ctx, gw, H * (FE + 2), H * (FE + 2), part.p, red.p);
         B2S_LAUNCH(ctx, k_gate_grads, 1, 64, 0, red.p, gl);
-        // weights [W_s; W_m] (128 x 64): dW = dSM^T H_l ; dH_l += dSM W
+        // weights [W_s; W_m] (128 x 64): dW = dSM^T H_l ; dH_l = dH_{l+1} (the residual) + dSM W
         B2S_LAUNCH(ctx, (k_linear_bwd_weight<H, 2 * H, true>), gwb, 256, 0, n, rows_per, dSM.p, G.Hs[l].p, wpart.p);
-        B2S_LAUNCH(ctx, k_reduce_partials, 64, 256, 0, gwb, (uint32_t)(2 * H * H + 2 * H), (uint32_t)(2 * H * H),
-                   wpart.p, gl + L_WS, 0);
-        B2S_LAUNCH(ctx, (k_linear_bwd_data<H, 2 * H>), g64, 256, 0, n, dSM.p, Wl + L_WS, dH2.p, 1);
-        std::swap(dH, dH2);
+        reduce_partials(ctx, gwb, 2 * H * H + 2 * H, 2 * H * H, wpart.p, gl + L_WS);
+        B2S_LAUNCH(ctx, (k_linear_bwd_data<H, 2 * H>), g64, 256, 0, n, dSM.p, Wl + L_WS, dH.p);
     }
     // input layer: dpre0 = dH0 * (pre0 > 0) ; dW_in = dpre0^T F ; db_in
     B2S_LAUNCH(ctx, k_relu_mask, stream_grid(ctx, (uint64_t)n * H), kThreads, 0, (uint64_t)n * H, G.pre0.p, dH.p,
                dSM.p);
     B2S_LAUNCH(ctx, (k_linear_bwd_weight<FIN, H, false>), gwb, 256, 0, n, rows_per, dSM.p, G.F.p, wpart.p);
-    B2S_LAUNCH(ctx, k_reduce_partials, 4, 256, 0, gwb, (uint32_t)(H * FIN + H), (uint32_t)(H * FIN + H), wpart.p,
-               net.g.p + OFF_WIN, 0);
+    reduce_partials(ctx, gwb, H * FIN + H, H * FIN + H, wpart.p, net.g.p + OFF_WIN);
 
     double lossv = 0;
     d2h(ctx, &lossv, T.scal.p + 3, sizeof(double));
