@@ -8,11 +8,11 @@
 // multiplication by inv(U_KK), update of row I's U blocks, Gauss-Jordan
 // inverse of the diagonal block) -- bit-equal factors.
 // Apply: block forward substitution and block back substitution times the
-// cached inverse, in FP64 or FP32: chunked (default, trsv_chunk.cuh), per
-// level or sync-free.
+// cached inverse, in FP64 or FP32: chunked (trsv_chunk.cuh) or in level order
+// (trsv_wave.cuh), by wave_pays, or level by level.
 #include "block_ops.cuh"
 #include "trisolve.cuh"
-#include "trsv_chunk.cuh"
+#include "trsv_wave.cuh"
 
 #include <exception>
 #include <thread>
@@ -173,11 +173,6 @@ struct BTrsvOp
     const RT* rhs;
     XT* x;
     double* out64;
-    __device__ bool ready(uint32_t row, const uint32_t* flags, uint32_t epoch) const
-    {
-        return deps_ready<LOWER>(row, rp, ci, flags, epoch);
-    }
-    template <bool SYNCFREE>
     __device__ __forceinline__ void row_compute(uint32_t I) const
     {
         constexpr int BV = BS * BS;
@@ -190,7 +185,7 @@ struct BTrsvOp
             if (LOWER ? !(J < I) : !(J > I)) continue;
             XT xJ[BS];
 #pragma unroll
-            for (int c = 0; c < BS; ++c) xJ[c] = SYNCFREE ? __ldcg(&x[(size_t)J * BS + c]) : x[(size_t)J * BS + c];
+            for (int c = 0; c < BS; ++c) xJ[c] = x[(size_t)J * BS + c];
 #pragma unroll
             for (int r = 0; r < BS; ++r)
             {
@@ -222,7 +217,6 @@ struct BTrsvOp
             }
         }
     }
-    __device__ void compute(uint32_t row) const { row_compute<true>(row); }
 };
 
 __global__ void k_to32(const double* __restrict__ a, float* __restrict__ b, uint64_t n)
@@ -242,43 +236,58 @@ struct PcBILU0 final : PcImpl
     DBuf<double> inv, y;
     DBuf<float> inv32, y32, z32;
     LevelSchedule sl, su;
-    SyncFree sfl, sfu;
+    WaveSchedule wl, wu;
     ChunkSchedule csl, csu;
-    bool chunks = false;
+    bool chunk_l = false, chunk_u = false;  // the triangle takes the chunked schedule
 
     template <int BS>
     void apply_t(b2s_ctx* ctx, const double* r, double* z, const int* done)
     {
-        if (chunks)
+        if (mode == B2S_TRSV_LEVEL)
         {
             if (!fp32)
             {
-                csl.run_block<true, BS, double, double, double>(ctx, L.v.p, nullptr, r, y.p, nullptr, done);
-                csu.run_block<false, BS, double, double, double>(ctx, U.v.p, inv.p, y.p, z, nullptr, done);
+                run_levels(ctx, sl, BTrsvOp<BS, true, double, double, double>{L.rp.p, L.ci.p, L.v.p, nullptr, r, y.p, nullptr},
+                           done);
+                run_levels(ctx, su, BTrsvOp<BS, false, double, double, double>{U.rp.p, U.ci.p, U.v.p, inv.p, y.p, z, nullptr},
+                           done);
             }
             else
             {
-                csl.run_block<true, BS, float, float, double>(ctx, L.v32.p, nullptr, r, y32.p, nullptr, done);
-                csu.run_block<false, BS, float, float, float>(ctx, U.v32.p, inv32.p, y32.p, z32.p, z, done);
+                run_levels(ctx, sl,
+                           BTrsvOp<BS, true, float, float, double>{L.rp.p, L.ci.p, L.v32.p, nullptr, r, y32.p, nullptr}, done);
+                run_levels(ctx, su,
+                           BTrsvOp<BS, false, float, float, float>{U.rp.p, U.ci.p, U.v32.p, inv32.p, y32.p, z32.p, z}, done);
             }
             return;
         }
         if (!fp32)
         {
-            run_schedule(ctx, mode, sl, sfl,
-                         BTrsvOp<BS, true, double, double, double>{L.rp.p, L.ci.p, L.v.p, nullptr, r, y.p, nullptr}, done);
-            run_schedule(ctx, mode, su, sfu,
-                         BTrsvOp<BS, false, double, double, double>{U.rp.p, U.ci.p, U.v.p, inv.p, y.p, z, nullptr}, done);
+            lower<BS, double>(ctx, L.v.p, r, y.p, done);
+            upper<BS, double>(ctx, U.v.p, inv.p, y.p, z, (double*)nullptr, done);
         }
         else
         {
-            run_schedule(ctx, mode, sl, sfl,
-                         BTrsvOp<BS, true, float, float, double>{L.rp.p, L.ci.p, L.v32.p, nullptr, r, y32.p, nullptr},
-                         done);
-            run_schedule(ctx, mode, su, sfu,
-                         BTrsvOp<BS, false, float, float, float>{U.rp.p, U.ci.p, U.v32.p, inv32.p, y32.p, z32.p, z},
-                         done);
+            lower<BS, float>(ctx, L.v32.p, r, y32.p, done);
+            upper<BS, float>(ctx, U.v32.p, inv32.p, y32.p, z32.p, z, done);
         }
+    }
+
+    template <int BS, typename T>
+    void lower(b2s_ctx* ctx, const T* v, const double* r, T* x, const int* done)
+    {
+        if (chunk_l)
+            csl.run_block<true, BS, T, T, double>(ctx, v, (const T*)nullptr, r, x, nullptr, done);
+        else
+            wl.run<BS, true, WaveDiag::BlockUnit>(ctx, L.rp.p, L.ci.p, v, (const T*)nullptr, r, x, nullptr, done);
+    }
+    template <int BS, typename T>
+    void upper(b2s_ctx* ctx, const T* v, const T* d, const T* r, T* x, double* out64, const int* done)
+    {
+        if (chunk_u)
+            csu.run_block<false, BS, T, T, T>(ctx, v, d, r, x, out64, done);
+        else
+            wu.run<BS, false, WaveDiag::BlockInverse>(ctx, U.rp.p, U.ci.p, v, d, r, x, out64, done);
     }
 
     void apply(b2s_ctx* ctx, const double* r, double* z, const int* done) override
@@ -391,13 +400,13 @@ std::unique_ptr<PcImpl> make_pc_bilu0(b2s_ctx* ctx, const BaijDev& A, const b2s_
             plan_parallel(2, 2, [&](uint32_t side, unsigned) {
                 if (side == 0)
                 {
-                    if (chunked)
+                    if (chunked && !wave_pays(llev, lrp.data(), lci.data(), true))
                         lplan = plan_chunks(nb, lrp.data(), lci.data(), true, 0, vs, vs, 8, kChunkSmemBudget,
                                             (uint32_t)bs, &llev);
                     return;
                 }
                 compute_levels(nb, urp.data(), uci.data(), false, ulev);
-                if (chunked)
+                if (chunked && !wave_pays(ulev, urp.data(), uci.data(), false))
                     uplan = plan_chunks(nb, urp.data(), uci.data(), false, (uint32_t)bv, vs, vs, 8, kChunkSmemBudget,
                                         (uint32_t)bs, &ulev);
             });
@@ -429,13 +438,16 @@ std::unique_ptr<PcImpl> make_pc_bilu0(b2s_ctx* ctx, const BaijDev& A, const b2s_
         fail(B2S_SINGULAR_BLOCK, "Block-ILU(0) breakdown: diagonal block " + std::to_string(h[1]) + " is singular");
     th.join();
     if (perr) std::rethrow_exception(perr);
-    if (chunked) pc->chunks = pc->csl.load(ctx, lplan, vs) && pc->csu.load(ctx, uplan, vs);
-    if (!pc->chunks)
+    pc->chunk_l = chunked && pc->csl.load(ctx, lplan, vs);
+    pc->chunk_u = chunked && pc->csu.load(ctx, uplan, vs);
+    if (pc->mode == B2S_TRSV_LEVEL)
     {
-        if (pc->mode == B2S_TRSV_CHUNK) pc->mode = B2S_TRSV_SYNCFREE;
         if (nb) pc->su.build_host(ctx, ulev);
-        pc->sfl.init(ctx, nb);
-        pc->sfu.init(ctx, nb);
+    }
+    else
+    {
+        if (!pc->chunk_l) pc->wl.build(ctx, llev, lrp.data(), (uint32_t)bs);
+        if (!pc->chunk_u) pc->wu.build(ctx, ulev, urp.data(), (uint32_t)bs);
     }
     pc->y.alloc((size_t)nb * bs + 1);
     if (pc->fp32)
@@ -450,18 +462,19 @@ std::unique_ptr<PcImpl> make_pc_bilu0(b2s_ctx* ctx, const BaijDev& A, const b2s_
         pc->y32.alloc((size_t)nb * bs + 1);
         pc->z32.alloc((size_t)nb * bs + 1);
     }
-    if (pc->chunks)
+    if (pc->chunk_l)
     {
         if (pc->fp32)
-        {
             pc->csl.pack<float>(ctx, pc->L.v32.p, nullptr);
-            pc->csu.pack<float>(ctx, pc->U.v32.p, pc->inv32.p);
-        }
         else
-        {
             pc->csl.pack<double>(ctx, pc->L.v.p, nullptr);
+    }
+    if (pc->chunk_u)
+    {
+        if (pc->fp32)
+            pc->csu.pack<float>(ctx, pc->U.v32.p, pc->inv32.p);
+        else
             pc->csu.pack<double>(ctx, pc->U.v.p, pc->inv.p);
-        }
     }
     sync(ctx);
     return pc;

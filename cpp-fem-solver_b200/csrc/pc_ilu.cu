@@ -24,6 +24,7 @@
 
 #include "trisolve.cuh"
 #include "trsv_chunk.cuh"
+#include "trsv_wave.cuh"
 #include "trsv_band.cuh"
 #include "pcg_band.cuh"
 #include "pcg_tile.cuh"
@@ -398,12 +399,6 @@ static void transpose_strict(b2s_ctx* ctx, const Csr32& L, Csr32& T)
 
 // ------------------------------------------------------------ triangular solves
 
-template <typename T>
-__device__ __forceinline__ T ld_dep(const T* p)
-{
-    return __ldcg(p);
-}
-
 // One row of a triangular solve:  x_i = (rhs_i - sum_{deps j} V_ij x_j) [/ d_i]
 // in the row's column order.  VT: factor storage, XT: solution / accumulation
 // type, RT: right-hand-side type.  out64 (optional) receives x as FP64.
@@ -416,11 +411,6 @@ struct TrsvOp
     const RT* rhs;
     XT* x;
     double* out64;
-    __device__ bool ready(uint32_t row, const uint32_t* flags, uint32_t epoch) const
-    {
-        return deps_ready<LOWER>(row, rp, ci, flags, epoch);
-    }
-    template <bool SYNCFREE>
     __device__ __forceinline__ void row_compute(uint32_t row) const
     {
         XT sum = (XT)rhs[row];
@@ -430,15 +420,13 @@ struct TrsvOp
             const uint32_t j = __ldg(&ci[p]);
             if (LOWER ? (j < row) : (j > row))
             {
-                const XT xj = SYNCFREE ? ld_dep(&x[j]) : x[j];
-                sum -= (XT)__ldg(&v[p]) * xj;
+                sum -= (XT)__ldg(&v[p]) * x[j];
             }
         }
         const XT r = UNIT ? sum : sum / (XT)__ldg(&d[row]);
         x[row] = r;
         if (out64) out64[row] = (double)r;
     }
-    __device__ void compute(uint32_t row) const { row_compute<true>(row); }
 };
 
 // D^-1 a in a Jacobi sweep: FP64 divides (the exact solves' arithmetic, so
@@ -506,8 +494,8 @@ struct Tri
     const double* d64 = nullptr;
     const float* d32 = nullptr;
     LevelSchedule sched;
-    SyncFree sf;
     ChunkSchedule cs;
+    WaveSchedule wave;
     Grid5Tri g5;  // 5-point grid factors: the exact solve with a lane per grid line
     Grid7Tri g7;  // 7-point grid factors: the same with planes handed on
     bool has_chunks = false, sched_ready = false;
@@ -603,9 +591,14 @@ struct Tri
             g7.run<LOWER, UNIT, VT, XT, RT>(ctx, rhs, x, out64, done);
         else if (mode == B2S_TRSV_CHUNK && has_chunks && cs.usable<VT, XT, RT>())
             cs.run<LOWER, UNIT, VT, XT, RT>(ctx, v, d, rhs, x, out64, done);
+        else if (mode == B2S_TRSV_LEVEL)
+            run_levels(ctx, sched, TrsvOp<LOWER, UNIT, VT, XT, RT>{m->rp.p, m->ci.p, v, d, rhs, x, out64}, done);
         else
-            run_schedule(ctx, mode == B2S_TRSV_LEVEL ? B2S_TRSV_LEVEL : B2S_TRSV_SYNCFREE, sched, sf,
-                         TrsvOp<LOWER, UNIT, VT, XT, RT>{m->rp.p, m->ci.p, v, d, rhs, x, out64}, done);
+        {
+            need(wave.n == n, B2S_UNSUPPORTED, "triangular solve: no schedule was prepared");
+            wave.run<1, LOWER, UNIT ? WaveDiag::Unit : WaveDiag::Divide>(ctx, m->rp.p, m->ci.p, v, d, rhs, x, out64,
+                                                                         done);
+        }
     }
 
     // x = T^-1 rhs; precision per the type parameters.  With out64 the results
@@ -632,7 +625,7 @@ struct Tri
         n = mat.n;
     }
 
-    // level schedule: the factorisation, the level / sync-free solves and export use it
+    // level schedule: the factorisation, the level-by-level solves and export use it
     void ensure_sched(b2s_ctx* ctx)
     {
         if (sched_ready) return;
@@ -640,15 +633,22 @@ struct Tri
             sched.build_host(ctx, h_level);
         else
             sched.build(ctx, n, m->rp.p, m->ci.p, lower);
-        sf.init(ctx, n);
         sched_ready = true;
     }
 
-    // a host chunk plan -> device; falls back to the level schedule when no plan is usable
-    void load_chunks(b2s_ctx* ctx, int mode, const ChunkPlan* plan, uint32_t vs)
+    // The exact solves' schedule: a host chunk plan, the level-by-level one, or
+    // the level-order traversal (where it pays, wave_pays, and where no chunk
+    // plan is usable).  rp: the triangle's rows (host); grid: a grid schedule
+    // takes the solves.
+    void load_exact(b2s_ctx* ctx, int mode, const ChunkPlan* plan, uint32_t vs, const uint32_t* rp, bool grid)
     {
-        has_chunks = mode == B2S_TRSV_CHUNK && n && plan && cs.load(ctx, *plan, vs);
-        if (!has_chunks && mode != B2S_TRSV_JACOBI) ensure_sched(ctx);
+        if (mode == B2S_TRSV_JACOBI || grid || !n) return;
+        has_chunks = mode == B2S_TRSV_CHUNK && plan && cs.load(ctx, *plan, vs);
+        if (has_chunks) return;
+        if (mode == B2S_TRSV_LEVEL)
+            ensure_sched(ctx);
+        else
+            wave.build(ctx, h_level, rp, 1);
     }
 
     // lay the final factor values out for the chunk schedule (no-op otherwise)
@@ -1334,13 +1334,13 @@ std::unique_ptr<PcImpl> make_pc_ic0_ex(b2s_ctx* ctx, const CsrDev& A, const b2s_
             plan_parallel(2, 2, [&](uint32_t side, unsigned) {
                 if (side == 0)
                 {
-                    if (ha.chunked)
+                    if (ha.chunked && !wave_pays(pc->fwd.h_level, hrp.data(), hci.data(), true))
                         ha.lo_plan = plan_chunks(n, hrp.data(), hci.data(), true, 1, vs, vs, 8, kChunkSmemBudget, 1,
                                                  &pc->fwd.h_level);
                     return;
                 }
                 compute_levels(n, ha.up_rp.data(), ha.up_ci.data(), false, ha.up_level);
-                if (ha.chunked)
+                if (ha.chunked && !wave_pays(ha.up_level, ha.up_rp.data(), ha.up_ci.data(), false))
                     ha.up_plan = plan_chunks(n, ha.up_rp.data(), ha.up_ci.data(), false, 1, vs, vs, 8,
                                              kChunkSmemBudget, 1, &ha.up_level);
             });
@@ -1379,8 +1379,8 @@ std::unique_ptr<PcImpl> make_pc_ic0_ex(b2s_ctx* ctx, const CsrDev& A, const b2s_
     ha.wait();
     pc->bwd.init(pc->LT, false, false);
     pc->bwd.h_level = std::move(ha.up_level);
-    pc->fwd.load_chunks(ctx, pc->mode, ha.chunked ? &ha.lo_plan : nullptr, vs);
-    pc->bwd.load_chunks(ctx, pc->mode, ha.chunked ? &ha.up_plan : nullptr, vs);
+    pc->fwd.load_exact(ctx, pc->mode, ha.chunked ? &ha.lo_plan : nullptr, vs, hrp.data(), gs.any());
+    pc->bwd.load_exact(ctx, pc->mode, ha.chunked ? &ha.up_plan : nullptr, vs, ha.up_rp.data(), gs.any());
     enable_grid(pc->fwd, pc->bwd, gs, n);
     if (sweeps)
     {
@@ -1496,13 +1496,13 @@ std::unique_ptr<PcImpl> make_pc_ilu0(b2s_ctx* ctx, const CsrDev& A, const b2s_pc
             plan_parallel(2, 2, [&](uint32_t side, unsigned) {
                 if (side == 0)
                 {
-                    if (ha.chunked)
+                    if (ha.chunked && !wave_pays(pc->fwd.h_level, lrp.data(), lci.data(), true))
                         ha.lo_plan = plan_chunks(n, lrp.data(), lci.data(), true, 0, vs, vs, 8, kChunkSmemBudget, 1,
                                                  &pc->fwd.h_level);
                     return;
                 }
                 compute_levels(n, urp.data(), uci.data(), false, ha.up_level);
-                if (ha.chunked)
+                if (ha.chunked && !wave_pays(ha.up_level, urp.data(), uci.data(), false))
                     ha.up_plan = plan_chunks(n, urp.data(), uci.data(), false, 1, vs, vs, 8, kChunkSmemBudget, 1,
                                              &ha.up_level);
             });
@@ -1534,8 +1534,8 @@ std::unique_ptr<PcImpl> make_pc_ilu0(b2s_ctx* ctx, const CsrDev& A, const b2s_pc
     ha.wait();
     pc->bwd.init(pc->U, false, false);
     pc->bwd.h_level = std::move(ha.up_level);
-    pc->fwd.load_chunks(ctx, pc->mode, ha.chunked ? &ha.lo_plan : nullptr, vs);
-    pc->bwd.load_chunks(ctx, pc->mode, ha.chunked ? &ha.up_plan : nullptr, vs);
+    pc->fwd.load_exact(ctx, pc->mode, ha.chunked ? &ha.lo_plan : nullptr, vs, lrp.data(), gs.any());
+    pc->bwd.load_exact(ctx, pc->mode, ha.chunked ? &ha.up_plan : nullptr, vs, urp.data(), gs.any());
     enable_grid(pc->fwd, pc->bwd, gs, n);
     if (pc->mode == B2S_TRSV_JACOBI)
     {

@@ -1,6 +1,6 @@
-// Level schedules of triangular dependency DAGs and the two ways of running
-// a per-row operation over them (one launch per level, or one sync-free
-// launch).  Shared by the scalar and block incomplete factorisations.
+// Level schedules of triangular dependency DAGs and a per-row operation run
+// over them, one launch per level.  Shared by the scalar and block incomplete
+// factorisations.
 #pragma once
 #include <cub/cub.cuh>
 
@@ -177,27 +177,20 @@ __global__ void __launch_bounds__(kThreads) k_trsv_level(const uint32_t* __restr
 {
     if (done && *done) return;
     const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t < count) op.template row_compute<false>(rows[t]);
+    if (t < count) op.row_compute(rows[t]);
 }
 
-
-// Runs op over every row of a schedule: B2S_TRSV_LEVEL launches one kernel
-// per level (rows of a level are independent); otherwise one sync-free
-// traversal in level-sorted order.
+// Runs op over every row of a schedule, one launch per level (rows of a level
+// are independent): B2S_TRSV_LEVEL.
 template <typename Op>
-void run_schedule(b2s_ctx* ctx, int mode, const LevelSchedule& sched, SyncFree& sf, const Op& op, const int* done)
+void run_levels(b2s_ctx* ctx, const LevelSchedule& sched, const Op& op, const int* done)
 {
-    if (mode == B2S_TRSV_LEVEL)
+    for (uint32_t l = 0; l < sched.nlev; ++l)
     {
-        for (uint32_t l = 0; l < sched.nlev; ++l)
-        {
-            const uint32_t a = sched.h_ptr[l], cnt = sched.h_ptr[l + 1] - a;
-            B2S_LAUNCH(ctx, k_trsv_level<Op>, (cnt + kThreads - 1) / kThreads, kThreads, 0, sched.rows.p + a, cnt, op,
-                       done);
-        }
+        const uint32_t a = sched.h_ptr[l], cnt = sched.h_ptr[l + 1] - a;
+        B2S_LAUNCH(ctx, k_trsv_level<Op>, (cnt + kThreads - 1) / kThreads, kThreads, 0, sched.rows.p + a, cnt, op,
+                   done);
     }
-    else
-        sf.run(ctx, sched.rows.p, false, op, done);
 }
 
 }  // namespace b2s

@@ -76,8 +76,9 @@ uint64_t b2s_ctx_kernel_launches(const b2s_ctx* ctx);
  * (IC(0) / ILU(0) / block ILU(0) with B2S_TRSV_CHUNK, the default): a wait
  * polls spin_polls times without sleeping, then sleeps 1 us per poll, drawing
  * on a budget of sleep_polls per thread for the whole launch.  The 5- and
- * 7-point grid schedules of the same solves poll a group's hand-over words
- * up to spin_polls + sleep_polls times (at least once) without sleeping.  A
+ * 7-point grid schedules and the level-order traversal (B2S_TRSV_SYNCFREE) of
+ * the same solves poll a wait's words up to spin_polls + sleep_polls times (at
+ * least once) without sleeping.  A
  * wait that runs out, and every later wait of the same launch, gives up at
  * once and the call reports B2S_TIMEOUT (the synchronous calls at their end, the _device
  * ones at the next b2s_ctx_synchronize or solve).  (0, 0) restores the
@@ -208,9 +209,11 @@ typedef enum b2s_trsv
 {
     B2S_TRSV_AUTO = 0,
     B2S_TRSV_LEVEL = 1,    /* one launch per level of the dependency DAG */
-    B2S_TRSV_SYNCFREE = 2, /* one launch; rows wait on bounded per-row ready flags */
-    B2S_TRSV_CHUNK = 3,    /* one launch; row chunks staged in shared memory, local levels split by
-                              barriers, bounded flags between chunks (the AUTO choice) */
+    B2S_TRSV_SYNCFREE = 2, /* one launch; rows in level order, each waiting (bounded) for its operands */
+    B2S_TRSV_CHUNK = 3,    /* one launch (the AUTO choice): row chunks staged in shared memory, local
+                              levels split by barriers, bounded flags between chunks; triangles with
+                              wide rows or many rows a level take SYNCFREE's traversal instead, and
+                              5- / 7-point grid factors their grid schedules */
     B2S_TRSV_JACOBI = 4    /* inexact: rows grouped into segments of trsv_segment consecutive rows;
                               each segment solved on its own, then trsv_sweeps block-Jacobi sweeps
                               (Gauss-Seidel inside a segment, the previous sweep's values outside);

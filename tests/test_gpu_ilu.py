@@ -712,3 +712,31 @@ def test_tiled_grid_blobs_match_general_planner(b2s, ctx, monkeypatch, nx, ny, k
     x2, s2 = b2s.solve(ctx, A, b, b2s.PCG, M_bfs, tol=1e-8, maxit=5000)
     assert s1["status"] == 0 and s1["relres_true"] < 1e-8
     assert s1["iterations"] == s2["iterations"] and np.array_equal(x1, x2)
+
+
+@pytest.mark.parametrize("width", [1, 4, 5, 8, 9, 16, 17, 32, 33])
+def test_level_order_traversal_widths(b2s, ctx, orc, width):
+    """B2S_TRSV_SYNCFREE on both sides of each lane-group width (4, 8, 16, 32
+    entries a row, the diagonal of U among them) and past the widest: bands of
+    which every third row keeps all `width` lower entries, so levels end in
+    part-filled warps.  FP64 equals the restatement bit for bit, FP32 the
+    chunked schedule's bits (the same arithmetic)."""
+    n, rng = 700, np.random.default_rng(width)
+    R, Cc, V = [], [], []
+    for i in range(n):
+        for j in range(max(0, i - width), i):
+            if i % 3 == 0 or rng.random() < 0.3:
+                a = -rng.uniform(0.1, 1.0)
+                R += [i, j]; Cc += [j, i]; V += [a, a]
+    R, Cc, V = np.array(R + list(range(n))), np.array(Cc + list(range(n))), np.array(V + [4.0 * width] * n)
+    n, rp, ci, v = (n,) + P.coo_to_csr(n, n, R, Cc, V)
+    A = b2s.CSR(ctx, n, n, rp, ci, v)
+    r = b2s.uniform(width, n)
+    for kind in ("ic0", "ilu0"):
+        k = b2s.PC_NAMES[kind]
+        z = b2s.Precond(ctx, A, k, trsv=b2s.TRSV_SYNCFREE).apply(r)
+        assert np.array_equal(z, orc.pc(orc.csr(n, n, rp, ci, v), kind).apply(r)), kind
+        z32 = b2s.Precond(ctx, A, k, precision=b2s.FP32, trsv=b2s.TRSV_SYNCFREE).apply(r)
+        if width <= 4:  # wider rows take the traversal under CHUNK too
+            assert np.array_equal(z32, b2s.Precond(ctx, A, k, precision=b2s.FP32, trsv=b2s.TRSV_CHUNK).apply(r)), kind
+        assert rel(z32, z) < 1e-4, kind
