@@ -784,9 +784,9 @@ static void export_grid5(const Tri& fwd, const Tri& bwd, uint64_t* sizes)
 static void export_grid7(const Tri& fwd, const Tri& bwd, uint64_t* sizes)
 {
     const bool on = fwd.g7.on && bwd.g7.on && fwd.g7.packed_v && bwd.g7.packed_v;
-    sizes[0] = on ? fwd.g7.B : 0;
-    sizes[1] = on ? fwd.g7.ny : 0;
-    sizes[2] = on ? fwd.g7.nz : 0;
+    sizes[0] = on ? fwd.g7.sh.B : 0;
+    sizes[1] = on ? fwd.g7.sh.ny : 0;
+    sizes[2] = on ? fwd.g7.sh.nz : 0;
 }
 
 // the grid row length B of a lower triangle that is a 5-point grid's, else 0
@@ -823,7 +823,7 @@ static GridShape grid_shape(uint32_t n, const std::vector<uint32_t>& lrp, const 
         std::copy(d, d + 3, g.d7);
     return g;
 }
-static void enable_grid(Tri& fwd, Tri& bwd, const GridShape& g, uint32_t n)
+static void enable_grid(b2s_ctx* ctx, Tri& fwd, Tri& bwd, const GridShape& g, uint32_t n)
 {
     if (g.b5)
     {
@@ -832,8 +832,8 @@ static void enable_grid(Tri& fwd, Tri& bwd, const GridShape& g, uint32_t n)
     }
     else if (g.d7[0])
     {
-        fwd.g7.enable(g.d7[0], g.d7[1], g.d7[2]);
-        bwd.g7.enable(g.d7[0], g.d7[1], g.d7[2]);
+        fwd.g7.enable(ctx, g.d7[0], g.d7[1], g.d7[2]);
+        bwd.g7.enable(ctx, g.d7[0], g.d7[1], g.d7[2]);
     }
 }
 
@@ -1381,7 +1381,7 @@ std::unique_ptr<PcImpl> make_pc_ic0_ex(b2s_ctx* ctx, const CsrDev& A, const b2s_
     pc->bwd.h_level = std::move(ha.up_level);
     pc->fwd.load_exact(ctx, pc->mode, ha.chunked ? &ha.lo_plan : nullptr, vs, hrp.data(), gs.any());
     pc->bwd.load_exact(ctx, pc->mode, ha.chunked ? &ha.up_plan : nullptr, vs, ha.up_rp.data(), gs.any());
-    enable_grid(pc->fwd, pc->bwd, gs, n);
+    enable_grid(ctx, pc->fwd, pc->bwd, gs, n);
     if (sweeps)
     {
         pc->fwd.prepare_sweeps(ctx, nsweeps, seg, pc->fp32, &ha.lo_band);
@@ -1536,7 +1536,7 @@ std::unique_ptr<PcImpl> make_pc_ilu0(b2s_ctx* ctx, const CsrDev& A, const b2s_pc
     pc->bwd.h_level = std::move(ha.up_level);
     pc->fwd.load_exact(ctx, pc->mode, ha.chunked ? &ha.lo_plan : nullptr, vs, lrp.data(), gs.any());
     pc->bwd.load_exact(ctx, pc->mode, ha.chunked ? &ha.up_plan : nullptr, vs, urp.data(), gs.any());
-    enable_grid(pc->fwd, pc->bwd, gs, n);
+    enable_grid(ctx, pc->fwd, pc->bwd, gs, n);
     if (pc->mode == B2S_TRSV_JACOBI)
     {
         const int k = sweep_count(o);

@@ -740,3 +740,21 @@ def test_level_order_traversal_widths(b2s, ctx, orc, width):
         if width <= 4:  # wider rows take the traversal under CHUNK too
             assert np.array_equal(z32, b2s.Precond(ctx, A, k, precision=b2s.FP32, trsv=b2s.TRSV_CHUNK).apply(r)), kind
         assert rel(z32, z) < 1e-4, kind
+
+
+@pytest.mark.parametrize("nx,ny,nz", [(2, 2, 2), (5, 8, 4), (33, 2, 40), (4, 70, 2), (3, 17, 13), (4, 3, 100),
+                                      (40, 100, 3), (18, 33, 31)])
+def test_grid7_tile_shapes(b2s, ctx, orc, nx, ny, nz):
+    """The 7-point schedule's tilings, from 1 x 32 to 32 x 1 lines a warp by the
+    grid's shape, with exact fits, remainders in y, z and both, and lines
+    shorter and longer than the operand ring: FP64 applies bit for bit as the
+    restatement, FP32 as the FP32 emulation."""
+    n, rp, ci, v = P.diffusion3d(nx, ny, nz, seed=nx + 3 * ny + nz)
+    A = b2s.CSR(ctx, n, n, rp, ci, v)
+    r = b2s.uniform(nx * ny + nz, n)
+    for kind in ("ic0", "ilu0"):
+        M = b2s.Precond(ctx, A, b2s.PC_NAMES[kind])
+        assert M.sizes("trsv.grid7") == (nx, ny, nz), kind
+        assert np.array_equal(M.apply(r), orc.pc(orc.csr(n, n, rp, ci, v), kind).apply(r)), kind
+        M32 = b2s.Precond(ctx, A, b2s.PC_NAMES[kind], precision=b2s.FP32)
+        assert np.array_equal(M32.apply(r), _f32_want(M32, kind, r)), kind
