@@ -28,8 +28,7 @@
 #include "trsv_band.cuh"
 #include "pcg_band.cuh"
 #include "pcg_tile.cuh"
-#include "trsv_grid5.cuh"
-#include "trsv_grid7.cuh"
+#include "trsv_grid.cuh"
 
 #include <cstdlib>
 #include <cstring>
@@ -496,8 +495,7 @@ struct Tri
     LevelSchedule sched;
     ChunkSchedule cs;
     WaveSchedule wave;
-    Grid5Tri g5;  // 5-point grid factors: the exact solve with a lane per grid line
-    Grid7Tri g7;  // 7-point grid factors: the same with planes handed on
+    GridTri grid;  // 5- and 7-point grid factors: the exact solve with a lane per grid line
     bool has_chunks = false, sched_ready = false;
     std::vector<uint32_t> h_level;  // host copy of the rows' levels (compute_levels), when known
     int sweeps = 8;                 // B2S_TRSV_JACOBI: sweeps after pass 0
@@ -585,10 +583,8 @@ struct Tri
     {
         if (mode == B2S_TRSV_JACOBI)
             run_sweeps<LOWER, UNIT, VT, XT, RT>(ctx, v, d, rhs, x, out64, done);
-        else if (mode == B2S_TRSV_CHUNK && g5.usable<VT, XT>() && g5.packed_v == (const void*)v)
-            g5.run<LOWER, UNIT, VT, XT, RT>(ctx, rhs, x, out64, done);
-        else if (mode == B2S_TRSV_CHUNK && g7.usable<VT, XT>() && g7.packed_v == (const void*)v)
-            g7.run<LOWER, UNIT, VT, XT, RT>(ctx, rhs, x, out64, done);
+        else if (mode == B2S_TRSV_CHUNK && grid.usable<VT, XT>() && grid.packed_v == (const void*)v)
+            grid.run<LOWER, UNIT, VT, XT, RT>(ctx, rhs, x, out64, done);
         else if (mode == B2S_TRSV_CHUNK && has_chunks && cs.usable<VT, XT, RT>())
             cs.run<LOWER, UNIT, VT, XT, RT>(ctx, v, d, rhs, x, out64, done);
         else if (mode == B2S_TRSV_LEVEL)
@@ -656,8 +652,7 @@ struct Tri
     void pack(b2s_ctx* ctx, const VT* v, const VT* d)
     {
         if (has_chunks && sizeof(VT) <= cs.plan_vs) cs.pack<VT>(ctx, v, d);
-        g5.pack<VT>(ctx, m->rp.p, m->ci.p, v, d, lower, unit);
-        g7.pack<VT>(ctx, m->rp.p, m->ci.p, v, d, lower, unit);
+        grid.pack<VT>(ctx, m->rp.p, m->ci.p, v, d, lower, unit);
         if constexpr (sizeof(VT) == 4)
         {
             if (band.T && n)
@@ -773,20 +768,20 @@ static PatternStats pattern_stats(b2s_ctx* ctx, const Csr32& L)
 // both triangles' coefficients are packed}
 static void export_grid5(const Tri& fwd, const Tri& bwd, uint64_t* sizes)
 {
-    const bool on = fwd.g5.on && bwd.g5.on;
-    sizes[0] = on ? fwd.g5.B : 0;
-    sizes[1] = on ? fwd.g5.ny : 0;
-    sizes[2] = on && fwd.g5.packed_v && bwd.g5.packed_v ? 1 : 0;
+    const bool on = fwd.grid.on && bwd.grid.on && fwd.grid.sh.nz == 1;
+    sizes[0] = on ? fwd.grid.sh.B : 0;
+    sizes[1] = on ? fwd.grid.sh.ny : 0;
+    sizes[2] = on && fwd.grid.packed_v && bwd.grid.packed_v ? 1 : 0;
 }
 
 // "trsv.grid7": sizes = {B, ny, nz} of the 7-point grid schedule when both
 // triangles take it (packed), else zeros
 static void export_grid7(const Tri& fwd, const Tri& bwd, uint64_t* sizes)
 {
-    const bool on = fwd.g7.on && bwd.g7.on && fwd.g7.packed_v && bwd.g7.packed_v;
-    sizes[0] = on ? fwd.g7.sh.B : 0;
-    sizes[1] = on ? fwd.g7.sh.ny : 0;
-    sizes[2] = on ? fwd.g7.sh.nz : 0;
+    const bool on = fwd.grid.on && bwd.grid.on && fwd.grid.sh.nz > 1 && fwd.grid.packed_v && bwd.grid.packed_v;
+    sizes[0] = on ? fwd.grid.sh.B : 0;
+    sizes[1] = on ? fwd.grid.sh.ny : 0;
+    sizes[2] = on ? fwd.grid.sh.nz : 0;
 }
 
 // the grid row length B of a lower triangle that is a 5-point grid's, else 0
@@ -813,28 +808,22 @@ static GridShape grid_shape(uint32_t n, const std::vector<uint32_t>& lrp, const 
     if (!n) return g;
     if (const uint32_t B = grid5_lower_b(n, lrp, lci))
     {
-        if (Grid5Tri::fits(B, n / B) && (!urp || grid5_triangle(n, urp->data(), uci->data(), B, false))) g.b5 = B;
+        if (GridTri::fits5(B, n / B) && (!urp || grid5_triangle(n, urp->data(), uci->data(), B, false))) g.b5 = B;
         return g;
     }
     uint32_t d[3];
     grid7_dims(n, lrp.data(), lci.data(), d);
-    if (d[0] && Grid7Tri::fits(d[0], d[1], d[2]) &&
+    if (d[0] && GridTri::fits7(d[0], d[1], d[2]) &&
         (!urp || grid7_triangle(n, urp->data(), uci->data(), d[0], d[1], false)))
         std::copy(d, d + 3, g.d7);
     return g;
 }
 static void enable_grid(b2s_ctx* ctx, Tri& fwd, Tri& bwd, const GridShape& g, uint32_t n)
 {
-    if (g.b5)
-    {
-        fwd.g5.enable(g.b5, n / g.b5);
-        bwd.g5.enable(g.b5, n / g.b5);
-    }
-    else if (g.d7[0])
-    {
-        fwd.g7.enable(ctx, g.d7[0], g.d7[1], g.d7[2]);
-        bwd.g7.enable(ctx, g.d7[0], g.d7[1], g.d7[2]);
-    }
+    if (!g.any()) return;
+    const uint32_t b = g.b5 ? g.b5 : g.d7[0], y = g.b5 ? n / g.b5 : g.d7[1], z = g.b5 ? 1u : g.d7[2];
+    fwd.grid.enable(ctx, b, y, z);
+    bwd.grid.enable(ctx, b, y, z);
 }
 
 static void copy_pattern(b2s_ctx* ctx, const Csr32& M, std::vector<uint32_t>& rp, std::vector<uint32_t>& ci)

@@ -22,7 +22,7 @@
 // The last CTA to leave resets the ticket and advances the epoch; the exchange
 // array is never cleared and a captured launch can be replayed.
 #pragma once
-#include "trsv_grid5.cuh"
+#include "trsv_grid.cuh"
 
 namespace b2s {
 
@@ -113,7 +113,7 @@ __global__ void __launch_bounds__(wave_threads(GL)) k_trsv_wave(WaveArgs a, cons
     else
         for (XT& e : dv) e = XT(1);
     // FP32 multiplies by the reciprocal rounded once from FP64, FP64 forms the
-    // quotient from the reciprocal (g5_quotient): both before the wait
+    // quotient from the reciprocal (grid_quotient): both before the wait
     [[maybe_unused]] XT rc = XT(1);
     if constexpr (DIAG == WaveDiag::Divide) rc = (XT)(1.0 / (double)dv[0]);
 
@@ -191,7 +191,7 @@ __global__ void __launch_bounds__(wave_threads(GL)) k_trsv_wave(WaveArgs a, cons
         else
         {
             bool bad = false;
-            r = g5_quotient(sum, dv[0], rc, true, bad);
+            r = grid_quotient(sum, dv[0], rc, true, bad);
             if (bad) r = sum / dv[0];
         }
     }
