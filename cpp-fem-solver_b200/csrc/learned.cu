@@ -156,7 +156,7 @@ __global__ void k_logdiag_sum(uint32_t n, const double* __restrict__ d, double* 
 
 // Y (n x NO) = act(X (n x K) W^T + b), W (NO x K) in BF16, FP32 accumulation.
 // Optionally stores the pre-activation; RES adds X (K == NO) after the activation.
-constexpr int kFwdRows = 32, kBwdRows = 16;
+constexpr int kFwdRows = 32;
 
 template <int K, int NO, bool RELU>
 __global__ void __launch_bounds__(256) k_linear(uint32_t n, const float* __restrict__ X,
@@ -201,99 +201,143 @@ __global__ void __launch_bounds__(256) k_linear(uint32_t n, const float* __restr
     }
 }
 
-// dX (n x K) += dY (n x NO) W (NO x K)
+// The backward products run on the CUDA cores in FP32: dY is an FP32 gradient, and
+// rounding it to BF16 for the tensor cores would lose what the sums are made of.
+// Each thread holds an 8 x 4 tile of the result in registers and reads 12 operands
+// from shared memory for its 32 multiply-adds (explicit FMA: one rounding, where
+// the library's flags would round twice).  512^2: dX 0.370 -> 0.153 ms, dW 0.529
+// -> 0.174 ms a layer (a thread a column, or a scalar product at a time, before).
+constexpr int kTileR = 8, kTileC = 4;
+
+// dX (n x K) += dY (n x NO) W (NO x K): a CTA's 256 threads cover 8 * 256 / (K / 4) rows
 template <int K, int NO>
 __global__ void __launch_bounds__(256) k_linear_bwd_data(uint32_t n, const float* __restrict__ dY,
                                                          const __nv_bfloat16* __restrict__ W, float* __restrict__ dX)
 {
-    constexpr int ROWS = kBwdRows, TPR = 256 / ROWS, CPT = K / TPR;
-    __shared__ float Ws[NO][K + 1];
-    __shared__ float Ds[ROWS][NO + 1];
-    for (int t = threadIdx.x; t < K * NO; t += blockDim.x)
-    {
-        const int o = t / K, k = t % K;
-        Ws[o][k] = __bfloat162float(W[t]);
-    }
+    constexpr int CG = K / kTileC, RG = 256 / CG, ROWS = RG * kTileR, DEPTH = 32;
+    static_assert(K % kTileC == 0 && 256 % CG == 0 && NO % DEPTH == 0 && ROWS * DEPTH % 1024 == 0, "tile");
+    __shared__ __align__(16) float Ds[DEPTH][ROWS + 4];
+    __shared__ __align__(16) float Ws[DEPTH][K];
+    const int cg = threadIdx.x % CG, rg = threadIdx.x / CG;
     const uint32_t r0 = blockIdx.x * ROWS;
-    for (int t = threadIdx.x; t < ROWS * NO; t += blockDim.x)
+    float acc[kTileR][kTileC] = {};
+    for (int o0 = 0; o0 < NO; o0 += DEPTH)
     {
-        const int r = t / NO, o = t % NO;
-        Ds[r][o] = (r0 + r < n) ? dY[(size_t)(r0 + r) * NO + o] : 0.f;
-    }
-    __syncthreads();
-    const int r = threadIdx.x / TPR, cg = threadIdx.x % TPR;
-    float acc[CPT];
-#pragma unroll
-    for (int c = 0; c < CPT; ++c) acc[c] = 0.f;
-#pragma unroll 8
-    for (int o = 0; o < NO; ++o)
-    {
-        const float d = Ds[r][o];
-#pragma unroll
-        for (int c = 0; c < CPT; ++c) acc[c] += d * Ws[o][cg + c * TPR];
-    }
-    if (r0 + r < n)
-#pragma unroll
-        for (int c = 0; c < CPT; ++c)
+        __syncthreads();
+        // DEPTH columns of ROWS rows, transposed: a thread reads 4 columns of a row
+        for (int t = threadIdx.x; t < ROWS * DEPTH / 4; t += 256)
         {
-            const size_t idx = (size_t)(r0 + r) * K + cg + c * TPR;
-            dX[idx] += acc[c];
+            const int r = t / (DEPTH / 4), o = t % (DEPTH / 4) * 4;
+            const float4 d = r0 + r < n ? *reinterpret_cast<const float4*>(dY + (size_t)(r0 + r) * NO + o0 + o)
+                                        : make_float4(0.f, 0.f, 0.f, 0.f);
+            Ds[o][r] = d.x;
+            Ds[o + 1][r] = d.y;
+            Ds[o + 2][r] = d.z;
+            Ds[o + 3][r] = d.w;
         }
+        for (int t = threadIdx.x; t < DEPTH * K; t += 256) Ws[t / K][t % K] = __bfloat162float(W[(size_t)o0 * K + t]);
+        __syncthreads();
+#pragma unroll 4
+        for (int o = 0; o < DEPTH; ++o)
+        {
+            const float4 w = *reinterpret_cast<const float4*>(&Ws[o][cg * kTileC]);
+            const float4 a = *reinterpret_cast<const float4*>(&Ds[o][rg * kTileR]);
+            const float4 b = *reinterpret_cast<const float4*>(&Ds[o][rg * kTileR + 4]);
+            const float d[kTileR] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w}, v[kTileC] = {w.x, w.y, w.z, w.w};
+#pragma unroll
+            for (int r = 0; r < kTileR; ++r)
+#pragma unroll
+                for (int c = 0; c < kTileC; ++c) acc[r][c] = fmaf(d[r], v[c], acc[r][c]);
+        }
+    }
+#pragma unroll
+    for (int r = 0; r < kTileR; ++r)
+    {
+        const uint32_t row = r0 + rg * kTileR + r;
+        if (row >= n) break;
+        float4* out = reinterpret_cast<float4*>(dX + (size_t)row * K + cg * kTileC);
+        float4 x = *out;
+        x.x += acc[r][0];
+        x.y += acc[r][1];
+        x.z += acc[r][2];
+        x.w += acc[r][3];
+        *out = x;
+    }
 }
 
-// per-CTA partial of dW (NO x K) = dY^T X and db = sum dY over a row chunk;
-// RX: X rounded to BF16 first, the operand the tensor-core forward multiplied
-template <int K, int NO, bool RX>
+// per-CTA partial of dW (NO x K) = dY^T X and, with BIAS, of db = sum dY, over a
+// row chunk; RX: X rounded to BF16 first, the operand the tensor-core forward
+// multiplied.  Where the result has fewer tiles than the CTA has threads, SUB
+// groups of threads take every SUB-th row and are added in order at the end.
+template <int K, int NO, bool RX, bool BIAS>
 __global__ void __launch_bounds__(256) k_linear_bwd_weight(uint32_t n, uint32_t rows_per_cta, const float* __restrict__ dY,
                                                            const float* __restrict__ X, float* __restrict__ partial)
 {
-    constexpr int PAIRS = NO * K, PPT = (PAIRS + 255) / 256, TILE = 32;
-    __shared__ float Ds[TILE][NO];
-    __shared__ float Xs[TILE][K];
-    float acc[PPT];
+    constexpr int PAIRS = NO * K, KG = K / kTileC, NT = NO / kTileR * KG, SUB = 256 / NT, TILE = 32;
+    static_assert(NO % kTileR == 0 && K % kTileC == 0 && 256 % NT == 0 && TILE % SUB == 0 && NO <= 256, "tile");
+    // the rows of a pass, and at the end the SUB partial sums
+    __shared__ __align__(16) float sm[TILE * (NO + K) > (SUB > 1 ? SUB * PAIRS : 0) ? TILE * (NO + K) : SUB * PAIRS];
+    float(*Ds)[NO] = reinterpret_cast<float(*)[NO]>(sm);
+    float(*Xs)[K] = reinterpret_cast<float(*)[K]>(sm + TILE * NO);
+    const int sub = threadIdx.x / NT, t0 = threadIdx.x % NT, o0 = t0 / KG * kTileR, k0 = t0 % KG * kTileC;
+    float acc[kTileR][kTileC] = {};
     float bacc = 0.f;
-#pragma unroll
-    for (int q = 0; q < PPT; ++q) acc[q] = 0.f;
-    const uint32_t r_begin = blockIdx.x * rows_per_cta;
-    const uint32_t r_end = min(n, r_begin + rows_per_cta);
-    for (uint32_t t0 = r_begin; t0 < r_end; t0 += TILE)
+    const uint32_t r_begin = blockIdx.x * rows_per_cta, r_end = min(n, r_begin + rows_per_cta);
+    const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+    for (uint32_t rt = r_begin; rt < r_end; rt += TILE)
     {
         __syncthreads();
-        for (int t = threadIdx.x; t < TILE * NO; t += blockDim.x)
+        for (int t = threadIdx.x; t < TILE * NO / 4; t += 256)
         {
-            const int rr = t / NO, o = t % NO;
-            Ds[rr][o] = (t0 + rr < r_end) ? dY[(size_t)(t0 + rr) * NO + o] : 0.f;
+            const uint32_t rr = t / (NO / 4), o = t % (NO / 4) * 4;
+            *reinterpret_cast<float4*>(&Ds[rr][o]) =
+                rt + rr < r_end ? *reinterpret_cast<const float4*>(dY + (size_t)(rt + rr) * NO + o) : zero;
         }
-        for (int t = threadIdx.x; t < TILE * K; t += blockDim.x)
+        for (int t = threadIdx.x; t < TILE * K / 4; t += 256)
         {
-            const int rr = t / K, k = t % K;
-            const float x = (t0 + rr < r_end) ? X[(size_t)(t0 + rr) * K + k] : 0.f;
-            Xs[rr][k] = RX ? __bfloat162float(__float2bfloat16_rn(x)) : x;
+            const uint32_t rr = t / (K / 4), k = t % (K / 4) * 4;
+            float4 x = rt + rr < r_end ? *reinterpret_cast<const float4*>(X + (size_t)(rt + rr) * K + k) : zero;
+            if constexpr (RX)
+                x = make_float4(__bfloat162float(__float2bfloat16_rn(x.x)), __bfloat162float(__float2bfloat16_rn(x.y)),
+                                __bfloat162float(__float2bfloat16_rn(x.z)), __bfloat162float(__float2bfloat16_rn(x.w)));
+            *reinterpret_cast<float4*>(&Xs[rr][k]) = x;
         }
         __syncthreads();
-#pragma unroll
-        for (int q = 0; q < PPT; ++q)
+#pragma unroll 4
+        for (int rr = sub; rr < TILE; rr += SUB)
         {
-            const int pr = threadIdx.x + q * 256;
-            if (pr < PAIRS)
-            {
-                const int o = pr / K, k = pr % K;
-                float a = acc[q];
-                for (int rr = 0; rr < TILE; ++rr) a += Ds[rr][o] * Xs[rr][k];
-                acc[q] = a;
-            }
-        }
-        if (threadIdx.x < NO)
-            for (int rr = 0; rr < TILE; ++rr) bacc += Ds[rr][threadIdx.x];
-    }
-    float* out = partial + (size_t)blockIdx.x * (PAIRS + NO);
+            const float4 a = *reinterpret_cast<const float4*>(&Ds[rr][o0]);
+            const float4 b = *reinterpret_cast<const float4*>(&Ds[rr][o0 + 4]);
+            const float4 x = *reinterpret_cast<const float4*>(&Xs[rr][k0]);
+            const float d[kTileR] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w}, v[kTileC] = {x.x, x.y, x.z, x.w};
 #pragma unroll
-    for (int q = 0; q < PPT; ++q)
-    {
-        const int pr = threadIdx.x + q * 256;
-        if (pr < PAIRS) out[pr] = acc[q];
+            for (int o = 0; o < kTileR; ++o)
+#pragma unroll
+                for (int c = 0; c < kTileC; ++c) acc[o][c] = fmaf(d[o], v[c], acc[o][c]);
+        }
+        if constexpr (BIAS)
+            if (threadIdx.x < NO)
+                for (int rr = 0; rr < TILE; ++rr) bacc += Ds[rr][threadIdx.x];
     }
-    if (threadIdx.x < NO) out[PAIRS + threadIdx.x] = bacc;
+    float* out = partial + (size_t)blockIdx.x * (PAIRS + (BIAS ? NO : 0));
+    float* to = SUB > 1 ? sm + sub * PAIRS : out;
+    if constexpr (SUB > 1) __syncthreads();
+#pragma unroll
+    for (int o = 0; o < kTileR; ++o)
+#pragma unroll
+        for (int c = 0; c < kTileC; ++c) to[(o0 + o) * K + k0 + c] = acc[o][c];
+    if constexpr (SUB > 1)
+    {
+        __syncthreads();
+        for (int t = threadIdx.x; t < PAIRS; t += 256)
+        {
+            float a = 0.f;
+            for (int u = 0; u < SUB; ++u) a += sm[u * PAIRS + t];
+            out[t] = a;
+        }
+    }
+    if constexpr (BIAS)
+        if (threadIdx.x < NO) out[PAIRS + threadIdx.x] = bacc;
 }
 
 // out[j] = sum over b of partial[b * stride + j].  32 columns a CTA, one warp
@@ -334,66 +378,88 @@ static void reduce_partials(b2s_ctx* ctx, uint32_t nblocks, uint32_t stride, uin
 // ------------------------------------------------------------ message passing
 
 // SM = [s | m] (n x 128).  pre_i = s_i + b + invdeg_i sum_j g_ij m_j ;  Hn = relu(pre) + H
-__global__ void __launch_bounds__(256) k_aggregate(uint32_t n, const uint32_t* __restrict__ rp, const uint32_t* __restrict__ ci,
-                                                   const float* __restrict__ EF, const float* __restrict__ invdeg,
-                                                   const float* __restrict__ SM, const __nv_bfloat16* __restrict__ Wl,
-                                                   const float* __restrict__ Hin, float* __restrict__ pre,
-                                                   float* __restrict__ Hout)
+// Bound by instructions (a sigmoid an edge and channel).  Two neighbours at a
+// time and 6 CTAs an SM: 512^2 0.148 ms a layer; 4 and 4 0.168, 1 and 8 0.156;
+// 0.250 with the entries taken eight at a time, the diagonal and the slots past
+// the row among them, and a last wave of CTAs half empty.
+constexpr int kNeighbours = 2;
+
+__global__ void __launch_bounds__(256, 6) k_aggregate(uint32_t n, const uint32_t* __restrict__ rp,
+                                                      const uint32_t* __restrict__ ci, const float* __restrict__ EF,
+                                                      const float* __restrict__ invdeg, const float* __restrict__ SM,
+                                                      const __nv_bfloat16* __restrict__ Wl,
+                                                      const float* __restrict__ Hin, float* __restrict__ pre,
+                                                      float* __restrict__ Hout)
 {
     // one warp per node, 2 channels per lane
-    __shared__ float wg[H][FE], bg[H], bl[H];
-    for (int t = threadIdx.x; t < H * FE; t += blockDim.x) wg[t / FE][t % FE] = __bfloat162float(Wl[L_WG + t]);
-    for (int t = threadIdx.x; t < H; t += blockDim.x)
-    {
-        bg[t] = __bfloat162float(Wl[L_BG + t]);
-        bl[t] = __bfloat162float(Wl[L_B + t]);
-    }
-    __syncthreads();
     const int lane = threadIdx.x & 31;
-    const int c0 = lane, c1 = lane + 32;
-    // grid-stride over nodes, so the weights above are staged once per CTA
+    float wg[2][FE], bg[2], bl[2];
+#pragma unroll
+    for (int h = 0; h < 2; ++h)
+    {
+        const int c = lane + 32 * h;
+#pragma unroll
+        for (int f = 0; f < FE; ++f) wg[h][f] = __bfloat162float(Wl[L_WG + c * FE + f]);
+        bg[h] = __bfloat162float(Wl[L_BG + c]);
+        bl[h] = __bfloat162float(Wl[L_B + c]);
+    }
+    // grid-stride over nodes, so the weights above are read once per CTA
     for (uint32_t i = blockIdx.x * 8 + (threadIdx.x >> 5); i < n; i += gridDim.x * 8)
     {
-        float a0 = 0.f, a1 = 0.f;
-        // neighbours eight at a time: their indices, edge features and messages
-        // are all in flight before the gates are formed (same summation order)
+        float a[2] = {0.f, 0.f};
         const uint32_t pa = rp[i], pe = rp[i + 1];
-        for (uint32_t pb = pa; pb < pe; pb += 8)
-        {
-            uint32_t jj[8];
-            float4 ee[8];
-            float m0[8], m1[8];
-#pragma unroll
-            for (int k = 0; k < 8; ++k) jj[k] = pb + k < pe ? ci[pb + k] : i;
-#pragma unroll
-            for (int k = 0; k < 8; ++k)
-            {
-                const bool on = jj[k] != i;
-                ee[k] = on ? *reinterpret_cast<const float4*>(EF + (size_t)(pb + k) * FE) : make_float4(0.f, 0.f, 0.f, 0.f);
-                m0[k] = on ? SM[(size_t)jj[k] * 2 * H + H + c0] : 0.f;
-                m1[k] = on ? SM[(size_t)jj[k] * 2 * H + H + c1] : 0.f;
-            }
-#pragma unroll
-            for (int k = 0; k < 8; ++k)
-            {
-                if (jj[k] == i) continue;
-                const float4 e = ee[k];
-                const float g0 = sigm(bg[c0] + wg[c0][0] * e.x + wg[c0][1] * e.y + wg[c0][2] * e.z + wg[c0][3] * e.w);
-                const float g1 = sigm(bg[c1] + wg[c1][0] * e.x + wg[c1][1] * e.y + wg[c1][2] * e.z + wg[c1][3] * e.w);
-                a0 += g0 * m0[k];
-                a1 += g1 * m1[k];
-            }
-        }
         const float id = invdeg[i];
-        const float p0 = SM[(size_t)i * 2 * H + c0] + bl[c0] + id * a0;
-        const float p1 = SM[(size_t)i * 2 * H + c1] + bl[c1] + id * a1;
-        if (pre)  // kept for the backward pass (training only)
+        float s[2], hin[2];
+#pragma unroll
+        for (int h = 0; h < 2; ++h)
         {
-            pre[(size_t)i * H + c0] = p0;
-            pre[(size_t)i * H + c1] = p1;
+            s[h] = SM[(size_t)i * 2 * H + lane + 32 * h];
+            hin[h] = Hin[(size_t)i * H + lane + 32 * h];
         }
-        Hout[(size_t)i * H + c0] = fmaxf(p0, 0.f) + Hin[(size_t)i * H + c0];
-        Hout[(size_t)i * H + c1] = fmaxf(p1, 0.f) + Hin[(size_t)i * H + c1];
+        // a lane reads one of up to 32 entries; the warp then takes the neighbours
+        // (the diagonal left out) kNeighbours at a time, their features and messages in flight
+        // together, in row order
+        for (uint32_t pb = pa; pb < pe; pb += 32)
+        {
+            const uint32_t mine = pb + lane < pe ? ci[pb + lane] : i;
+            uint32_t m = __ballot_sync(0xffffffffu, mine != i);
+            while (m)
+            {
+                float4 e[kNeighbours];
+                float mk[kNeighbours][2];
+                bool on[kNeighbours];
+#pragma unroll
+                for (int k = 0; k < kNeighbours; ++k)
+                {
+                    on[k] = m != 0u;
+                    const int q = on[k] ? __ffs(m) - 1 : 0;
+                    const uint32_t j = __shfl_sync(0xffffffffu, mine, q);
+                    m &= m - 1u;
+                    if (on[k])
+                    {
+                        e[k] = *reinterpret_cast<const float4*>(EF + (size_t)(pb + q) * FE);
+#pragma unroll
+                        for (int h = 0; h < 2; ++h) mk[k][h] = SM[(size_t)j * 2 * H + H + lane + 32 * h];
+                    }
+                }
+#pragma unroll
+                for (int k = 0; k < kNeighbours; ++k)
+                    if (on[k])
+#pragma unroll
+                        for (int h = 0; h < 2; ++h)
+                            a[h] += sigm(bg[h] + wg[h][0] * e[k].x + wg[h][1] * e[k].y + wg[h][2] * e[k].z +
+                                         wg[h][3] * e[k].w) *
+                                    mk[k][h];
+            }
+        }
+#pragma unroll
+        for (int h = 0; h < 2; ++h)
+        {
+            const size_t o = (size_t)i * H + lane + 32 * h;
+            const float p = s[h] + bl[h] + id * a[h];
+            if (pre) pre[o] = p;  // kept for the backward pass (training only)
+            Hout[o] = fmaxf(p, 0.f) + hin[h];
+        }
     }
 }
 
@@ -403,14 +469,11 @@ __global__ void __launch_bounds__(256) k_aggregate(uint32_t n, const uint32_t* _
 //   per-CTA partials of dW_g (64x4), db_g (64), db (64)
 // One warp per node as in the forward kernel, grid-stride: a lane keeps its two
 // channels' gate gradients in registers over all its nodes, so a CTA writes one
-// 1.5 KB partial at its end instead of one for every 8 nodes, and a batch of
-// edges has all its gathers in flight before the gates are formed.  Bound by
-// the gathers' latency and the sigmoids (two an edge and channel): 512^2 in
-// 0.565 ms before (a node a warp and CTA lifetime, the partials summed in
-// shared memory).
-constexpr int kEdgeBatch = 4;
-
-__global__ void __launch_bounds__(256, 2) k_aggregate_bwd(uint32_t n, const uint32_t* __restrict__ rp,
+// 1.5 KB partial at its end instead of one for every 8 nodes.  Bound by the
+// instructions of the sigmoids (two an edge and channel); what hides the
+// gathers is warps, not edges in flight: 512^2 with 1 / 2 / 4 edges at a time
+// and 4 / 4 / 2 CTAs an SM 0.308 / 0.349 / 0.565 ms.
+__global__ void __launch_bounds__(256, 4) k_aggregate_bwd(uint32_t n, const uint32_t* __restrict__ rp,
                                                           const uint32_t* __restrict__ ci,
                                                           const uint32_t* __restrict__ rev,
                                                           const float* __restrict__ EF,
@@ -449,47 +512,27 @@ __global__ void __launch_bounds__(256, 2) k_aggregate_bwd(uint32_t n, const uint
             dpj[h] = dp[h] * idj;
             acc[h][FE + 1] += dp[h];
         }
-        const uint32_t pa = rp[j], pe = rp[j + 1];
-        for (uint32_t pb = pa; pb < pe; pb += kEdgeBatch)
+        const uint32_t pe = rp[j + 1];
+        for (uint32_t p = rp[j]; p < pe; ++p)
         {
-            uint32_t ii[kEdgeBatch];
-            float4 eo[kEdgeBatch], ei[kEdgeBatch];  // features of (j, i) and of (i, j), listed in row i at rev[p]
-            float di[kEdgeBatch][2], mi[kEdgeBatch][2], idi[kEdgeBatch];
+            const uint32_t i = ci[p];
+            if (i == j) continue;
+            // features of (j, i), and of (i, j), which row i lists at rev[p]
+            const float4 eo = *reinterpret_cast<const float4*>(EF + (size_t)p * FE);
+            const float4 ei = *reinterpret_cast<const float4*>(EF + (size_t)rev[p] * FE);
+            const float idi = invdeg[i];
 #pragma unroll
-            for (int k = 0; k < kEdgeBatch; ++k) ii[k] = pb + k < pe ? ci[pb + k] : j;
-#pragma unroll
-            for (int k = 0; k < kEdgeBatch; ++k)
+            for (int h = 0; h < 2; ++h)
             {
-                const bool on = ii[k] != j;
-                const uint32_t q = on ? rev[pb + k] : 0u, i = on ? ii[k] : j;
-                const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
-                eo[k] = on ? *reinterpret_cast<const float4*>(EF + (size_t)(pb + k) * FE) : zero;
-                ei[k] = on ? *reinterpret_cast<const float4*>(EF + (size_t)q * FE) : zero;
-                idi[k] = invdeg[i];
-#pragma unroll
-                for (int h = 0; h < 2; ++h)
-                {
-                    const size_t o = (size_t)i * H + lane + 32 * h;
-                    di[k][h] = pre[o] > 0.f ? dHout[o] : 0.f;
-                    mi[k][h] = SM[(size_t)i * 2 * H + H + lane + 32 * h];
-                }
-            }
-#pragma unroll
-            for (int k = 0; k < kEdgeBatch; ++k)
-            {
-                if (ii[k] == j) continue;  // the diagonal, or past the row's end: the whole warp
-#pragma unroll
-                for (int h = 0; h < 2; ++h)
-                {
-                    dm[h] += idi[k] * di[k][h] * gate(h, ei[k]);
-                    const float g = gate(h, eo[k]);
-                    const float dz = dpj[h] * mi[k][h] * g * (1.f - g);
-                    acc[h][0] += dz * eo[k].x;
-                    acc[h][1] += dz * eo[k].y;
-                    acc[h][2] += dz * eo[k].z;
-                    acc[h][3] += dz * eo[k].w;
-                    acc[h][FE] += dz;
-                }
+                const size_t o = (size_t)i * H + lane + 32 * h;
+                const float di = pre[o] > 0.f ? dHout[o] : 0.f, m = SM[(size_t)i * 2 * H + H + lane + 32 * h];
+                dm[h] += idi * di * gate(h, ei);
+                const float g = gate(h, eo), dz = dpj[h] * m * g * (1.f - g);
+                acc[h][0] += dz * eo.x;
+                acc[h][1] += dz * eo.y;
+                acc[h][2] += dz * eo.z;
+                acc[h][3] += dz * eo.w;
+                acc[h][FE] += dz;
             }
         }
 #pragma unroll
@@ -971,6 +1014,16 @@ __global__ void k_gate_grads(const float* __restrict__ red, float* __restrict__ 
 
 }  // namespace
 
+// CTAs of a grid-stride node kernel (8 nodes a pass of 256 threads): as many as
+// the SMs hold at once, so that no last wave is left over
+template <typename Kern>
+static unsigned node_grid(b2s_ctx* ctx, Kern kern, uint32_t n)
+{
+    int occ = 0;
+    B2S_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kern, 256, 0));
+    return std::min<unsigned>((n + 7) / 8, (unsigned)(ctx->sm_count * std::max(occ, 1)));
+}
+
 // ------------------------------------------------------------ network state
 
 // Y = bf16(X) W^T [+ bias] on the tensor cores (tc_linear.cuh)
@@ -1107,7 +1160,7 @@ struct GnnGraph
     void forward(b2s_ctx* ctx, const Gnn& net, const CsrDev& A)
     {
         const unsigned g64 = (n + kFwdRows - 1) / kFwdRows;
-        const unsigned gw = std::min<unsigned>((n + 7) / 8, (unsigned)ctx->sm_count * 8);
+        const unsigned gw = node_grid(ctx, k_aggregate, n);
         B2S_LAUNCH(ctx, (k_linear<FIN, H, true>), g64, 256, 0, n, F.p, net.pb.p + OFF_WIN, net.pr.p + OFF_BIN,
                    state_mut(0), training ? pre0.p : (float*)nullptr);
         for (int l = 0; l < NL; ++l)
@@ -1433,18 +1486,20 @@ static void train_step(b2s_ctx* ctx, Gnn& net, const CsrDev& A, int nprobes, uin
     B2S_LAUNCH(ctx, k_head_dc, stream_grid(ctx, Lnnz), kThreads, 0, Lnnz, dL.p, Lv.p, L0.p, C.p, dC.p);
 
     // backward
-    const unsigned g64 = (n + kBwdRows - 1) / kBwdRows;
-    // node kernels: grid-stride, at most 4 CTAs an SM (one partial of the parameter gradients each)
-    const unsigned gw = std::min<unsigned>((n + 7) / 8, (unsigned)ctx->sm_count * 4);
+    constexpr uint32_t bwd_rows = kTileR * 256 / (H / kTileC);
+    const unsigned g64 = (n + bwd_rows - 1) / bwd_rows;
+    const unsigned gw = node_grid(ctx, k_aggregate_bwd, n), gh = node_grid(ctx, k_head_bwd, n);
     B2S_CUDA(cudaMemsetAsync(net.g.p, 0, net.g.bytes(), ctx->stream));
     DBuf<float> dH(n * (size_t)H), dSM(n * (size_t)2 * H), part;
-    part.alloc((size_t)std::max<unsigned>(gw, 1) * (H * (FE + 2) > O_SIZE ? H * (FE + 2) : O_SIZE) + 16);
-    B2S_LAUNCH(ctx, k_head_bwd, gw, 256, 0, n, Lrp.p, Lci.p, Trp.p, Tpos.p, A.rp.p, G.EF.p, G.Hs[NL].p, net.pr.p,
+    part.alloc((size_t)std::max<unsigned>(std::max(gw, gh), 1) * (H * (FE + 2) > O_SIZE ? H * (FE + 2) : O_SIZE) + 16);
+    B2S_LAUNCH(ctx, k_head_bwd, gh, 256, 0, n, Lrp.p, Lci.p, Trp.p, Tpos.p, A.rp.p, G.EF.p, G.Hs[NL].p, net.pr.p,
                dC.p, dH.p, part.p);
-    reduce_partials(ctx, gw, O_SIZE, O_SIZE, part.p, net.g.p + OFF_OUT);
-    const uint32_t rows_per = 2048;
+    reduce_partials(ctx, gh, O_SIZE, O_SIZE, part.p, net.g.p + OFF_OUT);
+    // weight gradients: two CTAs an SM, whole passes of 32 rows each
+    const unsigned cta = (unsigned)ctx->sm_count * 2;
+    const uint32_t rows_per = std::max<uint32_t>(32u, ((n + cta - 1) / cta + 31u) / 32u * 32u);
     const unsigned gwb = (n + rows_per - 1) / rows_per;
-    DBuf<float> wpart((size_t)gwb * (2 * H * H + 2 * H) + 16), red(H * (FE + 2));
+    DBuf<float> wpart((size_t)gwb * (2 * H * H) + 16), red(H * (FE + 2));
     for (int l = NL - 1; l >= 0; --l)
     {
         const __nv_bfloat16* Wl = net.pb.p + LAYER0 + l * L_SIZE;
@@ -1456,14 +1511,14 @@ static void train_step(b2s_ctx* ctx, Gnn& net, const CsrDev& A, int nprobes, uin
         reduce_partials(ctx, gw, H * (FE + 2), H * (FE + 2), part.p, red.p);
         B2S_LAUNCH(ctx, k_gate_grads, 1, 64, 0, red.p, gl);
         // weights [W_s; W_m] (128 x 64): dW = dSM^T H_l ; dH_l = dH_{l+1} (the residual) + dSM W
-        B2S_LAUNCH(ctx, (k_linear_bwd_weight<H, 2 * H, true>), gwb, 256, 0, n, rows_per, dSM.p, G.Hs[l].p, wpart.p);
-        reduce_partials(ctx, gwb, 2 * H * H + 2 * H, 2 * H * H, wpart.p, gl + L_WS);
+        B2S_LAUNCH(ctx, (k_linear_bwd_weight<H, 2 * H, true, false>), gwb, 256, 0, n, rows_per, dSM.p, G.Hs[l].p, wpart.p);
+        reduce_partials(ctx, gwb, 2 * H * H, 2 * H * H, wpart.p, gl + L_WS);
         B2S_LAUNCH(ctx, (k_linear_bwd_data<H, 2 * H>), g64, 256, 0, n, dSM.p, Wl + L_WS, dH.p);
     }
     // input layer: dpre0 = dH0 * (pre0 > 0) ; dW_in = dpre0^T F ; db_in
     B2S_LAUNCH(ctx, k_relu_mask, stream_grid(ctx, (uint64_t)n * H), kThreads, 0, (uint64_t)n * H, G.pre0.p, dH.p,
                dSM.p);
-    B2S_LAUNCH(ctx, (k_linear_bwd_weight<FIN, H, false>), gwb, 256, 0, n, rows_per, dSM.p, G.F.p, wpart.p);
+    B2S_LAUNCH(ctx, (k_linear_bwd_weight<FIN, H, false, true>), gwb, 256, 0, n, rows_per, dSM.p, G.F.p, wpart.p);
     reduce_partials(ctx, gwb, H * FIN + H, H * FIN + H, wpart.p, net.g.p + OFF_WIN);
 
     double lossv = 0;
