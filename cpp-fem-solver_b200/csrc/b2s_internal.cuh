@@ -227,6 +227,15 @@ void baij_partition(b2s_ctx* ctx, BaijDev& M, const uint32_t* h_rp);
 // Preconditioner implementation.  apply() enqueues z = M^-1 r on ctx->stream
 // (device pointers).  `done` (device, may be null) lets the Krylov drivers
 // replay work after convergence: every kernel returns at once when *done != 0.
+// An IC(0) factor's device arrays (the preconditioner keeps them): L with the
+// diagonal last in each row, and the strict part of L^T.
+struct Ic0View
+{
+    const uint32_t *Lrp, *Lci, *Trp, *Tci;
+    const double* Lv;
+    uint32_t Lnnz, Tnnz;
+};
+
 struct PcImpl
 {
     virtual ~PcImpl() = default;
@@ -240,6 +249,7 @@ struct PcImpl
     {
         fail(B2S_UNSUPPORTED, "export '" + what + "' not available for this preconditioner");
     }
+    virtual bool ic0_view(Ic0View*) const { return false; }
     // PCG fusion: z = M^-1 r, then rz = r.z and the PCG scalar step
     // (pcg_next) on the device, in the apply's own launches; false (nothing
     // enqueued) when the preconditioner cannot fuse them

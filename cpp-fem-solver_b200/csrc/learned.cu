@@ -1345,29 +1345,18 @@ static void train_step(b2s_ctx* ctx, Gnn& net, const CsrDev& A, int nprobes, uin
     o.factor_sweeps = fsweeps;
     if (fsweeps > 0) o.trsv = B2S_TRSV_JACOBI;  // the fixed-point factor comes with the sweep schedule
     auto base = make_pc_ic0(ctx, A, o);
-    uint64_t sz[3];
-    base->export_data(ctx, "ic0.L", sz, nullptr, nullptr, nullptr);
-    const uint32_t Lnnz = (uint32_t)sz[1];
-    std::vector<uint32_t> hLrp(n + 1), hLci(Lnnz);
-    std::vector<double> hL0(Lnnz);
-    base->export_data(ctx, "ic0.L", sz, hLrp.data(), hLci.data(), hL0.data());
-    base->export_data(ctx, "ic0.LT", sz, nullptr, nullptr, nullptr);
-    const uint32_t Tnnz = (uint32_t)sz[1];
-    std::vector<uint32_t> hTrp(n + 1), hTci(Tnnz ? Tnnz : 1);
-    std::vector<double> hTv(Tnnz ? Tnnz : 1);
-    base->export_data(ctx, "ic0.LT", sz, hTrp.data(), hTci.data(), hTv.data());
-    auto Lrp = upload(ctx, hLrp.data(), n + 1), Lci = upload(ctx, hLci.data(), Lnnz);
-    auto L0 = upload(ctx, hL0.data(), Lnnz);
-    auto Trp = upload(ctx, hTrp.data(), n + 1), Tci = upload(ctx, hTci.data(), hTci.size());
-    DBuf<uint32_t> Tpos(hTci.size());
-    B2S_LAUNCH(ctx, k_lt_positions, stream_grid(ctx, n), kThreads, 0, n, Trp.p, Tci.p, Lrp.p, Lci.p, Tpos.p);
+    Ic0View f;
+    need(base->ic0_view(&f), B2S_UNSUPPORTED, "the base factor is not an IC(0)");
+    const uint32_t Lnnz = f.Lnnz;
+    DBuf<uint32_t> Tpos(f.Tnnz ? f.Tnnz : 1);
+    B2S_LAUNCH(ctx, k_lt_positions, stream_grid(ctx, n), kThreads, 0, n, f.Trp, f.Tci, f.Lrp, f.Lci, Tpos.p);
 
     GnnGraph G;
     G.build(ctx, A, true);
     G.forward(ctx, net, A);
     DBuf<double> Lv(Lnnz), dL(Lnnz);
     DBuf<float> C(Lnnz), dC(Lnnz);
-    G.head(ctx, net, A, Lrp.p, Lci.p, L0.p, Lv.p, C.p, (double*)nullptr);
+    G.head(ctx, net, A, f.Lrp, f.Lci, f.Lv, Lv.p, C.p, (double*)nullptr);
     B2S_CUDA(cudaMemsetAsync(dL.p, 0, dL.bytes(), ctx->stream));
 
     TrainBuffers T;
@@ -1429,10 +1418,10 @@ static void train_step(b2s_ctx* ctx, Gnn& net, const CsrDev& A, int nprobes, uin
             const int K = ksweeps;
             // y = F Aw (k sweeps of L~), z = F^T y (k sweeps of L~^T), e = w - z
             for (int s = 0; s <= K; ++s)
-                B2S_LAUNCH(ctx, k_sw_lo, gn, kThreads, 0, n, Lrp.p, Lci.p, Lv.p, T.Aw.p,
+                B2S_LAUNCH(ctx, k_sw_lo, gn, kThreads, 0, n, f.Lrp, f.Lci, Lv.p, T.Aw.p,
                            s ? ys[s - 1].p : (const double*)nullptr, ys[s].p);
             for (int s = 0; s <= K; ++s)
-                B2S_LAUNCH(ctx, k_sw_up, gn, kThreads, 0, n, Lrp.p, Trp.p, Tci.p, Tpos.p, Lv.p, ys[K].p,
+                B2S_LAUNCH(ctx, k_sw_up, gn, kThreads, 0, n, f.Lrp, f.Trp, f.Tci, Tpos.p, Lv.p, ys[K].p,
                            s ? zs[s - 1].p : (const double*)nullptr, zs[s].p);
             B2S_LAUNCH(ctx, k_sub, gn, kThreads, 0, n, T.w.p, zs[K].p, T.vres.p);
             dot_dev(ctx, n, T.vres.p, T.vres.p, T.scal.p);
@@ -1443,17 +1432,17 @@ static void train_step(b2s_ctx* ctx, Gnn& net, const CsrDev& A, int nprobes, uin
             B2S_CUDA(cudaMemsetAsync(ub.p, 0, ub.bytes(), ctx->stream));
             for (int s = K; s >= 0; --s)
             {
-                B2S_LAUNCH(ctx, k_sw_h, gn, kThreads, 0, n, Lrp.p, Lv.p, gb.p, zs[s].p, hb.p, ub.p, dL.p);
+                B2S_LAUNCH(ctx, k_sw_h, gn, kThreads, 0, n, f.Lrp, Lv.p, gb.p, zs[s].p, hb.p, ub.p, dL.p);
                 if (s == 0) break;
-                B2S_LAUNCH(ctx, k_sw_up_adj, gn, kThreads, 0, n, Lrp.p, Lci.p, Lv.p, hb.p, zs[s - 1].p, gb2.p, dL.p);
+                B2S_LAUNCH(ctx, k_sw_up_adj, gn, kThreads, 0, n, f.Lrp, f.Lci, Lv.p, hb.p, zs[s - 1].p, gb2.p, dL.p);
                 std::swap(gb, gb2);
             }
             // back through the lower sweeps from y_K's adjoint ub (Aw is a constant)
             for (int s = K; s >= 0; --s)
             {
-                B2S_LAUNCH(ctx, k_sw_h, gn, kThreads, 0, n, Lrp.p, Lv.p, ub.p, ys[s].p, hb.p, (double*)nullptr, dL.p);
+                B2S_LAUNCH(ctx, k_sw_h, gn, kThreads, 0, n, f.Lrp, Lv.p, ub.p, ys[s].p, hb.p, (double*)nullptr, dL.p);
                 if (s == 0) break;
-                B2S_LAUNCH(ctx, k_sw_lo_adj, gn, kThreads, 0, n, Trp.p, Tci.p, Tpos.p, Lv.p, hb.p, ys[s - 1].p,
+                B2S_LAUNCH(ctx, k_sw_lo_adj, gn, kThreads, 0, n, f.Trp, f.Tci, Tpos.p, Lv.p, hb.p, ys[s - 1].p,
                            gb2.p, dL.p);
                 std::swap(ub, gb2);
             }
@@ -1472,18 +1461,18 @@ static void train_step(b2s_ctx* ctx, Gnn& net, const CsrDev& A, int nprobes, uin
             B2S_LAUNCH(ctx, k_neg_scale, gn, kThreads, 0, n, T.vres.p, T.scal.p + 2, T.Aw.p);
             M->solve_factor(ctx, false, T.Aw.p, ya.p, nullptr);
             M->solve_factor(ctx, true, ya.p, yb.p, nullptr);
-            B2S_LAUNCH(ctx, k_dL_pc, gn, kThreads, 0, n, Lrp.p, Lci.p, T.qv.p, ya.p, yb.p, T.u.p, dL.p);
+            B2S_LAUNCH(ctx, k_dL_pc, gn, kThreads, 0, n, f.Lrp, f.Lci, T.qv.p, ya.p, yb.p, T.u.p, dL.p);
             continue;
         }
         dot_dev(ctx, n, T.Aw.p, T.Aw.p, T.scal.p + 1);
-        B2S_LAUNCH(ctx, k_ltmul, gn, kThreads, 0, n, Lrp.p, Trp.p, Tci.p, Tpos.p, Lv.p, T.w.p, T.u.p);
-        B2S_LAUNCH(ctx, k_lmul_res, gn, kThreads, 0, n, Lrp.p, Lci.p, Lv.p, T.u.p, T.Aw.p, T.vres.p, T.scal.p,
+        B2S_LAUNCH(ctx, k_ltmul, gn, kThreads, 0, n, f.Lrp, f.Trp, f.Tci, Tpos.p, Lv.p, T.w.p, T.u.p);
+        B2S_LAUNCH(ctx, k_lmul_res, gn, kThreads, 0, n, f.Lrp, f.Lci, Lv.p, T.u.p, T.Aw.p, T.vres.p, T.scal.p,
                    ctx->partial.p, ctx->counter.p);
         B2S_LAUNCH(ctx, k_loss_scale, 1, 1, 0, T.scal.p, T.scal.p + 1, nprobes, T.scal.p + 2, T.scal.p + 3);
-        B2S_LAUNCH(ctx, k_ltmul, gn, kThreads, 0, n, Lrp.p, Trp.p, Tci.p, Tpos.p, Lv.p, T.vres.p, T.qv.p);
-        B2S_LAUNCH(ctx, k_dL, gn, kThreads, 0, n, Lrp.p, Lci.p, T.vres.p, T.u.p, T.w.p, T.qv.p, T.scal.p + 2, dL.p);
+        B2S_LAUNCH(ctx, k_ltmul, gn, kThreads, 0, n, f.Lrp, f.Trp, f.Tci, Tpos.p, Lv.p, T.vres.p, T.qv.p);
+        B2S_LAUNCH(ctx, k_dL, gn, kThreads, 0, n, f.Lrp, f.Lci, T.vres.p, T.u.p, T.w.p, T.qv.p, T.scal.p + 2, dL.p);
     }
-    B2S_LAUNCH(ctx, k_head_dc, stream_grid(ctx, Lnnz), kThreads, 0, Lnnz, dL.p, Lv.p, L0.p, C.p, dC.p);
+    B2S_LAUNCH(ctx, k_head_dc, stream_grid(ctx, Lnnz), kThreads, 0, Lnnz, dL.p, Lv.p, f.Lv, C.p, dC.p);
 
     // backward
     constexpr uint32_t bwd_rows = kTileR * 256 / (H / kTileC);
@@ -1492,7 +1481,7 @@ static void train_step(b2s_ctx* ctx, Gnn& net, const CsrDev& A, int nprobes, uin
     B2S_CUDA(cudaMemsetAsync(net.g.p, 0, net.g.bytes(), ctx->stream));
     DBuf<float> dH(n * (size_t)H), dSM(n * (size_t)2 * H), part;
     part.alloc((size_t)std::max<unsigned>(std::max(gw, gh), 1) * (H * (FE + 2) > O_SIZE ? H * (FE + 2) : O_SIZE) + 16);
-    B2S_LAUNCH(ctx, k_head_bwd, gh, 256, 0, n, Lrp.p, Lci.p, Trp.p, Tpos.p, A.rp.p, G.EF.p, G.Hs[NL].p, net.pr.p,
+    B2S_LAUNCH(ctx, k_head_bwd, gh, 256, 0, n, f.Lrp, f.Lci, f.Trp, Tpos.p, A.rp.p, G.EF.p, G.Hs[NL].p, net.pr.p,
                dC.p, dH.p, part.p);
     reduce_partials(ctx, gh, O_SIZE, O_SIZE, part.p, net.g.p + OFF_OUT);
     // weight gradients: two CTAs an SM, whole passes of 32 rows each

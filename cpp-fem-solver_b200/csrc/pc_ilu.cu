@@ -913,6 +913,12 @@ struct PcIC0 final : PcImpl
         }
     }
 
+    bool ic0_view(Ic0View* v) const override
+    {
+        *v = Ic0View{L.rp.p, L.ci.p, LT.rp.p, LT.ci.p, L.v.p, L.nnz, LT.nnz};
+        return true;
+    }
+
     bool can_fuse_pcg() const override { return fp32 && mode == B2S_TRSV_JACOBI && fwd.band.T && bwd.band.T; }
 
     DBuf<unsigned> pcg_ctl;  // grid-barrier counter, error word
