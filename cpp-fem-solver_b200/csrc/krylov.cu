@@ -19,6 +19,7 @@
 //   gmres    it_end = total Arnoldi steps - 1
 #include <cmath>
 
+#include "grid_sum.cuh"
 #include "spmv_staged.cuh"
 
 namespace b2s {
@@ -648,6 +649,169 @@ __global__ void k_gm_advance(KState* st)
     st->aux[2] += 1.0;
 }
 
+// Column j's modified Gram-Schmidt, norm, Givens step and next basis vector in one
+// cooperative launch of one CTA an SM: the CTA's slice of w stays in registers,
+// V_i comes through two shared-memory buffers (cp.async, V_{i+1} on its way while
+// V_i's dot crosses the grid), and each thread reads only what it copied itself.
+// The arithmetic of every element is BodyGmMgs' and BodyGmNext's; the dots are
+// summed in another fixed order.  A launch a step read and wrote w and read two
+// basis vectors each: 9.3 us a step on 96^3, 495 of them in a 28-iteration solve;
+// here a step reads one vector and costs its sum over the grid, about 3 us (96^3
+// solve 9.4 -> 6.1 ms).  Vectors longer than the SMs hold keep the launch a step.
+constexpr int kMgsThreads = 512;
+
+struct GmMgsArgs
+{
+    uint64_t n, pn;
+    uint32_t chunk;  // elements per CTA (even)
+    const double* w;
+    double* V;  // columns pn apart
+    KState* st;
+    GmSmall sm;
+    int j;
+    unsigned long long* lines;
+    uint32_t epoch;  // the first sum's
+    int* err;
+};
+
+// Q: pairs of elements per thread
+template <int Q>
+__global__ void __launch_bounds__(kMgsThreads, 1) k_gm_mgs(GmMgsArgs a, const int* skip)
+{
+    if (*skip) return;
+    extern __shared__ __align__(16) double mgs_sm[];  // two slices of V
+    __shared__ GridSum<kMgsThreads> gs;
+    if (threadIdx.x == 0) gs.failed = 0;
+    const uint64_t base = (uint64_t)blockIdx.x * a.chunk;
+    const uint32_t count = base < a.n ? (uint32_t)min((uint64_t)a.chunk, a.n - base) : 0u;
+    // pair q of this thread starts at element e(q) of the slice
+    auto e = [&](int q) { return 2u * (threadIdx.x + (uint32_t)q * kMgsThreads); };
+    auto copy = [&](int i) {
+        double* buf = mgs_sm + (size_t)(i & 1) * a.chunk;
+        const double* v = a.V + (size_t)i * a.pn + base;
+#pragma unroll
+        for (int q = 0; q < Q; ++q)
+            if (e(q) < count)  // a last odd element's partner is zero-filled
+                asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(
+                                 (uint32_t)__cvta_generic_to_shared(buf + e(q))),
+                             "l"(v + e(q)), "r"(e(q) + 1u < count ? 16u : 8u)
+                             : "memory");
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    copy(0);
+    if (a.j >= 1)
+        copy(1);
+    double2 w[Q];
+#pragma unroll
+    for (int q = 0; q < Q; ++q)
+    {
+        w[q].x = e(q) < count ? a.w[base + e(q)] : 0.0;
+        w[q].y = e(q) + 1u < count ? a.w[base + e(q) + 1u] : 0.0;
+    }
+    __syncthreads();
+    uint32_t epoch = a.epoch;
+    for (int i = 0; i <= a.j; ++i)
+    {
+        if (i < a.j)
+            asm volatile("cp.async.wait_group 1;" ::: "memory");
+        else
+            asm volatile("cp.async.wait_group 0;" ::: "memory");
+        const double* buf = mgs_sm + (size_t)(i & 1) * a.chunk;
+        double acc = 0.0, h;
+#pragma unroll
+        for (int q = 0; q < Q; ++q)
+            if (e(q) < count)
+            {
+                const double2 v = *reinterpret_cast<const double2*>(buf + e(q));
+                acc += w[q].x * v.x;
+                acc += w[q].y * v.y;
+            }
+        if (!grid_sum(gs, a.lines, epoch++, acc, h, a.err)) return;
+        if (blockIdx.x == 0 && threadIdx.x == 0) a.sm.H[(size_t)i * a.sm.m + a.j] = h;
+#pragma unroll
+        for (int q = 0; q < Q; ++q)
+            if (e(q) < count)
+            {
+                const double2 v = *reinterpret_cast<const double2*>(buf + e(q));
+                w[q].x -= h * v.x;
+                w[q].y -= h * v.y;
+            }
+        if (i + 2 <= a.j) copy(i + 2);
+    }
+    double acc = 0.0, ww;
+#pragma unroll
+    for (int q = 0; q < Q; ++q)
+    {
+        acc += w[q].x * w[q].x;
+        acc += w[q].y * w[q].y;
+    }
+    if (!grid_sum(gs, a.lines, epoch, acc, ww, a.err)) return;
+    const double hn = sqrt(ww);  // gm_column_tail's H[j+1][j]
+    if (hn > kBreak)
+    {
+        double* next = a.V + (size_t)(a.j + 1) * a.pn + base;
+        const double inv = 1.0 / hn;
+#pragma unroll
+        for (int q = 0; q < Q; ++q)
+        {
+            if (e(q) < count) next[e(q)] = w[q].x * inv;
+            if (e(q) + 1u < count) next[e(q) + 1u] = w[q].y * inv;
+        }
+    }
+    if (blockIdx.x == 0 && threadIdx.x == 0)
+    {
+        gm_column_tail(a.st, a.sm, ww);
+        if (!a.st->done) a.st->aux[2] += 1.0;  // k_gm_advance
+    }
+}
+
+// The launches of k_gm_mgs for one solve.
+struct GmMgs
+{
+    bool on = false;
+    uint32_t ctas = 0, chunk = 0, epoch = 1;
+    DBuf<unsigned long long> lines;
+    const void* kern = nullptr;
+    size_t smem = 0;
+
+    GmMgs(b2s_ctx* ctx, uint64_t n, int orth)
+    {
+        if (orth != B2S_ORTH_MGS || !n || n > 0xffffffffull) return;
+        int coop = 0, optin = 0;
+        B2S_CUDA(cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, ctx->device));
+        B2S_CUDA(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, ctx->device));
+        // no more CTAs than have a pair for each thread of a warp
+        ctas = (uint32_t)std::min<uint64_t>((n + 63) / 64, std::min<uint32_t>((uint32_t)ctx->sm_count, kGridSumMaxCtas));
+        chunk = (uint32_t)((n + ctas - 1) / ctas + 1) & ~1u;
+        smem = 2 * (size_t)chunk * sizeof(double);
+        if (!coop || smem + sizeof(GridSum<kMgsThreads>) + 1024 > (size_t)optin) return;
+        const uint32_t q = (chunk / 2 + kMgsThreads - 1) / kMgsThreads;
+        if (q <= 1) kern = (const void*)k_gm_mgs<1>;
+        else if (q <= 3) kern = (const void*)k_gm_mgs<3>;
+        else if (q <= 6) kern = (const void*)k_gm_mgs<6>;
+        else if (q <= 10) kern = (const void*)k_gm_mgs<10>;
+        else if (q <= 14) kern = (const void*)k_gm_mgs<14>;
+        else return;
+        B2S_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        int occ = 0;
+        B2S_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kern, kMgsThreads, smem));
+        if (occ < 1) return;
+        lines.alloc(grid_sum_words(ctas));
+        B2S_CUDA(cudaMemsetAsync(lines.p, 0, lines.bytes(), ctx->stream));
+        on = true;
+    }
+    // column j of w against V (columns pn apart)
+    void run(b2s_ctx* ctx, uint64_t n, uint64_t pn, const double* w, double* V, KState* st, const GmSmall& sm, int j,
+             const int* skip)
+    {
+        GmMgsArgs a{n, pn, chunk, w, V, st, sm, j, lines.p, epoch, ctx->errword()};
+        epoch += (uint32_t)j + 2u;
+        void* params[] = {&a, &skip};
+        B2S_CUDA(cudaLaunchCooperativeKernel(kern, dim3(ctas), dim3(kMgsThreads), params, smem, ctx->stream));
+        note_launch(ctx, "k_gm_mgs");
+    }
+};
+
 // back substitution R y = g (array.cpp:4369-4379)
 __global__ void k_gm_backsub(KState* st, GmSmall sm)
 {
@@ -1066,6 +1230,8 @@ static void run_gmres(Solve& S, const double* b, double* x, b2s_stats* stats, bo
     auto Vj = [&](int j) { return V + pn * (size_t)j; };
     auto Zj = [&](int j) { return Z + pn * (size_t)j; };
 
+    GmMgs mgs(ctx, n, S.o.orth);
+
     S.init_state();
     B2S_CUDA(cudaEventRecord(ctx->ev0, ctx->stream));
     fill(ctx, x, 0.0, n);
@@ -1104,14 +1270,19 @@ static void run_gmres(Solve& S, const double* b, double* x, b2s_stats* stats, bo
                 }
                 launch_vec(ctx, n, g, BodyGmMgs{w, nullptr, nullptr, st, sm, j + 1});
             }
-            else
+            else if (!mgs.on)
             {
                 for (int i = 0; i <= j; ++i)
                     launch_vec(ctx, n, g, BodyGmMgs{w, i > 0 ? Vj(i - 1) : nullptr, Vj(i), st, sm, i});
                 launch_vec(ctx, n, g, BodyGmMgs{w, Vj(j), nullptr, st, sm, j + 1});
             }
-            launch_vec(ctx, n, g, BodyGmNext{Vj(j + 1), w, st});
-            B2S_LAUNCH(ctx, k_gm_advance, 1, 1, 0, st);
+            if (mgs.on)
+                mgs.run(ctx, n, pn, w, V, st, sm, j, g);
+            else
+            {
+                launch_vec(ctx, n, g, BodyGmNext{Vj(j + 1), w, st});
+                B2S_LAUNCH(ctx, k_gm_advance, 1, 1, 0, st);
+            }
             if ((j + 1) % poll == 0 || j + 1 == m)
             {
                 h = S.read_state();

@@ -295,3 +295,19 @@ def test_csr_matmul_shape_error(b2s, ctx):
         M * b2s.SMatrix(3, 3, np.zeros(0), row_ptr=np.zeros(4, np.uint32), col_idx=np.zeros(0, np.uint32))
     P2 = M * M
     assert P2.rows() == n and np.array_equal(M.transpose().col_idx(), ci)
+
+
+@pytest.mark.parametrize("N,restart", [(1, 5), (2, 30), (7, 6), (8, 30), (31, 30), (97, 30)])
+def test_gmres_orthogonalisation_sizes(b2s, ctx, orc, N, restart):
+    """The one-launch Gram-Schmidt column at the sizes where it can go wrong: one
+    row, fewer rows than a warp, an odd count (a slice's last pair half empty),
+    a last CTA with fewer rows than the others, restarts.  GMRES and FGMRES
+    against the restatement."""
+    n, rp, ci, v = P.convdiff2d(N)
+    A, b = b2s.CSR(ctx, n, n, rp, ci, v), b2s.uniform(N, n)
+    xo, io = orc.solve(orc.csr(n, n, rp, ci, v), 2, "none", b, 1e-10, 2000, restart)
+    for method in (b2s.GMRES, b2s.FGMRES):
+        x, st = b2s.solve(ctx, A, b, method, None, tol=1e-10, maxit=2000, restart=restart)
+        assert abs(st["it"] - io) <= 2 and st["relres_true"] < 1e-9
+        # two solutions of relative residual 1e-10, condition numbers below 1e3 at these sizes
+        assert np.linalg.norm(x - xo) <= 1e-7 * np.linalg.norm(xo)
