@@ -1,68 +1,83 @@
 // A sum over all CTAs of a cooperative launch, in a fixed order and without
 // atomics, for persistent kernels that take a scalar step after every pass.
 //
-// Each CTA adds its threads' terms (shuffles, then one warp over the warps) and
-// publishes the total as two 64-bit words {epoch, 32 value bits} in a 128-byte
-// line of its own; thread 32 + b of every CTA polls line b until it carries the
-// epoch, and every warp adds the totals in CTA order, so all threads of the grid
-// hold the same bits after two block barriers.  It is a grid barrier too, but
-// orders no other memory: what the CTAs exchange besides the sum needs its own
-// fences.  Two sets of lines alternate: a CTA writes a set again only after a sum
-// over the other one, which every CTA took part in after it had read this one.
-// A wait ends after kGridSumPolls polls: the CTA records B2S_TIMEOUT and leaves,
-// the others give up at their next sum, and the launch ends.
+// Each CTA adds its threads' terms block by block and publishes the block sums as
+// two 64-bit words {epoch, 32 value bits} each in a 128-byte line of its own;
+// every CTA polls the lines until they carry the epoch and adds the sums in the
+// same order, so all threads of the grid hold the same bits.  It is a grid barrier
+// too, but orders no other memory.  Two sets of lines alternate: a CTA writes a set
+// again only after a sum over the other one, which every CTA took part in after it
+// had read this one.  A wait ends after kGridSumPolls polls: the CTA records
+// B2S_TIMEOUT and leaves, the others give up at their next sum, and the launch ends.
 #pragma once
 #include "b2s_internal.cuh"
 
 namespace b2s {
 
 constexpr unsigned kGridSumPolls = 1u << 21;  // about a second
-constexpr uint32_t kGridSumMaxCtas = 224;  // pollers: threads 32 .. 32 + CTAs - 1 of at least 256
 constexpr uint32_t kGridSumStride = 16;    // words between two CTAs' lines
-
-template <int NT>
-struct GridSum
-{
-    static_assert(NT >= 256 && NT % 32 == 0 && NT <= 1024, "block size");
-    double warp_part[NT / 32];
-    double part[kGridSumMaxCtas];
-    int failed;
-};
 
 // words a launch of `ctas` CTAs needs, zeroed before the epochs start at 1
 inline size_t grid_sum_words(uint32_t ctas) { return 2ull * kGridSumStride * ctas; }
 
-__device__ __forceinline__ double warp_sum_all(double a)
+// The association is that of grid_reduce_last (one value) over a grid of `blocks`
+// blocks of kThreads threads, so that a persistent kernel's dots
+// have the bits of the launch-a-pass kernels'.  Block CTA * vb + 2 s + half is the
+// one whose thread t is this CTA's thread half * kThreads + t with term[s]; a CTA
+// publishes its vb <= 8 block sums in its line.
+constexpr uint32_t kBlockSumMaxBlocks = 8 * 160;
+constexpr int kBlockSumThreads = 2 * kThreads;
+
+struct BlockSum
+{
+    double warp_part[8][kThreads / 32];  // [block of the CTA][warp of the block]
+    double part[kBlockSumMaxBlocks];
+    double last[kThreads / 32];
+    int failed;
+};
+
+// lane 0's sum of grid_reduce_last's shuffle tree
+__device__ __forceinline__ double warp_sum_down(double a)
 {
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) a += __shfl_xor_sync(0xffffffffu, a, o);
+    for (int o = 16; o > 0; o >>= 1) a += __shfl_down_sync(0xffffffffu, a, o);
     return a;
 }
 
-// s.failed must be zero; false (in every thread of the CTA) when a wait gave up
-template <int NT>
-__device__ __forceinline__ bool grid_sum(GridSum<NT>& s, unsigned long long* lines, uint32_t epoch, double term,
-                                         double& sum, int* err)
+template <int S>
+__device__ __forceinline__ bool block_sum(BlockSum& s, unsigned long long* lines, uint32_t epoch, uint32_t blocks,
+                                          uint32_t vb, const double (&term)[S], double& sum, int* err)
 {
-    const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5, ctas = gridDim.x;
-    lines += (size_t)(epoch & 1u) * kGridSumStride * ctas;
-    const double a = warp_sum_all(term);
-    if (lane == 0) s.warp_part[warp] = a;
-    __syncthreads();
-    if (warp == 0)
+    static_assert(S <= 4, "at most 8 blocks a CTA");
+    constexpr uint32_t W = kThreads / 32;
+    const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5, half = tid / kThreads;
+    lines += (size_t)(epoch & 1u) * kGridSumStride * gridDim.x;
+#pragma unroll
+    for (int k = 0; k < S; ++k)
     {
-        const double t = warp_sum_all(lane < NT / 32 ? s.warp_part[lane] : 0.0);
-        if (lane == 0)
+        const double a = warp_sum_down(term[k]);
+        if (lane == 0) s.warp_part[2 * k + half][warp % W] = a;
+    }
+    __syncthreads();
+    if (warp < (2u * S * W + 31u) / 32u)
+    {
+        // eight lanes a block: the tree's last three steps (the wider ones add zeros)
+        const uint32_t b = warp * (32u / W) + lane / W;
+        double a = b < 2u * S ? s.warp_part[b][lane % W] : 0.0;
+#pragma unroll
+        for (int o = W / 2; o > 0; o >>= 1) a += __shfl_down_sync(0xffffffffu, a, o);
+        if (lane % W == 0 && b < vb && blockIdx.x * vb + b < blocks)
         {
-            const unsigned long long e = (unsigned long long)epoch << 32, b = (unsigned long long)__double_as_longlong(t);
-            asm volatile("st.relaxed.gpu.global.v2.u64 [%0], {%1, %2};" ::"l"(lines + (size_t)kGridSumStride * blockIdx.x),
-                         "l"(e | (b & 0xffffffffull)), "l"(e | (b >> 32))
+            const unsigned long long e = (unsigned long long)epoch << 32, w = (unsigned long long)__double_as_longlong(a);
+            asm volatile("st.relaxed.gpu.global.v2.u64 [%0], {%1, %2};" ::"l"(
+                             lines + (size_t)kGridSumStride * blockIdx.x + 2 * b),
+                         "l"(e | (w & 0xffffffffull)), "l"(e | (w >> 32))
                          : "memory");
         }
     }
-    else if (tid - 32u < ctas)
+    for (uint32_t b = tid; b < blocks; b += kBlockSumThreads)
     {
-        const unsigned long long* w = lines + (size_t)kGridSumStride * (tid - 32u);
+        const unsigned long long* w = lines + (size_t)kGridSumStride * (b / vb) + 2u * (b % vb);
         unsigned long long lo = 0, hi = 0;
         bool seen = false;
         for (unsigned polls = 0; polls < kGridSumPolls && !seen; ++polls)
@@ -75,12 +90,19 @@ __device__ __forceinline__ bool grid_sum(GridSum<NT>& s, unsigned long long* lin
             s.failed = 1;
             atomicCAS(err, 0, (int)B2S_TIMEOUT);
         }
-        s.part[tid - 32u] = __longlong_as_double((long long)((hi << 32) | (lo & 0xffffffffull)));
+        s.part[b] = __longlong_as_double((long long)((hi << 32) | (lo & 0xffffffffull)));
     }
     __syncthreads();
-    double t = 0.0;
-    for (uint32_t b = lane; b < ctas; b += 32) t += s.part[b];
-    sum = warp_sum_all(t);
+    if (warp < W)
+    {
+        double a = 0.0;
+        for (uint32_t b = tid; b < blocks; b += kThreads) a += s.part[b];
+        a = warp_sum_down(a);
+        if (lane == 0) s.last[warp] = a;
+    }
+    __syncthreads();
+    static_assert(W == 8, "the tree below");
+    sum = ((s.last[0] + s.last[4]) + (s.last[2] + s.last[6])) + ((s.last[1] + s.last[5]) + (s.last[3] + s.last[7]));
     return s.failed == 0;
 }
 

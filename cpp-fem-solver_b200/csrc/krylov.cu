@@ -101,17 +101,23 @@ __global__ void __launch_bounds__(kThreads) k_vec(uint64_t n, const int* done, B
     }
 }
 
+// one wave: no more CTAs than fit at once (bodies with many sums hold more registers)
 template <typename Body>
-void launch_vec(b2s_ctx* ctx, uint64_t n, const int* done, const Body& body)
+unsigned vec_grid(b2s_ctx* ctx, uint64_t n)
 {
-    // one wave: no more CTAs than fit at once (bodies with many sums hold more registers)
     static const int occ = [] {
         int o = 0;
         if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&o, k_vec<Body>, kThreads, 0) != cudaSuccess) o = 0;
         return o;
     }();
-    unsigned g = stream_grid(ctx, n);
-    if (occ > 0) g = std::min(g, (unsigned)(occ * ctx->sm_count));
+    const unsigned g = stream_grid(ctx, n);
+    return occ > 0 ? std::min(g, (unsigned)(occ * ctx->sm_count)) : g;
+}
+
+template <typename Body>
+void launch_vec(b2s_ctx* ctx, uint64_t n, const int* done, const Body& body)
+{
+    const unsigned g = vec_grid<Body>(ctx, n);
     if (Body::NV > 0) reserve_reduction(ctx, g);
     B2S_LAUNCH(ctx, k_vec<Body>, g, kThreads, 0, n, done, body, ctx->partial.p, ctx->counter.p);
 }
@@ -650,20 +656,21 @@ __global__ void k_gm_advance(KState* st)
 }
 
 // Column j's modified Gram-Schmidt, norm, Givens step and next basis vector in one
-// cooperative launch of one CTA an SM: the CTA's slice of w stays in registers,
+// cooperative launch of one CTA an SM: the CTA's elements of w stay in registers,
 // V_i comes through two shared-memory buffers (cp.async, V_{i+1} on its way while
 // V_i's dot crosses the grid), and each thread reads only what it copied itself.
-// The arithmetic of every element is BodyGmMgs' and BodyGmNext's; the dots are
-// summed in another fixed order.  A launch a step read and wrote w and read two
-// basis vectors each: 9.3 us a step on 96^3, 495 of them in a 28-iteration solve;
-// here a step reads one vector and costs its sum over the grid, about 3 us (96^3
-// solve 9.4 -> 6.1 ms).  Vectors longer than the SMs hold keep the launch a step.
-constexpr int kMgsThreads = 512;
+// The arithmetic of every element is BodyGmMgs' and BodyGmNext's, and the CTAs
+// take the blocks and elements of its launch (block_sum), so the bits are the
+// same.  A launch a step read and wrote w and read two basis vectors each: 9.3 us
+// a step on 96^3, 495 of them in a 28-iteration solve; here a step reads one
+// vector and costs its sum over the grid, about 4 us (96^3 solve 9.4 -> 6.5 ms).
+// Vectors longer than the SMs hold keep the launch a step.
+constexpr int kMgsThreads = kBlockSumThreads;
 
 struct GmMgsArgs
 {
     uint64_t n, pn;
-    uint32_t chunk;  // elements per CTA (even)
+    uint32_t blocks, vb;  // blocks of the launch whose dots are repeated, and per CTA
     const double* w;
     double* V;  // columns pn apart
     KState* st;
@@ -674,39 +681,39 @@ struct GmMgsArgs
     int* err;
 };
 
-// Q: pairs of elements per thread
-template <int Q>
+// S: blocks a thread belongs to, K: elements it has in each
+template <int S, int K>
 __global__ void __launch_bounds__(kMgsThreads, 1) k_gm_mgs(GmMgsArgs a, const int* skip)
 {
     if (*skip) return;
-    extern __shared__ __align__(16) double mgs_sm[];  // two slices of V
-    __shared__ GridSum<kMgsThreads> gs;
-    if (threadIdx.x == 0) gs.failed = 0;
-    const uint64_t base = (uint64_t)blockIdx.x * a.chunk;
-    const uint32_t count = base < a.n ? (uint32_t)min((uint64_t)a.chunk, a.n - base) : 0u;
-    // pair q of this thread starts at element e(q) of the slice
-    auto e = [&](int q) { return 2u * (threadIdx.x + (uint32_t)q * kMgsThreads); };
+    extern __shared__ __align__(16) double mgs_sm[];  // two sets of V's elements
+    __shared__ BlockSum bs;
+    if (threadIdx.x == 0) bs.failed = 0;
+    // element k of this thread in its s-th block (n where there is none)
+    auto at = [&](int s, int k) -> uint64_t {
+        const uint32_t b = 2u * (uint32_t)s + threadIdx.x / kThreads, blk = blockIdx.x * a.vb + b;
+        if (b >= a.vb || blk >= a.blocks) return a.n;
+        return (uint64_t)blk * kThreads + threadIdx.x % kThreads + (uint64_t)k * a.blocks * kThreads;
+    };
     auto copy = [&](int i) {
-        double* buf = mgs_sm + (size_t)(i & 1) * a.chunk;
-        const double* v = a.V + (size_t)i * a.pn + base;
+        const double* v = a.V + (size_t)i * a.pn;
 #pragma unroll
-        for (int q = 0; q < Q; ++q)
-            if (e(q) < count)  // a last odd element's partner is zero-filled
-                asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(
-                                 (uint32_t)__cvta_generic_to_shared(buf + e(q))),
-                             "l"(v + e(q)), "r"(e(q) + 1u < count ? 16u : 8u)
+        for (int q = 0; q < S * K; ++q)
+            if (const uint64_t e = at(q / K, q % K); e < a.n)
+                asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"((uint32_t)__cvta_generic_to_shared(
+                                 mgs_sm + ((i & 1) * S * K + q) * kMgsThreads + threadIdx.x)),
+                             "l"(v + e)
                              : "memory");
         asm volatile("cp.async.commit_group;" ::: "memory");
     };
     copy(0);
-    if (a.j >= 1)
-        copy(1);
-    double2 w[Q];
+    if (a.j >= 1) copy(1);
+    double w[S * K];
 #pragma unroll
-    for (int q = 0; q < Q; ++q)
+    for (int q = 0; q < S * K; ++q)
     {
-        w[q].x = e(q) < count ? a.w[base + e(q)] : 0.0;
-        w[q].y = e(q) + 1u < count ? a.w[base + e(q) + 1u] : 0.0;
+        const uint64_t e = at(q / K, q % K);
+        w[q] = e < a.n ? a.w[e] : 0.0;
     }
     __syncthreads();
     uint32_t epoch = a.epoch;
@@ -716,47 +723,34 @@ __global__ void __launch_bounds__(kMgsThreads, 1) k_gm_mgs(GmMgsArgs a, const in
             asm volatile("cp.async.wait_group 1;" ::: "memory");
         else
             asm volatile("cp.async.wait_group 0;" ::: "memory");
-        const double* buf = mgs_sm + (size_t)(i & 1) * a.chunk;
-        double acc = 0.0, h;
+        const double* v = mgs_sm + (size_t)(i & 1) * S * K * kMgsThreads + threadIdx.x;
+        double acc[S], h;
 #pragma unroll
-        for (int q = 0; q < Q; ++q)
-            if (e(q) < count)
-            {
-                const double2 v = *reinterpret_cast<const double2*>(buf + e(q));
-                acc += w[q].x * v.x;
-                acc += w[q].y * v.y;
-            }
-        if (!grid_sum(gs, a.lines, epoch++, acc, h, a.err)) return;
+        for (int s = 0; s < S; ++s) acc[s] = 0.0;
+#pragma unroll
+        for (int q = 0; q < S * K; ++q)
+            if (at(q / K, q % K) < a.n) acc[q / K] += w[q] * v[q * kMgsThreads];
+        if (!block_sum(bs, a.lines, epoch++, a.blocks, a.vb, acc, h, a.err)) return;
         if (blockIdx.x == 0 && threadIdx.x == 0) a.sm.H[(size_t)i * a.sm.m + a.j] = h;
 #pragma unroll
-        for (int q = 0; q < Q; ++q)
-            if (e(q) < count)
-            {
-                const double2 v = *reinterpret_cast<const double2*>(buf + e(q));
-                w[q].x -= h * v.x;
-                w[q].y -= h * v.y;
-            }
+        for (int q = 0; q < S * K; ++q)
+            if (at(q / K, q % K) < a.n) w[q] -= h * v[q * kMgsThreads];
         if (i + 2 <= a.j) copy(i + 2);
     }
-    double acc = 0.0, ww;
+    double acc[S], ww;
 #pragma unroll
-    for (int q = 0; q < Q; ++q)
-    {
-        acc += w[q].x * w[q].x;
-        acc += w[q].y * w[q].y;
-    }
-    if (!grid_sum(gs, a.lines, epoch, acc, ww, a.err)) return;
+    for (int s = 0; s < S; ++s) acc[s] = 0.0;
+#pragma unroll
+    for (int q = 0; q < S * K; ++q)
+        if (at(q / K, q % K) < a.n) acc[q / K] += w[q] * w[q];
+    if (!block_sum(bs, a.lines, epoch, a.blocks, a.vb, acc, ww, a.err)) return;
     const double hn = sqrt(ww);  // gm_column_tail's H[j+1][j]
     if (hn > kBreak)
     {
-        double* next = a.V + (size_t)(a.j + 1) * a.pn + base;
-        const double inv = 1.0 / hn;
+        double* next = a.V + (size_t)(a.j + 1) * a.pn;
 #pragma unroll
-        for (int q = 0; q < Q; ++q)
-        {
-            if (e(q) < count) next[e(q)] = w[q].x * inv;
-            if (e(q) + 1u < count) next[e(q) + 1u] = w[q].y * inv;
-        }
+        for (int q = 0; q < S * K; ++q)
+            if (const uint64_t e = at(q / K, q % K); e < a.n) next[e] = w[q] * (1.0 / hn);
     }
     if (blockIdx.x == 0 && threadIdx.x == 0)
     {
@@ -769,29 +763,29 @@ __global__ void __launch_bounds__(kMgsThreads, 1) k_gm_mgs(GmMgsArgs a, const in
 struct GmMgs
 {
     bool on = false;
-    uint32_t ctas = 0, chunk = 0, epoch = 1;
+    uint32_t blocks = 0, vb = 0, ctas = 0, epoch = 1;
     DBuf<unsigned long long> lines;
     const void* kern = nullptr;
     size_t smem = 0;
 
     GmMgs(b2s_ctx* ctx, uint64_t n, int orth)
     {
-        if (orth != B2S_ORTH_MGS || !n || n > 0xffffffffull) return;
+        if (orth != B2S_ORTH_MGS || !n) return;
         int coop = 0, optin = 0;
         B2S_CUDA(cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, ctx->device));
         B2S_CUDA(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, ctx->device));
-        // no more CTAs than have a pair for each thread of a warp
-        ctas = (uint32_t)std::min<uint64_t>((n + 63) / 64, std::min<uint32_t>((uint32_t)ctx->sm_count, kGridSumMaxCtas));
-        chunk = (uint32_t)((n + ctas - 1) / ctas + 1) & ~1u;
-        smem = 2 * (size_t)chunk * sizeof(double);
-        if (!coop || smem + sizeof(GridSum<kMgsThreads>) + 1024 > (size_t)optin) return;
-        const uint32_t q = (chunk / 2 + kMgsThreads - 1) / kMgsThreads;
-        if (q <= 1) kern = (const void*)k_gm_mgs<1>;
-        else if (q <= 3) kern = (const void*)k_gm_mgs<3>;
-        else if (q <= 6) kern = (const void*)k_gm_mgs<6>;
-        else if (q <= 10) kern = (const void*)k_gm_mgs<10>;
-        else if (q <= 14) kern = (const void*)k_gm_mgs<14>;
-        else return;
+        blocks = vec_grid<BodyGmMgs>(ctx, n);
+        vb = (blocks + (uint32_t)ctx->sm_count - 1) / (uint32_t)ctx->sm_count;
+        ctas = (blocks + vb - 1) / vb;
+        const uint64_t k = (n + (uint64_t)blocks * kThreads - 1) / ((uint64_t)blocks * kThreads);
+        if (!coop || vb > 8 || blocks > kBlockSumMaxBlocks || k > 6) return;
+        const int s = vb <= 2 ? 1 : vb <= 4 ? 2 : 4;
+        const void* const wide[6] = {(const void*)k_gm_mgs<4, 1>, (const void*)k_gm_mgs<4, 2>, (const void*)k_gm_mgs<4, 3>,
+                                     (const void*)k_gm_mgs<4, 4>, (const void*)k_gm_mgs<4, 5>, (const void*)k_gm_mgs<4, 6>};
+        if (s < 4 && k > 1) return;  // (a grid of that few blocks has an element a thread)
+        kern = s == 4 ? wide[k - 1] : s == 2 ? (const void*)k_gm_mgs<2, 1> : (const void*)k_gm_mgs<1, 1>;
+        smem = 2 * (size_t)s * k * kMgsThreads * sizeof(double);
+        if (smem + sizeof(BlockSum) + 1024 > (size_t)optin) return;
         B2S_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
         int occ = 0;
         B2S_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kern, kMgsThreads, smem));
@@ -804,7 +798,7 @@ struct GmMgs
     void run(b2s_ctx* ctx, uint64_t n, uint64_t pn, const double* w, double* V, KState* st, const GmSmall& sm, int j,
              const int* skip)
     {
-        GmMgsArgs a{n, pn, chunk, w, V, st, sm, j, lines.p, epoch, ctx->errword()};
+        GmMgsArgs a{n, pn, blocks, vb, w, V, st, sm, j, lines.p, epoch, ctx->errword()};
         epoch += (uint32_t)j + 2u;
         void* params[] = {&a, &skip};
         B2S_CUDA(cudaLaunchCooperativeKernel(kern, dim3(ctas), dim3(kMgsThreads), params, smem, ctx->stream));
