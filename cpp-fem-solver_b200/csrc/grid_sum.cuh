@@ -1,27 +1,123 @@
 // A sum over all CTAs of a cooperative launch, in a fixed order and without
 // atomics, for persistent kernels that take a scalar step after every pass.
 //
-// Each CTA adds its threads' terms block by block and publishes the block sums as
-// two 64-bit words {epoch, 32 value bits} each in a 128-byte line of its own;
-// every CTA polls the lines until they carry the epoch and adds the sums in the
-// same order, so all threads of the grid hold the same bits.  It is a grid barrier
-// too, but orders no other memory.  Two sets of lines alternate: a CTA writes a set
-// again only after a sum over the other one, which every CTA took part in after it
-// had read this one.  A wait ends after kGridSumPolls polls: the CTA records
-// B2S_TIMEOUT and leaves, the others give up at their next sum, and the launch ends.
+// Each CTA adds its threads' terms (shuffles, then over the warps) and publishes
+// the totals as two 64-bit words {epoch, 32 value bits} each in a 128-byte line of
+// its own; threads of every CTA poll the lines until they carry the epoch, and
+// the totals are added in CTA order, so all threads of the grid hold the same
+// bits.  It is a grid barrier too, but orders no other memory: what the CTAs
+// exchange besides carries the epoch in its own words.  Two sets of lines
+// alternate: a CTA writes a set again only after a sum over the other one, which
+// every CTA took part in after it had read this one.  A wait ends after
+// kGridSumPolls polls: the CTA records B2S_TIMEOUT and leaves, the others give up
+// at their next sum, and the launch ends.
+//
+// It costs two trips through L2 and their spread over the SMs, about 2 us on 148
+// CTAs.  A line for every pair of CTAs instead of one polled by all was no faster
+// (5,000 cycles against 4,000); ordering other stores by fences made it 8,200.
 #pragma once
 #include "b2s_internal.cuh"
 
 namespace b2s {
 
 constexpr unsigned kGridSumPolls = 1u << 21;  // about a second
+constexpr uint32_t kGridSumMaxCtas = 224;  // pollers: threads 32 .. 32 + CTAs - 1 of at least 256
 constexpr uint32_t kGridSumStride = 16;    // words between two CTAs' lines
 
-// words a launch of `ctas` CTAs needs, zeroed before the epochs start at 1
-inline size_t grid_sum_words(uint32_t ctas) { return 2ull * kGridSumStride * ctas; }
+template <int NT, int NV = 1>
+struct GridSum
+{
+    static_assert(NT >= 256 && NT % 32 == 0 && NT <= 1024 && 2 * NV <= (int)kGridSumStride, "block size, line");
+    double warp_part[NV][NT / 32];
+    double part[NV][kGridSumMaxCtas];
+    int failed;
+};
 
-// The association is that of grid_reduce_last (one value) over a grid of `blocks`
-// blocks of kThreads threads, so that a persistent kernel's dots
+// words a launch of `ctas` CTAs needs, zeroed before the epochs start at 1
+__host__ __device__ inline size_t grid_sum_words(uint32_t ctas) { return 2ull * kGridSumStride * ctas; }
+
+__device__ __forceinline__ double warp_sum_all(double a)
+{
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) a += __shfl_xor_sync(0xffffffffu, a, o);
+    return a;
+}
+
+// Publishes the CTA's terms (between this and grid_sum_wait a thread may do other
+// work; s.failed must be zero at the first).
+template <int NT, int NV>
+__device__ __forceinline__ void grid_sum_post(GridSum<NT, NV>& s, unsigned long long* lines, uint32_t epoch,
+                                              const double (&term)[NV])
+{
+    const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+    lines += ((size_t)(epoch & 1u) * gridDim.x + blockIdx.x) * kGridSumStride;
+#pragma unroll
+    for (int v = 0; v < NV; ++v)
+    {
+        const double a = warp_sum_all(term[v]);
+        if (lane == 0) s.warp_part[v][warp] = a;
+    }
+    __syncthreads();
+    if (warp != 0) return;
+    const unsigned long long e = (unsigned long long)epoch << 32;
+#pragma unroll
+    for (int v = 0; v < NV; ++v)
+    {
+        const double t = warp_sum_all(lane < NT / 32 ? s.warp_part[v][lane] : 0.0);
+        const unsigned long long b = (unsigned long long)__double_as_longlong(t);
+        if (lane == 0)
+            asm volatile("st.relaxed.gpu.global.v2.u64 [%0], {%1, %2};" ::"l"(lines + 2 * v),
+                         "l"(e | (b & 0xffffffffull)), "l"(e | (b >> 32))
+                         : "memory");
+    }
+}
+
+// The sums; false (in every thread of the CTA) when a wait gave up.
+template <int NT, int NV>
+__device__ __forceinline__ bool grid_sum_wait(GridSum<NT, NV>& s, const unsigned long long* lines, uint32_t epoch,
+                                              double (&sum)[NV], int* err)
+{
+    const uint32_t tid = threadIdx.x, lane = tid & 31u, ctas = gridDim.x;
+    if (tid - 32u < ctas)  // (the first warp publishes)
+    {
+        const unsigned long long* w = lines + ((size_t)(epoch & 1u) * ctas + (tid - 32u)) * kGridSumStride;
+        unsigned long long lo[NV], hi[NV];
+        bool seen = false;
+        for (unsigned polls = 0; polls < kGridSumPolls && !seen; ++polls)
+        {
+            seen = true;
+#pragma unroll
+            for (int v = 0; v < NV; ++v)
+                asm volatile("ld.relaxed.gpu.global.v2.u64 {%0, %1}, [%2];"
+                             : "=l"(lo[v]), "=l"(hi[v])
+                             : "l"(w + 2 * v)
+                             : "memory");
+#pragma unroll
+            for (int v = 0; v < NV; ++v)
+                seen = seen && (uint32_t)(lo[v] >> 32) == epoch && (uint32_t)(hi[v] >> 32) == epoch;
+        }
+        if (!seen)
+        {
+            s.failed = 1;
+            atomicCAS(err, 0, (int)B2S_TIMEOUT);
+        }
+#pragma unroll
+        for (int v = 0; v < NV; ++v)
+            s.part[v][tid - 32u] = __longlong_as_double((long long)((hi[v] << 32) | (lo[v] & 0xffffffffull)));
+    }
+    __syncthreads();
+#pragma unroll
+    for (int v = 0; v < NV; ++v)
+    {
+        double t = 0.0;
+        for (uint32_t b = lane; b < ctas; b += 32) t += s.part[v][b];
+        sum[v] = warp_sum_all(t);
+    }
+    return s.failed == 0;
+}
+
+// The same exchange with the association of grid_reduce_last (one value) over a
+// grid of `blocks` blocks of kThreads threads, so that a persistent kernel's dots
 // have the bits of the launch-a-pass kernels'.  Block CTA * vb + 2 s + half is the
 // one whose thread t is this CTA's thread half * kThreads + t with term[s]; a CTA
 // publishes its vb <= 8 block sums in its line.

@@ -288,6 +288,272 @@ struct BodyPUpdate  // p = z + beta p (array.cpp:3590-3593)
     __device__ void last(const double*) const {}
 };
 
+// The whole loop of a PCG without or with a diagonal preconditioner in one
+// cooperative launch, for banded CSR operators of short rows that the SMs' shared
+// memory holds.  A CTA keeps its rows of A in shared memory, their x, r, z, p and d
+// in registers, and p over its rows' band, [r0 - band, r1 + band), in shared
+// memory: every CTA forms p = z + beta p_old for the rows of others that it reads
+// itself, from their z, which their owner leaves as epoch-tagged words.  So an
+// iteration exchanges z and two sums, and the product reads shared memory alone.
+// The arithmetic of a row is EpiPAp's and BodyPcgUpdate's; the dots are summed in
+// another fixed order.  Bound by the two sums (grid_sum.cuh): 256^2 16 us an
+// iteration as three launches, 4.7 us here (8.2 with z and p read back through L2 behind
+// fences).
+constexpr int kPcgSmallThreads = 512;
+constexpr int kPcgSmallRows = 4;   // rows per thread at most
+constexpr int kPcgSmallHalo = 8;   // band entries of other CTAs per thread at most
+
+struct PcgSmallArgs
+{
+    uint32_t n, rows, band;  // rows per CTA; largest |i - j|
+    const uint32_t *rp, *ci;
+    const double *v, *d;  // d: the diagonal (null: no preconditioner)
+    double* x;
+    const double *r, *z, *p;    // the state before the first iteration
+    unsigned long long* zw;     // z as words, two a row, zero at launch
+    unsigned long long* lines;  // two regions of grid_sum_words
+    KState* st;
+    int* err;
+};
+
+// the largest |i - j| of a pattern
+__global__ void __launch_bounds__(kThreads) k_csr_band(uint32_t n, const uint32_t* __restrict__ rp,
+                                                       const uint32_t* __restrict__ ci, uint32_t* band)
+{
+    uint32_t b = 0;
+    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
+    {
+        const uint32_t e0 = rp[i], e1 = rp[i + 1];
+        if (e1 > e0) b = max(b, max(i > ci[e0] ? i - ci[e0] : 0u, ci[e1 - 1] > i ? ci[e1 - 1] - i : 0u));  // columns ascend
+    }
+    b = __reduce_max_sync(0xffffffffu, b);
+    if ((threadIdx.x & 31u) == 0 && b) atomicMax(band, b);
+}
+
+template <int Q>
+__global__ void __launch_bounds__(kPcgSmallThreads, 1) k_pcg_small(PcgSmallArgs a)
+{
+    constexpr uint32_t NT = kPcgSmallThreads;
+    constexpr int HQ = kPcgSmallHalo;
+    extern __shared__ __align__(16) double pcg_sm[];
+    __shared__ GridSum<NT, 1> g1;
+    __shared__ GridSum<NT, 2> g2;
+    __shared__ KState sst;
+    const uint32_t tid = threadIdx.x, r0 = min(blockIdx.x * a.rows, a.n), rows = min(a.rows, a.n - r0);
+    const uint32_t lo = r0 > a.band ? r0 - a.band : 0u, hi = min(a.n, r0 + rows + a.band);  // columns this CTA reads
+    const uint32_t own = r0 - lo, halo = hi - lo - rows;
+    const uint32_t e0 = a.rp[r0], ne = a.rp[r0 + rows] - e0;
+    double* const pw = pcg_sm;                           // p of columns lo .. hi - 1
+    double* const av = pw + a.rows + 2u * a.band;        // the rows' values, columns - lo, offsets
+    uint32_t* const ac = reinterpret_cast<uint32_t*>(av + ne);
+    uint32_t* const ap = ac + ne;
+    for (uint32_t i = tid; i < ne; i += NT)
+    {
+        av[i] = a.v[e0 + i];
+        ac[i] = a.ci[e0 + i] - lo;
+    }
+    for (uint32_t i = tid; i <= rows; i += NT) ap[i] = a.rp[r0 + i] - e0;
+    if (tid == 0)
+    {
+        sst = *a.st;
+        g1.failed = 0;
+        g2.failed = 0;
+    }
+    double x[Q], r[Q], p[Q], z[Q], d[Q], Ap[Q], zh[HQ];
+#pragma unroll
+    for (int q = 0; q < Q; ++q)
+    {
+        const uint32_t t = tid + (uint32_t)q * NT;
+        const bool on = t < rows;
+        x[q] = on ? a.x[r0 + t] : 0.0;
+        r[q] = on ? a.r[r0 + t] : 0.0;
+        p[q] = on ? a.p[r0 + t] : 0.0;
+        z[q] = on ? a.z[r0 + t] : 0.0;
+        d[q] = on && a.d ? a.d[r0 + t] : 1.0;
+    }
+    // entry k of the band's rows of other CTAs: its place in pw
+    auto place = [&](int k) {
+        const uint32_t h = tid + (uint32_t)k * NT;
+        return h < own ? h : h + rows;
+    };
+#pragma unroll
+    for (int k = 0; k < HQ; ++k)
+        if (tid + (uint32_t)k * NT < halo)
+        {
+            pw[place(k)] = a.p[lo + place(k)];
+            zh[k] = a.z[lo + place(k)];
+        }
+    __syncthreads();
+    const bool any = !sst.done;
+    double beta = sst.beta, rz_old = sst.rz_old, rr = 0.0;
+    int it = sst.it;
+    const int maxit = sst.maxit;
+    // r.r above this is a relative residual above tol, whatever the roundings of the
+    // square root and the quotient that decide below it
+    const double clear = sst.tol * sst.normb * (sst.tol * sst.normb) * (1.0 + 1e-12);
+    uint32_t epoch = 0;
+    while (any)
+    {
+#pragma unroll
+        for (int q = 0; q < Q; ++q)
+        {
+            const uint32_t t = tid + (uint32_t)q * NT;
+            p[q] = z[q] + beta * p[q];
+            if (t < rows) pw[own + t] = p[q];
+        }
+#pragma unroll
+        for (int k = 0; k < HQ; ++k)
+            if (tid + (uint32_t)k * NT < halo) pw[place(k)] = zh[k] + beta * pw[place(k)];
+        __syncthreads();
+        double one[1] = {0.0}, pAp[1];
+#pragma unroll
+        for (int q = 0; q < Q; ++q)
+        {
+            const uint32_t t = tid + (uint32_t)q * NT;
+            if (t >= rows) continue;
+            double sum = 0.0;
+            const uint32_t i1 = ap[t + 1];
+#pragma unroll 4
+            for (uint32_t i = ap[t]; i < i1; ++i) sum += av[i] * pw[ac[i]];
+            Ap[q] = sum;
+            one[0] += p[q] * sum;
+        }
+        ++epoch;
+        grid_sum_post(g1, a.lines, epoch, one);
+        if (!grid_sum_wait(g1, a.lines, epoch, pAp, a.err)) break;
+        if (!(pAp[0] >= kBreak))  // breakdown, not SPD or NaN: the state's own test decides
+        {
+            __syncthreads();
+            if (tid == 0)
+            {
+                sst.it = it;
+                sst.rz_old = rz_old;
+                if (it > 0)  // as the steps before left them
+                {
+                    sst.it_end = it - 1;
+                    sst.iters = it;
+                    sst.normr = sqrt(rr);
+                    sst.relres = sst.normr / sst.normb;
+                }
+                EpiPAp{nullptr, nullptr, &sst}.last(pAp);
+            }
+            __syncthreads();
+            if (sst.done) break;
+        }
+        const double alpha = rz_old / pAp[0];
+        double two[2] = {0.0, 0.0}, tot[2];
+#pragma unroll
+        for (int q = 0; q < Q; ++q)
+        {
+            const uint32_t t = tid + (uint32_t)q * NT;
+            if (t >= rows) continue;
+            x[q] += alpha * p[q];
+            r[q] = r[q] - alpha * Ap[q];
+            z[q] = a.d ? r[q] / d[q] : r[q];
+            const unsigned long long e = (unsigned long long)epoch << 32, b = (unsigned long long)__double_as_longlong(z[q]);
+            asm volatile("st.relaxed.gpu.global.v2.u64 [%0], {%1, %2};" ::"l"(a.zw + 2 * (size_t)(r0 + t)),
+                         "l"(e | (b & 0xffffffffull)), "l"(e | (b >> 32))
+                         : "memory");
+            two[0] += r[q] * r[q];
+            two[1] += r[q] * z[q];
+        }
+        grid_sum_post(g2, a.lines + grid_sum_words(gridDim.x), epoch, two);
+        // the others' z while the sum crosses the grid
+#pragma unroll
+        for (int k = 0; k < HQ; ++k)
+            if (tid + (uint32_t)k * NT < halo)
+            {
+                unsigned long long wl = 0, wh = 0;
+                bool seen = false;
+                for (unsigned polls = 0; polls < kGridSumPolls && !seen; ++polls)
+                {
+                    asm volatile("ld.relaxed.gpu.global.v2.u64 {%0, %1}, [%2];"
+                                 : "=l"(wl), "=l"(wh)
+                                 : "l"(a.zw + 2 * (size_t)(lo + place(k)))
+                                 : "memory");
+                    seen = (uint32_t)(wl >> 32) == epoch && (uint32_t)(wh >> 32) == epoch;
+                }
+                if (!seen)
+                {
+                    g2.failed = 1;
+                    atomicCAS(a.err, 0, (int)B2S_TIMEOUT);
+                }
+                zh[k] = __longlong_as_double((long long)((wh << 32) | (wl & 0xffffffffull)));
+            }
+        if (!grid_sum_wait(g2, a.lines + grid_sum_words(gridDim.x), epoch, tot, a.err)) break;
+        rr = tot[0];
+        if (tot[0] > clear && tot[0] < HUGE_VAL && tot[1] > 0.0 && it + 1 < maxit)
+        {
+            beta = tot[1] / rz_old;
+            rz_old = tot[1];
+            ++it;
+            continue;
+        }
+        __syncthreads();
+        if (tid == 0)
+        {
+            sst.it = it;
+            sst.it_end = it > 0 ? it - 1 : 0;
+            sst.alpha = alpha;
+            sst.pAp = pAp[0];
+            sst.rz_old = rz_old;
+            if (!pcg_check_converged(&sst, tot[0])) pcg_next(&sst, tot[1]);
+        }
+        __syncthreads();
+        if (sst.done) break;
+        beta = sst.beta;
+        rz_old = sst.rz_old;
+        it = sst.it;
+    }
+#pragma unroll
+    for (int q = 0; q < Q; ++q)
+    {
+        const uint32_t t = tid + (uint32_t)q * NT;
+        if (t < rows) a.x[r0 + t] = x[q];
+    }
+    if (blockIdx.x == 0 && tid == 0) *a.st = sst;
+}
+
+// Runs the loop from the state before the first iteration; false, with nothing
+// of it enqueued, when the operator does not fit.
+static bool pcg_small(b2s_ctx* ctx, const CsrDev& A, const double* d, double* x, const double* r, const double* z,
+                      const double* p, KState* st)
+{
+    if (!spmv_by_rows(A)) return false;
+    int coop = 0, optin = 0;
+    B2S_CUDA(cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, ctx->device));
+    B2S_CUDA(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, ctx->device));
+    constexpr uint32_t NT = kPcgSmallThreads;
+    // at least 256 rows a CTA: fewer leave more CTAs to sum over than work for them
+    const uint32_t ctas = std::min((A.n + 255u) / 256u, std::min((uint32_t)ctx->sm_count, kGridSumMaxCtas));
+    const uint32_t rows = (A.n + ctas - 1) / ctas;
+    // a CTA's entries: every row at its longest
+    const size_t base = (size_t)rows * 8 + (size_t)rows * A.max_row * 12 + ((size_t)rows + 1) * 4 + 12288;
+    if (!coop || rows > NT * kPcgSmallRows || base > (size_t)optin) return false;
+    DBuf<uint32_t> band_d(1);
+    B2S_CUDA(cudaMemsetAsync(band_d.p, 0, sizeof(uint32_t), ctx->stream));
+    B2S_LAUNCH(ctx, k_csr_band, stream_grid(ctx, A.n), kThreads, 0, A.n, A.rp.p, A.ci.p, band_d.p);
+    uint32_t band = 0;
+    d2h(ctx, &band, band_d.p, sizeof(band));
+    sync(ctx);
+    if (2ull * band > (uint64_t)NT * kPcgSmallHalo || base + 16ull * band > (size_t)optin) return false;
+    const size_t smem = base - 12288 + 16 * (size_t)band;
+    const uint32_t q = (rows + NT - 1) / NT;
+    const void* kern = q <= 1 ? (const void*)k_pcg_small<1> : q == 2 ? (const void*)k_pcg_small<2> : (const void*)k_pcg_small<4>;
+    B2S_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    int occ = 0;
+    B2S_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kern, NT, smem));
+    if (occ < 1) return false;
+    DBuf<unsigned long long> words(2 * grid_sum_words(ctas) + 2 * (size_t)A.n);
+    B2S_CUDA(cudaMemsetAsync(words.p, 0, words.bytes(), ctx->stream));
+    unsigned long long* zw = words.p + 2 * grid_sum_words(ctas);
+    PcgSmallArgs a{A.n, rows, band, A.rp.p, A.ci.p, A.v.p, d, x, r, z, p, zw, words.p, st, ctx->errword()};
+    void* params[] = {&a};
+    B2S_CUDA(cudaLaunchCooperativeKernel(kern, dim3(ctas), dim3(NT), params, smem, ctx->stream));
+    note_launch(ctx, "k_pcg_small");
+    return true;
+}
+
 // ---------------------------------------------------------------- BiCGSTAB
 
 // speculative rho for the next iteration + the checks of array.cpp:3694-3716
@@ -1114,6 +1380,9 @@ static void run_pcg(Solve& S, const double* b, double* x, b2s_stats* stats)
             };
             S.loop(body);
         }
+        else if (fuse != 0 && S.A.csr && S.o.persistent != 2 && S.stall_window <= 0 &&
+                 pcg_small(ctx, *S.A.csr, dfuse, x, r, z, p, st))
+            ;  // the whole loop is on the stream
         else
         {
         auto body = [&] {

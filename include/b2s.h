@@ -386,7 +386,9 @@ typedef struct b2s_solve_opts
                          continues with plain FP64 IC(0) from its iterate (b2s_stats.fallbacks) */
     int persistent;   /* PCG with an FP32 IC(0)-type preconditioner applied by plain Jacobi sweeps:
                          0 = the whole loop in one launch, over 2-D tiles when they can be planned,
-                         else over row strips; 1 = row strips only; 2 = three launches per iteration */
+                         else over row strips; 1 = row strips only; 2 = three launches per iteration.
+                         PCG without or with the diagonal preconditioner on a CSR operator that the
+                         SMs' shared memory holds: one launch, 2 = three launches per iteration */
 } b2s_solve_opts;
 
 void b2s_solve_opts_default(b2s_solve_opts* opts);

@@ -311,3 +311,27 @@ def test_gmres_orthogonalisation_sizes(b2s, ctx, orc, N, restart):
         assert abs(st["it"] - io) <= 2 and st["relres_true"] < 1e-9
         # two solutions of relative residual 1e-10, condition numbers below 1e3 at these sizes
         assert np.linalg.norm(x - xo) <= 1e-7 * np.linalg.norm(xo)
+
+
+@pytest.mark.parametrize("pc", ["none", "diag"])
+@pytest.mark.parametrize("nx,ny,nz", [(1, 1, 1), (16, 16, 1), (257, 1, 1), (199, 190, 1), (41, 37, 29), (67, 64, 63)])
+def test_pcg_one_launch_sizes(b2s, ctx, orc, pc, nx, ny, nz):
+    """The one-launch PCG loop against the launch-by-launch one and the
+    restatement: one row, exactly one CTA, one row more, one to four rows a
+    thread, a last CTA with fewer rows."""
+    if nz > 1:
+        n, rp, ci, v = P.diffusion3d(nx, ny, nz, seed=nx)
+    elif ny > 1:
+        n, rp, ci, v = P.diffusion2d(nx, ny, seed=nx)
+    else:  # a chain
+        n, rp, ci, v = nx, *P.coo_to_csr(nx, nx, *zip(*[(i, j, 2.5 if i == j else -1.0) for i in range(nx)
+                                                        for j in (i - 1, i, i + 1) if 0 <= j < nx]))
+    A, b = b2s.CSR(ctx, n, n, rp, ci, v), b2s.uniform(nx + nz, n)
+    M = b2s.Precond(ctx, A, b2s.PC_DIAG) if pc == "diag" else None
+    got = [b2s.solve(ctx, A, b, b2s.PCG, M, tol=1e-8, maxit=5000, persistent=k) for k in (b2s.PERSIST_AUTO, b2s.PERSIST_OFF)]
+    xo, io = orc.solve(orc.csr(n, n, rp, ci, v), 0, pc, b, 1e-8, 5000)
+    for x, st in got:
+        assert st["status"] == 0 and st["relres_true"] < 2e-8
+        # iteration counts by the association of the dots alone; solutions of the same relative residual
+        assert abs(st["it"] - io) <= max(2, io // 50)
+        assert np.linalg.norm(x - xo) <= 1e-5 * np.linalg.norm(xo)
