@@ -21,9 +21,10 @@
 namespace b2s {
 
 constexpr unsigned kGridSumPolls = 1u << 21;  // about a second
-constexpr uint32_t kGridSumMaxCtas = 224;  // pollers: threads 32 .. 32 + CTAs - 1 of at least 256
+constexpr uint32_t kGridSumMaxCtas = 160;  // pollers: threads 32 .. 32 + CTAs - 1 of at least 256
 constexpr uint32_t kGridSumStride = 16;    // words between two CTAs' lines
 
+// room for sums of up to NV values; one struct serves sum after sum
 template <int NT, int NV = 1>
 struct GridSum
 {
@@ -45,8 +46,8 @@ __device__ __forceinline__ double warp_sum_all(double a)
 
 // Publishes the CTA's terms (between this and grid_sum_wait a thread may do other
 // work; s.failed must be zero at the first).
-template <int NT, int NV>
-__device__ __forceinline__ void grid_sum_post(GridSum<NT, NV>& s, unsigned long long* lines, uint32_t epoch,
+template <int NT, int ROOM, int NV>
+__device__ __forceinline__ void grid_sum_post(GridSum<NT, ROOM>& s, unsigned long long* lines, uint32_t epoch,
                                               const double (&term)[NV])
 {
     const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
@@ -73,8 +74,8 @@ __device__ __forceinline__ void grid_sum_post(GridSum<NT, NV>& s, unsigned long 
 }
 
 // The sums; false (in every thread of the CTA) when a wait gave up.
-template <int NT, int NV>
-__device__ __forceinline__ bool grid_sum_wait(GridSum<NT, NV>& s, const unsigned long long* lines, uint32_t epoch,
+template <int NT, int ROOM, int NV>
+__device__ __forceinline__ bool grid_sum_wait(GridSum<NT, ROOM>& s, const unsigned long long* lines, uint32_t epoch,
                                               double (&sum)[NV], int* err)
 {
     const uint32_t tid = threadIdx.x, lane = tid & 31u, ctas = gridDim.x;

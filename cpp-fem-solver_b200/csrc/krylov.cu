@@ -336,8 +336,7 @@ __global__ void __launch_bounds__(kPcgSmallThreads, 1) k_pcg_small(PcgSmallArgs 
     constexpr uint32_t NT = kPcgSmallThreads;
     constexpr int HQ = kPcgSmallHalo;
     extern __shared__ __align__(16) double pcg_sm[];
-    __shared__ GridSum<NT, 1> g1;
-    __shared__ GridSum<NT, 2> g2;
+    __shared__ GridSum<NT, 2> gs;
     __shared__ KState sst;
     const uint32_t tid = threadIdx.x, r0 = min(blockIdx.x * a.rows, a.n), rows = min(a.rows, a.n - r0);
     const uint32_t lo = r0 > a.band ? r0 - a.band : 0u, hi = min(a.n, r0 + rows + a.band);  // columns this CTA reads
@@ -356,8 +355,7 @@ __global__ void __launch_bounds__(kPcgSmallThreads, 1) k_pcg_small(PcgSmallArgs 
     if (tid == 0)
     {
         sst = *a.st;
-        g1.failed = 0;
-        g2.failed = 0;
+        gs.failed = 0;
     }
     double x[Q], r[Q], p[Q], z[Q], d[Q], Ap[Q], zh[HQ];
 #pragma unroll
@@ -419,8 +417,8 @@ __global__ void __launch_bounds__(kPcgSmallThreads, 1) k_pcg_small(PcgSmallArgs 
             one[0] += p[q] * sum;
         }
         ++epoch;
-        grid_sum_post(g1, a.lines, epoch, one);
-        if (!grid_sum_wait(g1, a.lines, epoch, pAp, a.err)) break;
+        grid_sum_post(gs, a.lines, epoch, one);
+        if (!grid_sum_wait(gs, a.lines, epoch, pAp, a.err)) break;
         if (!(pAp[0] >= kBreak))  // breakdown, not SPD or NaN: the state's own test decides
         {
             __syncthreads();
@@ -457,7 +455,7 @@ __global__ void __launch_bounds__(kPcgSmallThreads, 1) k_pcg_small(PcgSmallArgs 
             two[0] += r[q] * r[q];
             two[1] += r[q] * z[q];
         }
-        grid_sum_post(g2, a.lines + grid_sum_words(gridDim.x), epoch, two);
+        grid_sum_post(gs, a.lines + grid_sum_words(gridDim.x), epoch, two);
         // the others' z while the sum crosses the grid
 #pragma unroll
         for (int k = 0; k < HQ; ++k)
@@ -475,12 +473,12 @@ __global__ void __launch_bounds__(kPcgSmallThreads, 1) k_pcg_small(PcgSmallArgs 
                 }
                 if (!seen)
                 {
-                    g2.failed = 1;
+                    gs.failed = 1;
                     atomicCAS(a.err, 0, (int)B2S_TIMEOUT);
                 }
                 zh[k] = __longlong_as_double((long long)((wh << 32) | (wl & 0xffffffffull)));
             }
-        if (!grid_sum_wait(g2, a.lines + grid_sum_words(gridDim.x), epoch, tot, a.err)) break;
+        if (!grid_sum_wait(gs, a.lines + grid_sum_words(gridDim.x), epoch, tot, a.err)) break;
         rr = tot[0];
         if (tot[0] > clear && tot[0] < HUGE_VAL && tot[1] > 0.0 && it + 1 < maxit)
         {

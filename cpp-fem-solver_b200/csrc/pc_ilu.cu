@@ -926,11 +926,12 @@ struct PcIC0 final : PcImpl
     // the tiled persistent PCG kernel (pcg_tile.cuh), when its plan was made
     // and A's pattern matched it
     bool tiles_ready = false;
-    uint32_t tile_n = 0, tile_count = 0, tile_Q = 0, tile_smem = 0, tile_work = 0, tile_ystride = 0;
+    uint32_t tile_n = 0, tile_count = 0, tile_Q = 0, tile_smem = 0, tile_work = 0, tile_ystride = 0, tile_ring = 0;
     bool tile_fused = false;  // the forward set grown from the upper set: two all-reduces per iteration
     DBuf<TileDesc> tile_desc;
     DBuf<uint8_t> tile_idx, tile_vals;
-    DBuf<unsigned long long> tile_slots;
+    DBuf<unsigned long long> tile_words;  // the sums' lines, then z, Ap (and y) as words
+    DBuf<double> tile_loc;                // r over the lower sets, p over the rings
 
     // uploads the plan (a 5-point grid's index blobs are built on the device)
     // and packs the value blobs from A and the band arrays
@@ -954,7 +955,6 @@ struct PcIC0 final : PcImpl
         else
             tile_idx = upload(ctx, P.idx.data(), P.idx.size());
         tile_vals.alloc(P.vbytes ? P.vbytes : 16);
-        tile_slots.alloc(3ull * kTileSlotStride * P.ntiles);
         B2S_LAUNCH(ctx, k_tile_pack, P.ntiles, kThreads, 0, tile_desc.p, tile_idx.p, tile_vals.p, n, (int)P.k,
                    A.rp.p, A.ci.p, A.v.p, fwd.band_off.p, fwd.band_val.p, fwd.band_dinv.p, bwd.band_off.p,
                    bwd.band_val.p, bwd.band_dinv.p, bad.p);
@@ -969,6 +969,10 @@ struct PcIC0 final : PcImpl
         tile_work = P.work;
         tile_ystride = ::b2s::tile_ystride(P.max_ext);
         tile_fused = P.fused;
+        tile_ring = 0;
+        for (const TileDesc& t : P.desc) tile_ring = std::max<uint32_t>(tile_ring, t.n_ae - t.n_own);
+        tile_words.alloc(2 * grid_sum_words(tile_count) + (size_t)n * (tile_fused ? 3 : 4) + 1);
+        tile_loc.alloc((size_t)tile_count * (tile_ystride + tile_ring));
         tiles_ready = true;
     }
 
@@ -991,13 +995,13 @@ struct PcIC0 final : PcImpl
     }
 
     // the whole PCG loop as one k_pcg_tile launch; false (nothing enqueued) when it cannot run
-    bool pcg_tiles(b2s_ctx* ctx, const CsrDev& A, double* x, double* r0, double* r1, double* p0, double* p1,
-                   double* z, double* Ap, KState* st, int stall_window)
+    bool pcg_tiles(b2s_ctx* ctx, const CsrDev& A, double* x, const double* r, const double* p, const double* z,
+                   KState* st, int stall_window)
     {
         if (!tiles_ready || A.n != tile_n || A.rp.p == nullptr || fwd.sweeps != bwd.sweeps) return false;
         if (!pcg_ctl.p) pcg_ctl.alloc(2);
         B2S_CUDA(cudaMemsetAsync(pcg_ctl.p, 0, 2 * sizeof(unsigned), ctx->stream));
-        B2S_CUDA(cudaMemsetAsync(tile_slots.p, 0, tile_slots.bytes(), ctx->stream));
+        B2S_CUDA(cudaMemsetAsync(tile_words.p, 0, tile_words.bytes(), ctx->stream));
         PcgTileArgs a{};
         a.n = n;
         a.ntiles = tile_count;
@@ -1008,14 +1012,16 @@ struct PcIC0 final : PcImpl
         a.vals = reinterpret_cast<const uint4*>(tile_vals.p);
         a.idx = reinterpret_cast<const uint4*>(tile_idx.p);
         a.x = x;
-        a.r[0] = r0;
-        a.r[1] = r1;
-        a.p[0] = p0;
-        a.p[1] = p1;
+        a.r = r;
+        a.p = p;
         a.z = z;
-        a.Ap = Ap;
-        a.y32 = y32.p;
-        a.slots = tile_slots.p;
+        a.ring = tile_ring;
+        a.rloc = tile_loc.p;
+        a.ploc = tile_loc.p + (size_t)tile_count * tile_ystride;
+        a.lines = tile_words.p;
+        a.apw = a.lines + 2 * grid_sum_words(tile_count);
+        a.zw = a.apw + 2 * (size_t)n;
+        a.yw = a.zw + n;
         a.st = st;
         a.err = reinterpret_cast<int*>(pcg_ctl.p + 1);
         a.stall_window = stall_window;
@@ -1043,7 +1049,7 @@ struct PcIC0 final : PcImpl
     bool pcg_persistent(b2s_ctx* ctx, const CsrDev& A, double* x, double* r0, double* r1, double* p0, double* p1,
                         double* z, double* Ap, KState* st, int stall_window, int which) override
     {
-        if (can_fuse_pcg() && which == 0 && pcg_tiles(ctx, A, x, r0, r1, p0, p1, z, Ap, st, stall_window))
+        if (can_fuse_pcg() && which == 0 && pcg_tiles(ctx, A, x, r0, p0, z, st, stall_window))
             return true;
         const BandPlan &lb = fwd.band, &ub = bwd.band;
         if (!(can_fuse_pcg() && fwd.segment == 1 && bwd.segment == 1 && lb.W == 2 && ub.W == 2 && lb.T == ub.T &&

@@ -8,142 +8,92 @@
 // local indices, the triangles' strict entries and reciprocals, and its
 // owned rows of A with local columns.  Nothing static is read from global
 // memory again.  Each iteration is three phases:
-//   1. p = z + beta p_old staged for the SpMV's columns; Ap = A p and p.Ap
-//      for the owned rows (CSR order);
-//   2. the forward sweeps over the tile's lower extended set, the right-hand
-//      side r_old - alpha Ap gathered for every row of it; the owned rows
-//      store y, r and x += alpha p and reduce r.r;
+//   1. p = z + beta p_old for the owned rows and the SpMV's ring; Ap = A p and
+//      p.Ap for the owned rows (CSR order);
+//   2. r = r - alpha Ap for every row of the tile's lower extended set, and the
+//      forward sweeps over it; the owned rows take x += alpha p and r.r;
 //   3. the backward sweeps over the upper extended set on y; the owned rows
-//      store z and reduce r.z.
+//      take z and r.z.
 // Sweep s computes the rows of layers 0..k-s (a prefix of the local order),
 // so the owned rows equal the global sweep definition bit for bit, as the
 // banded kernel's do.  The arithmetic of every row is that of k_pcg_band;
-// only the association of the three per-iteration dot products differs (the
+// only the association of the two per-iteration dot products differs (the
 // tiles are other row sets).
 //
-// A phase ends with an all-reduce that is also the grid barrier: thread 0
-// fences (gpu scope, after the CTA's barrier) and publishes the tile's
-// partial as two 64-bit words {epoch, 32 value bits} in a line of its own;
-// thread b of every CTA polls tile b's words with relaxed loads until they
-// carry the phase's epoch, fences, and leaves the value in shared memory;
-// after one block barrier warp 0 sums them in tile order.  Every CTA gets the
-// same bits and takes the same scalar step.  Each wait is bounded
-// (kGridBarrierPolls polls); a CTA that gives up records B2S_TIMEOUT and
-// leaves, and the others give up at their next all-reduce, so the launch
-// always ends.
+// Every tile keeps r over its whole lower set and p over its ring itself, by the
+// owners' arithmetic, so what the tiles exchange is Ap (phase 1), z (phase 3; an
+// FP32 value) and, unfused, y (phase 2): 64-bit words {epoch, 32 value bits} that
+// a reader polls until they carry the iteration, while the phase's sum over the
+// grid (grid_sum.cuh) is on its way.  No store needs a fence, and a phase starts
+// with its operands in registers.  512^2, 6 sweeps: 20.0 us an iteration with the
+// vectors behind fenced all-reduces, about 15 us this way.  Each wait is bounded
+// (kGridSumPolls polls): a CTA that gives up records B2S_TIMEOUT and leaves, and
+// the others give up at their next sum, so the launch always ends.
 #pragma once
 
+#include "grid_sum.cuh"
 #include "pcg_band.cuh"
 #include "tile_plan.hpp"
 #include "trsv_chunk.cuh"
 
 namespace b2s {
 
-constexpr uint32_t kTileSlotStride = 16;      // words between two tiles' all-reduce slots (128 bytes)
+static_assert(kTileMaxTiles <= (int)kGridSumMaxCtas, "a poller per tile");
 
 struct PcgTileArgs
 {
-    uint32_t n, ntiles, work, ystride;
+    uint32_t n, ntiles, work, ystride, ring;
     int k;
     const TileDesc* desc;
     const uint4* vals;  // value blobs
     const uint4* idx;   // index blobs
     double* x;
-    double* r[2];
-    double* p[2];
-    double *z, *Ap;
-    float* y32;
-    unsigned long long* slots;  // 3 phases x ntiles x kTileSlotStride words, zero at launch
+    const double *r, *p, *z;        // the state before the first iteration
+    double* rloc;                   // ntiles x ystride: each tile's r over its lower set
+    double* ploc;                   // ntiles x ring: p over the rings (past one entry a thread)
+    unsigned long long *apw, *zw;   // Ap (two words a row) and z (one), zero at launch
+    unsigned long long* yw;         // unfused: the forward sweeps' results (one word a row)
+    unsigned long long* lines;      // two regions of grid_sum_words, zero at launch
     KState* st;
     int* err;
     int stall_window;
 };
 
-__device__ __forceinline__ void st_relaxed_gpu_u64(unsigned long long* p, unsigned long long v)
+__device__ __forceinline__ void tile_put(unsigned long long* w, float v, uint32_t epoch)
 {
-    asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
+    asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" ::"l"(w), "l"((unsigned long long)epoch << 32 | __float_as_uint(v))
+                 : "memory");
 }
-
-__device__ __forceinline__ unsigned long long ld_relaxed_gpu_u64(const unsigned long long* p)
+__device__ __forceinline__ void tile_put(unsigned long long* w, double v, uint32_t epoch)
 {
-    unsigned long long v;
-    asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
+    const unsigned long long e = (unsigned long long)epoch << 32, b = (unsigned long long)__double_as_longlong(v);
+    asm volatile("st.relaxed.gpu.global.v2.u64 [%0], {%1, %2};" ::"l"(w), "l"(e | (b & 0xffffffffull)), "l"(e | (b >> 32))
+                 : "memory");
+}
+__device__ __forceinline__ bool tile_get(const unsigned long long* w, uint32_t epoch, float& v)
+{
+    unsigned long long a;
+    asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(a) : "l"(w) : "memory");
+    v = __uint_as_float((uint32_t)a);
+    return (uint32_t)(a >> 32) == epoch;
+}
+__device__ __forceinline__ bool tile_get(const unsigned long long* w, uint32_t epoch, double& v)
+{
+    unsigned long long a, b;
+    asm volatile("ld.relaxed.gpu.global.v2.u64 {%0, %1}, [%2];" : "=l"(a), "=l"(b) : "l"(w) : "memory");
+    v = __longlong_as_double((long long)((b << 32) | (a & 0xffffffffull)));
+    return (uint32_t)(a >> 32) == epoch && (uint32_t)(b >> 32) == epoch;
+}
+// another tile's value of this iteration
+template <typename T>
+__device__ __forceinline__ T tile_await(const unsigned long long* w, uint32_t epoch, int* failed, int* err)
+{
+    T v;
+    for (unsigned polls = 0; polls < kGridSumPolls; ++polls)
+        if (tile_get(w, epoch, v)) return v;
+    *failed = 1;
+    atomicCAS(err, 0, (int)B2S_TIMEOUT);
     return v;
-}
-
-__device__ __forceinline__ void fence_acq_rel_gpu() { asm volatile("fence.acq_rel.gpu;" ::: "memory"); }
-
-// Thread 0 holds this tile's NV partials `part`.  Publishes them for `epoch`,
-// waits for every tile's and returns their sums in thread 0 (tile order, the
-// same association in every CTA, so the same bits); false in every thread,
-// with B2S_TIMEOUT recorded, when a wait gives up.  Each tile's 2 NV words
-// ({epoch, 32 value bits} per half) sit alone in a 128-byte line
-// (kTileSlotStride words apart), and thread b < ntiles polls tile b's words
-// only until they carry the epoch, so a tile that has arrived is not read
-// again and the polls of all CTAs spread over as many lines as tiles.
-template <int NV>
-__device__ __forceinline__ bool tile_allreduce(unsigned long long* slots, uint32_t tile, uint32_t ntiles,
-                                               uint32_t epoch, const double (&part)[NV], double (&sum)[NV], int* err,
-                                               double (*s_part)[kTileMaxTiles], int* s_fail)
-{
-    static_assert(2 * NV <= (int)kTileSlotStride, "slot line");
-    const uint32_t tid = threadIdx.x;
-    if (tid == 0)
-    {
-        // the CTA's writes (ordered before this thread by the barrier inside
-        // block_reduce) become visible before the words that announce them
-        fence_acq_rel_gpu();
-        const unsigned long long e = (unsigned long long)epoch << 32;
-#pragma unroll
-        for (int v = 0; v < NV; ++v)
-        {
-            const unsigned long long b = (unsigned long long)__double_as_longlong(part[v]);
-            st_relaxed_gpu_u64(&slots[(size_t)kTileSlotStride * tile + 2 * v], e | (b & 0xffffffffull));
-            st_relaxed_gpu_u64(&slots[(size_t)kTileSlotStride * tile + 2 * v + 1], e | (b >> 32));
-        }
-    }
-    if (tid < ntiles)
-    {
-        const unsigned long long* w = &slots[(size_t)kTileSlotStride * tid];
-        unsigned long long wd[2 * NV];
-        bool seen = false;
-        for (unsigned polls = 0; polls < kGridBarrierPolls && !seen; ++polls)
-        {
-            seen = true;
-#pragma unroll
-            for (int q = 0; q < 2 * NV; ++q)
-            {
-                wd[q] = ld_relaxed_gpu_u64(w + q);
-                seen &= (uint32_t)(wd[q] >> 32) == epoch;
-            }
-        }
-        if (!seen)
-        {
-            *s_fail = 1;
-            atomicExch(err, (int)B2S_TIMEOUT);
-        }
-        // the words seen carry the other CTAs' fenced writes: this fence (then
-        // the block barrier below) orders the CTA's later reads after them
-        fence_acq_rel_gpu();
-#pragma unroll
-        for (int v = 0; v < NV; ++v)
-            s_part[v][tid] =
-                __longlong_as_double((long long)(((wd[2 * v + 1] & 0xffffffffull) << 32) | (wd[2 * v] & 0xffffffffull)));
-    }
-    __syncthreads();
-    if (tid < 32)
-    {
-#pragma unroll
-        for (int v = 0; v < NV; ++v)
-        {
-            double t = 0.0;
-            for (uint32_t b = tid; b < ntiles; b += 32) t += s_part[v][b];
-#pragma unroll
-            for (int o = 16; o > 0; o >>= 1) t += __shfl_down_sync(0xffffffffu, t, o);
-            sum[v] = t;
-        }
-    }
-    return *s_fail == 0;
 }
 
 // k + 1 passes over the extended set; rows of layers 0..k-s at pass s.
@@ -217,8 +167,7 @@ __global__ void __launch_bounds__(kTileThreads, 1) k_pcg_tile(PcgTileArgs a)
     constexpr uint32_t NT = kTileThreads;
     extern __shared__ __align__(16) unsigned char smem[];
     __shared__ KState sst;
-    __shared__ int s_fail;
-    __shared__ double s_part[2][kTileMaxTiles];
+    __shared__ GridSum<NT, 2> gs;
     __shared__ double s_best;
     __shared__ int s_best_at;
     const uint32_t tile = blockIdx.x, ntiles = a.ntiles, tid = threadIdx.x;
@@ -243,7 +192,7 @@ __global__ void __launch_bounds__(kTileThreads, 1) k_pcg_tile(PcgTileArgs a)
     if (tid == 0)
     {
         sst = *a.st;
-        s_fail = 0;
+        gs.failed = 0;
         s_best = HUGE_VAL;
         s_best_at = 0;
     }
@@ -268,10 +217,8 @@ __global__ void __launch_bounds__(kTileThreads, 1) k_pcg_tile(PcgTileArgs a)
     const uint32_t lbase = s_lcnt[0];  // the lower set's layer 0: the owned rows, or (fused) the upper set
     const uint32_t dummy = a.ystride - 1;  // the sweeps' spare slot (past every set)
 
-    // the slot regions of the iteration's all-reduces (each ntiles lines)
-    unsigned long long* const slot_alpha = a.slots;
-    unsigned long long* const slot_rr = a.slots + (size_t)kTileSlotStride * ntiles;
-    unsigned long long* const slot_rz = a.slots + (size_t)(FUSED ? 1 : 2) * kTileSlotStride * ntiles;
+    unsigned long long* const lines1 = a.lines;
+    unsigned long long* const lines2 = a.lines + grid_sum_words(ntiles);
 
     // convergence test on r.r (thread 0), with the learned solve's stall guard
     auto converge = [&](double rr) {
@@ -291,67 +238,92 @@ __global__ void __launch_bounds__(kTileThreads, 1) k_pcg_tile(PcgTileArgs a)
         }
     };
 
-    uint32_t epoch = 0;
-    int parity = 0;
-    // The owned rows' p and x live in registers (thread's rows t = tid + NT q);
-    // p is also stored each iteration (other tiles read it), x once at the end.
-    double pv[Q], xv[Q];
+    // The owned rows' p and x live in registers (thread's rows t = tid + NT q), as
+    // does p of the thread's first ring entry; r of its rows of the lower set in
+    // its own words of rloc, read back while a sum is awaited.
+    double* const rl = a.rloc + (size_t)tile * a.ystride;
+    double* const pl = a.ploc + (size_t)tile * a.ring;
+    const uint32_t n_ring = n_ae - n_own;
+    auto lower_row = [&](uint32_t t) { return t < n_own ? owned[t] : t < lbase ? uhalo[t - n_own] : lhalo[t - lbase]; };
+    double pv[Q], xv[Q], ph = 0.0;
+    float zv[Q], zh = 0.f;
 #pragma unroll
     for (uint32_t q = 0; q < Q; ++q)
     {
         const uint32_t t = tid + NT * q;
-        const uint32_t g = t < n_own ? owned[t] : 0u;
         const bool in = t < n_own;
-        pv[q] = in ? a.p[0][g] : 0.0;
+        const uint32_t g = in ? owned[t] : 0u;
+        pv[q] = in ? a.p[g] : 0.0;
         xv[q] = in ? a.x[g] : 0.0;
+        zv[q] = in ? (float)a.z[g] : 0.f;  // (an FP32 value)
+        if (t < n_el) rl[t] = a.r[lower_row(t)];
+    }
+    for (uint32_t t = tid; t < n_ring; t += NT)
+    {
+        if (t >= NT) pl[t] = a.p[ahalo[t]];
+        if (t < NT)
+        {
+            ph = a.p[ahalo[t]];
+            zh = (float)a.z[ahalo[t]];
+        }
     }
     const float* yf = y0;  // the forward sweeps' result (phase 2 -> phase 3)
+    uint32_t epoch = 0;
     while (!sst.done)
     {
-        const double* pold = a.p[parity];
-        double* pnew = a.p[parity ^ 1];
-        const double* rold = a.r[parity];
-        double* rnew = a.r[parity ^ 1];
         // ---- 1. p = z + beta p_old at the SpMV's columns; Ap; p.Ap
+        double Apv[Q];
         {
             const double beta = sst.beta;
 #pragma unroll
             for (uint32_t q = 0; q < Q; ++q)
             {
                 const uint32_t t = tid + NT * q;
-                if (t < n_own) pe[t] = __ldcg(&a.z[owned[t]]) + beta * pv[q];
+                pv[q] = (double)zv[q] + beta * pv[q];
+                if (t < n_own) pe[t] = pv[q];
             }
-            for (uint32_t t = n_own + tid; t < n_ae; t += NT)
+            if (tid < n_ring)
             {
-                const uint32_t g = ahalo[t - n_own];
-                pe[t] = __ldcg(&a.z[g]) + beta * __ldcg(&pold[g]);
+                ph = (double)zh + beta * ph;
+                pe[n_own + tid] = ph;
             }
+            for (uint32_t t = tid + NT; t < n_ring; t += NT)
+            {
+                const float zt = epoch ? tile_await<float>(&a.zw[ahalo[t]], epoch, &gs.failed, a.err) : (float)a.z[ahalo[t]];
+                pe[n_own + t] = pl[t] = (double)zt + beta * pl[t];
+            }
+            ++epoch;
             __syncthreads();
-            double acc[1] = {0.0};
+            double acc[1] = {0.0}, tot[1];
 #pragma unroll
             for (uint32_t q = 0; q < Q; ++q)
             {
                 const uint32_t t = tid + NT * q;
+                Apv[q] = 0.0;
                 if (t < n_own)
                 {
                     double sum = 0.0;
                     for (uint32_t e = arp[t]; e < arp[t + 1]; ++e) sum += aval[e] * pe[acol[e]];
-                    const double pr = pe[t];
-                    const uint32_t g = owned[t];
-                    pnew[g] = pr;
-                    a.Ap[g] = sum;
-                    acc[0] += pr * sum;
-                    pv[q] = pr;
+                    tile_put(&a.apw[2 * (size_t)owned[t]], sum, epoch);
+                    acc[0] += pv[q] * sum;
+                    Apv[q] = sum;
                 }
             }
-            block_reduce<1, NT>(acc);
-            double tot[1];
-            if (!tile_allreduce<1>(slot_alpha, tile, ntiles, ++epoch, acc, tot, a.err, s_part, &s_fail)) break;
+            grid_sum_post(gs, lines1, epoch, acc);
+            // the other tiles' Ap over the lower set, while the sum is on its way
+#pragma unroll
+            for (uint32_t q = 0; q < Q; ++q)
+            {
+                const uint32_t t = tid + NT * q;
+                if (t >= n_own && t < n_el)
+                    Apv[q] = tile_await<double>(&a.apw[2 * (size_t)lower_row(t)], epoch, &gs.failed, a.err);
+            }
+            if (!grid_sum_wait(gs, lines1, epoch, tot, a.err)) break;
             if (tid == 0) pcg_alpha(&sst, tot[0]);
             __syncthreads();
             if (sst.done) break;
         }
-        // ---- 2. forward sweeps on r = r_old - alpha Ap; x, r; r.r
+        // ---- 2. r = r - alpha Ap, forward sweeps on it; x; r.r
         double rr_acc = 0.0;
         {
             const double alpha = sst.alpha;
@@ -363,38 +335,28 @@ __global__ void __launch_bounds__(kTileThreads, 1) k_pcg_tile(PcgTileArgs a)
             {
                 const uint32_t t = tid + NT * q;
                 const bool in = t < n_el;
-                const uint32_t g = !in ? 0u : t < n_own ? owned[t] : t < lbase ? uhalo[t - n_own] : lhalo[t - lbase];
                 dep[q] = tile_dep_slots(in ? ldeps[t] : 0xFFFFFFFFu, dummy);
                 val[q] = in ? lvals[t] : make_float2(0.f, 0.f);
                 di[q] = in ? ldinv[t] : 0.f;
-                const double rv = in ? __ldcg(&rold[g]) - alpha * __ldcg(&a.Ap[g]) : 0.0;
+                const double rv = in ? rl[t] - alpha * Apv[q] : 0.0;
                 rr[q] = (float)rv;
-                if (t < n_own)  // the owned rows' r, r.r and x now, before the sweeps
+                if (in) rl[t] = rv;
+                if (t < n_own)  // the owned rows' r.r and x now, before the sweeps
                 {
-                    rnew[g] = rv;
                     rr_acc += rv * rv;
                     xv[q] += alpha * pv[q];
                 }
             }
             yf = tile_sweeps<Q>(a.k, s_lcnt, dep, val, di, rr, y0, y1, dummy);
             if constexpr (!FUSED)
-            {
-                // other tiles read y at this tile's rows after the grid-wide exchange
 #pragma unroll
                 for (uint32_t q = 0; q < Q; ++q)
                 {
                     const uint32_t t = tid + NT * q;
-                    if (t < n_own) a.y32[owned[t]] = yf[t];
+                    if (t < n_own) tile_put(&a.yw[owned[t]], yf[t], epoch);
                 }
-                double acc[1] = {rr_acc}, tot[1];
-                block_reduce<1, NT>(acc);
-                if (!tile_allreduce<1>(slot_rr, tile, ntiles, ++epoch, acc, tot, a.err, s_part, &s_fail)) break;
-                if (tid == 0) converge(tot[0]);
-                __syncthreads();
-                if (sst.done) break;
-            }
         }
-        // ---- 3. backward sweeps on y; z; r.z and beta (fused: with r.r and the test)
+        // ---- 3. backward sweeps on y; z; r.r and r.z: the test and beta
         {
             uint32_t dep[Q];
             float2 val[Q];
@@ -412,44 +374,33 @@ __global__ void __launch_bounds__(kTileThreads, 1) k_pcg_tile(PcgTileArgs a)
                 if constexpr (FUSED)
                     rr[q] = in ? yf[t] : 0.f;
                 else
-                    rr[q] = t < n_own ? yf[t] : in ? __ldcg(&a.y32[uhalo[t - n_own]]) : 0.f;
+                    rr[q] = t < n_own ? yf[t]
+                            : in      ? tile_await<float>(&a.yw[uhalo[t - n_own]], epoch, &gs.failed, a.err)
+                                      : 0.f;
             }
             const float* yk = tile_sweeps<Q>(a.k, s_ucnt, dep, val, di, rr, y0, y1, dummy);
-            double acc[2] = {0.0, 0.0};
+            double acc[2] = {rr_acc, 0.0}, tot[2];
 #pragma unroll
             for (uint32_t q = 0; q < Q; ++q)
             {
                 const uint32_t t = tid + NT * q;
                 if (t < n_own)
                 {
-                    const uint32_t g = owned[t];
-                    const double zi = (double)yk[t];
-                    a.z[g] = zi;
-                    acc[1] += rnew[g] * zi;  // (this thread's own store of phase 2)
+                    zv[q] = yk[t];
+                    tile_put(&a.zw[owned[t]], zv[q], epoch);
+                    acc[1] += rl[t] * (double)zv[q];  // (this thread's own store of phase 2)
                 }
             }
-            if constexpr (FUSED)
+            grid_sum_post(gs, lines2, epoch, acc);
+            if (tid < n_ring) zh = tile_await<float>(&a.zw[ahalo[tid]], epoch, &gs.failed, a.err);
+            if (!grid_sum_wait(gs, lines2, epoch, tot, a.err)) break;
+            if (tid == 0)
             {
-                acc[0] = rr_acc;
-                double tot[2];
-                block_reduce<2, NT>(acc);
-                if (!tile_allreduce<2>(slot_rz, tile, ntiles, ++epoch, acc, tot, a.err, s_part, &s_fail)) break;
-                if (tid == 0)
-                {
-                    converge(tot[0]);
-                    if (!sst.done) pcg_next(&sst, tot[1]);
-                }
-            }
-            else
-            {
-                double one[1] = {acc[1]}, tot[1];
-                block_reduce<1, NT>(one);
-                if (!tile_allreduce<1>(slot_rz, tile, ntiles, ++epoch, one, tot, a.err, s_part, &s_fail)) break;
-                if (tid == 0) pcg_next(&sst, tot[0]);
+                converge(tot[0]);
+                if (!sst.done) pcg_next(&sst, tot[1]);
             }
             __syncthreads();
         }
-        parity ^= 1;
     }
 #pragma unroll
     for (uint32_t q = 0; q < Q; ++q)
