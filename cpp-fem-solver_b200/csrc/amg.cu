@@ -46,14 +46,17 @@ __global__ void k_find_diag(uint32_t nb, const uint32_t* __restrict__ rp, const 
 {
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < nb; i += gridDim.x * blockDim.x)
     {
-        uint32_t d = 0xFFFFFFFFu;
-        for (uint32_t p = rp[i]; p < rp[i + 1]; ++p)
-            if (ci[p] == i)
-            {
-                d = p;
-                break;
-            }
-        dptr[i] = d;
+        uint32_t lo = rp[i];
+        const uint32_t end = rp[i + 1];
+        for (uint32_t hi = end; lo < hi;)  // columns ascend
+        {
+            const uint32_t mid = lo + (hi - lo) / 2;
+            if (ci[mid] < i)
+                lo = mid + 1;
+            else
+                hi = mid;
+        }
+        dptr[i] = lo < end && ci[lo] == i ? lo : 0xFFFFFFFFu;
     }
 }
 
@@ -105,30 +108,54 @@ __device__ __forceinline__ double fro(const double* b)
     return sqrt(s);
 }
 
-template <int BS>
+// Strong columns of a row: ||A_ij|| >= theta max_k ||A_ik||, in row order.  GL lanes
+// a row: one for the short rows of a fine operator, a warp for the long rows of
+// the few that a coarse one has (a thread a row took 0.14 - 0.18 ms a pass at
+// 5,520 rows and below).
+template <int BS, int GL>
 __global__ void k_strength(uint32_t nb, const uint32_t* __restrict__ rp, const uint32_t* __restrict__ ci,
                            const double* __restrict__ v, const uint32_t* __restrict__ sp, uint32_t* __restrict__ cnt,
                            uint32_t* __restrict__ sc)
 {
     constexpr int BV = BS * BS;
-    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < nb; i += gridDim.x * blockDim.x)
+    const uint32_t l = threadIdx.x % GL, groups = gridDim.x * blockDim.x / GL;
+    for (uint32_t i = (blockIdx.x * blockDim.x + threadIdx.x) / GL; i < nb; i += groups)
     {
+        const uint32_t p0 = rp[i], p1 = rp[i + 1];
         double mx = 0.0;
-        for (uint32_t p = rp[i]; p < rp[i + 1]; ++p)
+        for (uint32_t p = p0 + l; p < p1; p += GL)
             if (ci[p] != i)
             {
                 const double f = fro<BS>(&v[(size_t)p * BV]);
                 mx = mx < f ? f : mx;
             }
-        const double thr = kTheta * mx;
-        uint32_t c = 0, w = sp ? sp[i] : 0;
-        for (uint32_t p = rp[i]; p < rp[i + 1]; ++p)
-            if (ci[p] != i && fro<BS>(&v[(size_t)p * BV]) >= thr)
+        if constexpr (GL > 1)
+#pragma unroll
+            for (int o = GL / 2; o; o >>= 1)
             {
-                if (sc) sc[w++] = ci[p];
+                const double f = __shfl_xor_sync(0xffffffffu, mx, o);
+                mx = mx < f ? f : mx;
+            }
+        const double thr = kTheta * mx;
+        uint32_t c = 0;
+        const uint32_t w = sp ? sp[i] : 0;
+        for (uint32_t q = p0; q < p1; q += GL)
+        {
+            const uint32_t p = q + l;
+            const bool strong = p < p1 && ci[p] != i && fro<BS>(&v[(size_t)p * BV]) >= thr;
+            if constexpr (GL > 1)
+            {
+                const uint32_t m = __ballot_sync(0xffffffffu, strong);
+                if (sc && strong) sc[w + c + __popc(m & ((1u << l) - 1u))] = ci[p];
+                c += __popc(m);
+            }
+            else if (strong)
+            {
+                if (sc) sc[w + c] = ci[p];
                 ++c;
             }
-        if (cnt) cnt[i] = c;
+        }
+        if (cnt && l == 0) cnt[i] = c;
     }
     if (cnt && blockIdx.x == 0 && threadIdx.x == 0) cnt[nb] = 0;
 }
@@ -412,11 +439,14 @@ static uint32_t aggregate_parallel(b2s_ctx* ctx, uint32_t n, const uint32_t* sp,
 
 // ------------------------------------------------------------ prolongation
 
-// distinct aggregates among {agg[i]} U {agg[k] : k in row i}, ascending
+// distinct aggregates among {agg[i]} U {agg[k] : k in row i}, ascending; GL lanes
+// (a thread, or a whole warp) hold the row, every lane gets the count
+template <int GL>
 __device__ __forceinline__ uint32_t p_row_cols(uint32_t i, const uint32_t* rp, const uint32_t* ci, const int32_t* agg,
                                                uint32_t* out)
 {
     // count distinct; write ascending when out != null
+    const uint32_t l = threadIdx.x % GL;
     uint32_t cnt = 0;
     int32_t last = -1;
     for (;;)
@@ -425,38 +455,48 @@ __device__ __forceinline__ uint32_t p_row_cols(uint32_t i, const uint32_t* rp, c
         int32_t best = 0x7fffffff;
         const int32_t gi = agg[i];
         if (gi > last && gi < best) best = gi;
-        for (uint32_t p = rp[i]; p < rp[i + 1]; ++p)
+        for (uint32_t p = rp[i] + l; p < rp[i + 1]; p += GL)
         {
             const int32_t g = agg[ci[p]];
             if (g > last && g < best) best = g;
         }
+        if constexpr (GL > 1) best = __reduce_min_sync(0xffffffffu, best);
         if (best == 0x7fffffff) break;
-        if (out) out[cnt] = (uint32_t)best;
+        if (out && l == 0) out[cnt] = (uint32_t)best;
         ++cnt;
         last = best;
     }
+    if constexpr (GL > 1) __syncwarp();  // the columns are read by every lane
     return cnt;
 }
 
+template <int GL>
 __global__ void k_p_count(uint32_t nb, const uint32_t* __restrict__ rp, const uint32_t* __restrict__ ci,
                           const int32_t* __restrict__ agg, uint32_t* __restrict__ cnt)
 {
-    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < nb; i += gridDim.x * blockDim.x)
-        cnt[i] = p_row_cols(i, rp, ci, agg, nullptr);
+    for (uint32_t i = (blockIdx.x * blockDim.x + threadIdx.x) / GL; i < nb; i += gridDim.x * blockDim.x / GL)
+    {
+        const uint32_t c = p_row_cols<GL>(i, rp, ci, agg, nullptr);
+        if (threadIdx.x % GL == 0) cnt[i] = c;
+    }
     if (blockIdx.x == 0 && threadIdx.x == 0) cnt[nb] = 0;
 }
 
-template <int BS>
+// Row i of P: the tentative prolongation's identity block and the smoothing
+// terms, each column's in row order.  With a warp a row, lane l owns every 32nd
+// column and adds that column's terms itself, so the order stays the row's.
+template <int BS, int GL>
 __global__ void k_p_fill(uint32_t nb, const uint32_t* __restrict__ rp, const uint32_t* __restrict__ ci,
                          const double* __restrict__ v, const double* __restrict__ dinv, const int32_t* __restrict__ agg,
-                         const uint32_t* __restrict__ prp, uint32_t* __restrict__ pci, double* __restrict__ pv)
+                         const uint32_t* __restrict__ prp, uint32_t* pci, double* __restrict__ pv)
 {
     constexpr int BV = BS * BS;
-    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < nb; i += gridDim.x * blockDim.x)
+    const uint32_t l = threadIdx.x % GL;
+    for (uint32_t i = (blockIdx.x * blockDim.x + threadIdx.x) / GL; i < nb; i += gridDim.x * blockDim.x / GL)
     {
         const uint32_t base = prp[i];
-        const uint32_t cnt = p_row_cols(i, rp, ci, agg, pci + base);
-        for (uint32_t s = 0; s < cnt; ++s)
+        const uint32_t cnt = p_row_cols<GL>(i, rp, ci, agg, pci + base);
+        for (uint32_t s = l; s < cnt; s += GL)
             for (int k = 0; k < BV; ++k) pv[(size_t)(base + s) * BV + k] = 0.0;
         auto slot = [&](uint32_t g) {
             uint32_t lo = 0, hi = cnt;
@@ -468,24 +508,34 @@ __global__ void k_p_fill(uint32_t nb, const uint32_t* __restrict__ rp, const uin
                 else
                     hi = mid;
             }
-            return base + lo;
+            return lo;
         };
+        const uint32_t diag = slot((uint32_t)agg[i]);
+        if (diag % GL == l)
         {
-            double* I = &pv[(size_t)slot((uint32_t)agg[i]) * BV];
+            double* I = &pv[(size_t)(base + diag) * BV];
             for (int r = 0; r < BS; ++r) I[r * BS + r] = 1.0;
         }
         const double* Di = &dinv[(size_t)i * BV];
-        for (uint32_t p = rp[i]; p < rp[i + 1]; ++p)
+        for (uint32_t q = rp[i]; q < rp[i + 1]; q += GL)
         {
-            const double* ab = &v[(size_t)p * BV];
-            double* dst = &pv[(size_t)slot((uint32_t)agg[ci[p]]) * BV];
-            for (int r = 0; r < BS; ++r)
-                for (int c = 0; c < BS; ++c)
-                {
-                    double s = 0.0;
-                    for (int m = 0; m < BS; ++m) s += Di[r * BS + m] * ab[m * BS + c];
-                    dst[r * BS + c] -= kOmega * s;
-                }
+            // GL entries' slots, then each entry by its column's owner
+            const uint32_t mine = q + l < rp[i + 1] ? slot((uint32_t)agg[ci[q + l]]) : 0u;
+            const uint32_t m = GL > 1 ? min((uint32_t)GL, rp[i + 1] - q) : 1u;
+            for (uint32_t t = 0; t < m; ++t)
+            {
+                const uint32_t at = GL > 1 ? __shfl_sync(0xffffffffu, mine, t) : mine;
+                if (at % GL != l) continue;
+                const double* ab = &v[(size_t)(q + t) * BV];
+                double* dst = &pv[(size_t)(base + at) * BV];
+                for (int r = 0; r < BS; ++r)
+                    for (int c = 0; c < BS; ++c)
+                    {
+                        double s = 0.0;
+                        for (int k = 0; k < BS; ++k) s += Di[r * BS + k] * ab[k * BS + c];
+                        dst[r * BS + c] -= kOmega * s;
+                    }
+            }
         }
     }
 }
@@ -587,101 +637,157 @@ __global__ void k_mm_unique_fill(uint32_t nr, const uint32_t* __restrict__ off, 
     }
 }
 
-// Symbolic product, one warp per row i of C = A B: the distinct columns of
-// the row are collected in a per-warp open-addressing hash table in shared
-// memory (inserted with atomicCAS; the lanes take B's row entries in
-// parallel).  COUNT: cnt[i] = their number.  Otherwise they are written in
-// ascending order (rank sort, the columns being distinct) to cci[crp[i]...].
-// A row whose columns do not fit the table raises *overflow and writes
-// nothing; the caller then uses the sort-based symbolic product.
-constexpr uint32_t kMmHashBits = 9;
-constexpr uint32_t kMmHashSlots = 1u << kMmHashBits;  // per warp
+// One row i of C = A B per group of GL lanes: the row's distinct columns are
+// collected in an open-addressing hash table of SL slots in shared memory
+// (inserted with atomicCAS), the group taking A's row entries in order and its
+// lanes one row of B.  MmMode::Count: cnt[i] = their number; Columns: they are
+// written in ascending order (rank sort, the columns being distinct) to
+// cci[crp[i]...]; Values (scalars): their sums too, every product added in A's
+// entry order -- the entries of one row of B have distinct columns, so no two
+// lanes add into one slot between two barriers -- which is the reference's order.
+// A row whose columns do not fit the table raises *overflow; the caller takes a
+// larger one.
+//
+// A row of B is as short as 3 or 4 entries (the prolongation), so a warp a row left
+// most lanes idle and cleared and searched a 512-slot table for 8 columns: 128^3,
+// A P and R (A P) of the first level 1.14 + 2.64 + 0.60 and 0.53 + 1.01 + 1.34 ms
+// (count, columns, values apart), 0.19 + 0.56 and 0.24 + 0.67 this way (values with the
+// columns).
+enum class MmMode
+{
+    Count,
+    Columns,
+    Values
+};
 constexpr uint32_t kMmEmpty = 0xFFFFFFFFu;
 
-template <bool COUNT>
-__global__ void __launch_bounds__(kThreads) k_mm_hash(uint32_t nr, const uint32_t* __restrict__ arp,
-                                                      const uint32_t* __restrict__ aci,
-                                                      const uint32_t* __restrict__ brp,
-                                                      const uint32_t* __restrict__ bci, uint32_t* __restrict__ cnt,
-                                                      const uint32_t* __restrict__ crp, uint32_t* __restrict__ cci,
-                                                      int* overflow)
+// shared memory of one group
+template <int SL, MmMode MODE>
+struct MmTable
 {
-    __shared__ uint32_t table[kThreads / 32][kMmHashSlots];
-    __shared__ uint32_t list[COUNT ? 1 : kThreads / 32][COUNT ? 1 : kMmHashSlots];
-    const uint32_t lane = threadIdx.x & 31u, wid = threadIdx.x >> 5;
-    uint32_t* T = table[wid];
-    if (COUNT && blockIdx.x == 0 && threadIdx.x == 0) cnt[nr] = 0;
-    const uint32_t warps = gridDim.x * (blockDim.x >> 5);
-    for (uint32_t i = blockIdx.x * (blockDim.x >> 5) + wid; i < nr; i += warps)
+    double val[MODE == MmMode::Values ? SL : 1];
+    uint32_t key[SL];
+    uint32_t list[MODE == MmMode::Count ? 1 : SL];  // the keys found, and their slots
+    uint16_t slot[MODE == MmMode::Count ? 2 : SL];
+};
+
+template <int GL, int SL, MmMode MODE>
+__global__ void __launch_bounds__(kThreads) k_mm_row(uint32_t nr, const uint32_t* __restrict__ arp,
+                                                     const uint32_t* __restrict__ aci, const double* __restrict__ av,
+                                                     const uint32_t* __restrict__ brp, const uint32_t* __restrict__ bci,
+                                                     const double* __restrict__ bv, uint32_t* __restrict__ cnt,
+                                                     const uint32_t* __restrict__ crp, uint32_t* __restrict__ cci,
+                                                     double* __restrict__ cv, int* overflow)
+{
+    static_assert(SL >= GL && SL % GL == 0 && (SL & (SL - 1)) == 0 && 32 % GL == 0, "table");
+    constexpr int RPC = kThreads / GL, U = MODE == MmMode::Count ? 2 : 4;
+    constexpr int SHIFT = 32 - (SL == 32 ? 5 : SL == 128 ? 7 : SL == 256 ? 8 : 9);
+    constexpr bool VALUES = MODE == MmMode::Values;
+    extern __shared__ __align__(16) unsigned char mm_sm[];
+    const uint32_t g = threadIdx.x / GL, l = threadIdx.x % GL, in_warp = (threadIdx.x & 31u) / GL;
+    MmTable<SL, MODE>& T = reinterpret_cast<MmTable<SL, MODE>*>(mm_sm)[g];
+    if (MODE == MmMode::Count && blockIdx.x == 0 && threadIdx.x == 0) cnt[nr] = 0;
+    for (uint32_t i0 = blockIdx.x * RPC; i0 < nr; i0 += gridDim.x * RPC)
     {
-        for (uint32_t s = lane; s < kMmHashSlots; s += 32) T[s] = kMmEmpty;
+        const uint32_t i = i0 + g;
+        for (uint32_t s = l; s < (uint32_t)SL; s += GL)
+        {
+            T.key[s] = kMmEmpty;
+            if constexpr (VALUES) T.val[s] = 0.0;
+        }
         __syncwarp();
+        const uint32_t a0 = i < nr ? arp[i] : 0u, na = i < nr ? arp[i + 1] - a0 : 0u;
+        const uint32_t nmax = __reduce_max_sync(0xffffffffu, na);
         uint32_t added = 0;
         bool full = false;
-        const uint32_t a1 = arp[i + 1];
-        for (uint32_t pa = arp[i]; pa < a1 && !full; ++pa)
-        {
-            const uint32_t k = aci[pa];
-            const uint32_t b1 = brp[k + 1];
-            for (uint32_t pb = brp[k] + lane; pb < b1; pb += 32)
+        // one entry of B into the table (s: the product's term)
+        auto take = [&](uint32_t j, double term) {
+            uint32_t h = (j * 2654435761u) >> SHIFT;
+            for (uint32_t probes = 0;; ++probes)
             {
-                const uint32_t j = bci[pb];
-                uint32_t h = (j * 2654435761u) >> (32 - kMmHashBits);
-                for (uint32_t probes = 0;; ++probes)
+                if (probes == (uint32_t)SL)
                 {
-                    if (probes == kMmHashSlots)
-                    {
-                        full = true;
-                        break;
-                    }
-                    const uint32_t old = atomicCAS(&T[h], kMmEmpty, j);
-                    if (old == kMmEmpty) ++added;
-                    if (old == kMmEmpty || old == j) break;
-                    h = (h + 1) & (kMmHashSlots - 1);
+                    full = true;
+                    return;
+                }
+                const uint32_t old = atomicCAS(&T.key[h], kMmEmpty, j);
+                if (old == kMmEmpty) ++added;
+                if (old == kMmEmpty || old == j) break;
+                h = (h + 1) & (SL - 1);
+            }
+            if constexpr (VALUES) T.val[h] += term;
+        };
+        for (uint32_t c = 0; c < nmax; c += GL)
+        {
+            // GL entries of A's row, one a lane
+            uint32_t b0 = 0, len = 0;
+            double a = 0.0;
+            if (c + l < na)
+            {
+                const uint32_t k = aci[a0 + c + l];
+                b0 = brp[k];
+                len = brp[k + 1] - b0;
+                if constexpr (VALUES) a = av[a0 + c + l];
+            }
+            // U of them at a time, their rows of B in flight together
+            for (uint32_t t = 0; t < (uint32_t)GL && c + t < nmax; t += U)
+            {
+                uint32_t kb[U], ln[U], j[U];
+                double v[U], ak[U];
+#pragma unroll
+                for (int u = 0; u < U; ++u)
+                {
+                    kb[u] = __shfl_sync(0xffffffffu, b0, t + u, GL);
+                    ln[u] = __shfl_sync(0xffffffffu, len, t + u, GL);
+                    ak[u] = VALUES ? __shfl_sync(0xffffffffu, a, t + u, GL) : 0.0;
+                    j[u] = l < ln[u] ? bci[kb[u] + l] : kMmEmpty;
+                    v[u] = VALUES && l < ln[u] ? bv[kb[u] + l] : 0.0;
+                }
+#pragma unroll
+                for (int u = 0; u < U; ++u)
+                {
+                    if (j[u] != kMmEmpty) take(j[u], 0.0 + ak[u] * v[u]);
+                    for (uint32_t q = l + GL; q < ln[u]; q += GL)
+                        take(bci[kb[u] + q], VALUES ? 0.0 + ak[u] * bv[kb[u] + q] : 0.0);
+                    if constexpr (VALUES) __syncwarp();
                 }
             }
         }
         __syncwarp();
-        if (__any_sync(0xffffffffu, full))
+        if (full) atomicExch(overflow, 1);
+        if constexpr (MODE == MmMode::Count)
         {
-            if (lane == 0)
-            {
-                atomicExch(overflow, 1);
-                if (COUNT) cnt[i] = 0;
-            }
-            __syncwarp();
-            continue;
-        }
-        uint32_t tot = added;
 #pragma unroll
-        for (int o = 16; o; o >>= 1) tot += __shfl_xor_sync(0xffffffffu, tot, o);
-        if (COUNT)
-        {
-            if (lane == 0) cnt[i] = tot;
+            for (int o = GL / 2; o; o >>= 1) added += __shfl_xor_sync(0xffffffffu, added, o);
+            if (l == 0 && i < nr) cnt[i] = added;
         }
         else
         {
-            uint32_t* Lst = list[wid];
-            uint32_t base = 0;
-            for (uint32_t s0 = 0; s0 < kMmHashSlots; s0 += 32)
+            uint32_t found = 0;
+            for (uint32_t s0 = 0; s0 < (uint32_t)SL; s0 += GL)
             {
-                const uint32_t v = T[s0 + lane];
-                const bool has = v != kMmEmpty;
-                const uint32_t m = __ballot_sync(0xffffffffu, has);
-                if (has) Lst[base + __popc(m & ((1u << lane) - 1u))] = v;
-                base += __popc(m);
+                const uint32_t key = T.key[s0 + l];
+                const uint32_t m = (__ballot_sync(0xffffffffu, key != kMmEmpty) >> (in_warp * GL)) & (0xffffffffu >> (32 - GL));
+                if (key != kMmEmpty)
+                {
+                    const uint32_t at = found + __popc(m & ((1u << l) - 1u));
+                    T.list[at] = key;
+                    T.slot[at] = (uint16_t)(s0 + l);
+                }
+                found += __popc(m);
             }
             __syncwarp();
-            const uint32_t out = crp[i];
-            for (uint32_t a = lane; a < base; a += 32)
+            const uint32_t out = i < nr ? crp[i] : 0u;
+            for (uint32_t x = l; x < found; x += GL)
             {
-                const uint32_t v = Lst[a];
+                const uint32_t key = T.list[x];
                 uint32_t r = 0;
-                for (uint32_t b = 0; b < base; ++b) r += Lst[b] < v;
-                cci[out + r] = v;
+                for (uint32_t y = 0; y < found; ++y) r += T.list[y] < key;
+                cci[out + r] = key;
+                if constexpr (VALUES) cv[out + r] = T.val[T.slot[x]];
             }
         }
-        __syncwarp();  // the table and list are reused by the next row
+        __syncwarp();  // the table is reused by the next row
     }
 }
 
@@ -786,6 +892,40 @@ __global__ void k_mm_numeric_warp(uint32_t nr, const uint32_t* __restrict__ arp,
     }
 }
 
+template <int GL, int SL, MmMode MODE>
+void mm_rows_t(b2s_ctx* ctx, const BaijDev& A, const BaijDev& B, BaijDev& C, uint32_t* cnt, int* overflow)
+{
+    constexpr uint32_t rpc = kThreads / GL, smem = rpc * sizeof(MmTable<SL, MODE>);
+    auto kern = k_mm_row<GL, SL, MODE>;
+    B2S_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    const unsigned grid = std::min<unsigned>((A.nbr + rpc - 1) / rpc, (unsigned)ctx->sm_count * 8);
+    B2S_LAUNCH(ctx, kern, grid, kThreads, smem, A.nbr, A.rp.p, A.ci.p, A.v.p, B.rp.p, B.ci.p, B.v.p, cnt, C.rp.p, C.ci.p,
+               C.v.p, overflow);
+}
+
+// tier: 32, 128, 256 or 512 slots a row; lanes a row by B's mean row length
+template <MmMode MODE>
+void mm_rows(b2s_ctx* ctx, int tier, double mean_b, const BaijDev& A, const BaijDev& B, BaijDev& C, uint32_t* cnt,
+             int* overflow)
+{
+    if (tier == 0 && mean_b <= 4.5)
+        mm_rows_t<4, 32, MODE>(ctx, A, B, C, cnt, overflow);
+    else if (tier == 0)
+        mm_rows_t<8, 32, MODE>(ctx, A, B, C, cnt, overflow);
+    else if (tier == 1 && mean_b <= 10.0)
+        mm_rows_t<8, 128, MODE>(ctx, A, B, C, cnt, overflow);
+    else if (tier == 1 && mean_b <= 20.0)
+        mm_rows_t<16, 128, MODE>(ctx, A, B, C, cnt, overflow);
+    else if (tier == 1)
+        mm_rows_t<32, 128, MODE>(ctx, A, B, C, cnt, overflow);
+    else if (tier == 2 && mean_b <= 20.0)
+        mm_rows_t<16, 256, MODE>(ctx, A, B, C, cnt, overflow);
+    else if (tier == 2)
+        mm_rows_t<32, 256, MODE>(ctx, A, B, C, cnt, overflow);
+    else
+        mm_rows_t<32, 512, MODE>(ctx, A, B, C, cnt, overflow);
+}
+
 template <int BS>
 void block_matmul(b2s_ctx* ctx, const BaijDev& A, const BaijDev& B, BaijDev& C)
 {
@@ -796,25 +936,33 @@ void block_matmul(b2s_ctx* ctx, const BaijDev& A, const BaijDev& B, BaijDev& C)
     C.nbc = B.nbc;
     DBuf<uint32_t> cnt(nr + 1);
     C.rp.alloc(nr + 1);
-    // symbolic: per-warp hash tables; rows too wide for them send the whole
-    // product to the candidate-sort path
+    // lanes by B's mean row, slots by the candidates of a row of C; a table that
+    // overflows is tried again at the next size, and past 512 columns the rows'
+    // candidates are sorted
+    const double mean_b = B.nbr ? (double)B.nnzb / B.nbr : 0.0, cand = nr ? (double)A.nnzb / nr * mean_b : 0.0;
+    int tier = cand <= 32.0 ? 0 : cand <= 1024.0 ? 1 : cand <= 8192.0 ? 2 : 3;
     DBuf<int> overflow(1);
-    B2S_CUDA(cudaMemsetAsync(overflow.p, 0, sizeof(int), ctx->stream));
-    const uint64_t hash_ctas = ((uint64_t)nr + kThreads / 32 - 1) / (kThreads / 32);
-    const unsigned hash_grid = (unsigned)std::max<uint64_t>(1, std::min<uint64_t>(hash_ctas, (uint64_t)ctx->sm_count * 8));
-    if (nr)
-        B2S_LAUNCH(ctx, k_mm_hash<true>, hash_grid, kThreads, 0, nr, A.rp.p, A.ci.p, B.rp.p, B.ci.p, cnt.p,
-                   (const uint32_t*)nullptr, (uint32_t*)nullptr, overflow.p);
-    uint32_t nnz = exclusive_scan(ctx, cnt.p, C.rp.p, nr);
+    uint32_t nnz = 0;
     int wide = 0;
-    d2h(ctx, &wide, overflow.p, sizeof(int));
-    sync(ctx);
+    for (; tier < 4; ++tier)
+    {
+        B2S_CUDA(cudaMemsetAsync(overflow.p, 0, sizeof(int), ctx->stream));
+        if (nr) mm_rows<MmMode::Count>(ctx, tier, mean_b, A, B, C, cnt.p, overflow.p);
+        nnz = exclusive_scan(ctx, cnt.p, C.rp.p, nr);
+        d2h(ctx, &wide, overflow.p, sizeof(int));
+        sync(ctx);
+        if (!wide) break;
+    }
+    bool values = false;
     if (!wide)
     {
         C.ci.alloc(nnz ? nnz : 1);
-        if (nr)
-            B2S_LAUNCH(ctx, k_mm_hash<false>, hash_grid, kThreads, 0, nr, A.rp.p, A.ci.p, B.rp.p, B.ci.p,
-                       (uint32_t*)nullptr, C.rp.p, C.ci.p, overflow.p);
+        C.v.alloc(nnz ? (size_t)nnz * BV : 1);
+        if (nr && BS == 1)
+            mm_rows<MmMode::Values>(ctx, tier, mean_b, A, B, C, nullptr, overflow.p);
+        else if (nr)
+            mm_rows<MmMode::Columns>(ctx, tier, mean_b, A, B, C, nullptr, overflow.p);
+        values = BS == 1;
     }
     else
     {
@@ -840,8 +988,8 @@ void block_matmul(b2s_ctx* ctx, const BaijDev& A, const BaijDev& B, BaijDev& C)
         C.ci.alloc(nnz ? nnz : 1);
         if (nr) B2S_LAUNCH(ctx, k_mm_unique_fill, stream_grid(ctx, nr), kThreads, 0, nr, off.p, sorted.p, C.rp.p, C.ci.p);
     }
-    C.v.alloc(nnz ? (size_t)nnz * BV : 1);
-    if (nr)
+    if (wide) C.v.alloc(nnz ? (size_t)nnz * BV : 1);
+    if (nr && !values)
     {
         // B's mean row length decides: warp per C row for long rows, thread per C row otherwise
         if (B.nbr && B.nnzb >= 8ull * B.nbr)
@@ -872,46 +1020,59 @@ __global__ void k_dense_from_baij(uint32_t nb, const uint32_t* __restrict__ rp, 
                     D[(size_t)(i * BS + r) * sz + ci[p] * BS + c] = v[(size_t)p * BV + r * BS + c];
 }
 
+// The coarsest operator fits shared memory up to this size (and a thread a row)
+constexpr int kDenseSmem = 160;
+inline size_t dense_smem(int sz) { return sz <= kDenseSmem ? (size_t)sz * (sz | 1) * sizeof(double) : 0; }
+
 // One CTA.  ref == 1: the reference's elimination (blockMatrix.hpp:962-981):
 // rows swapped, pivot clamped to +-1e-14, the multiplier column eliminated
 // along with the row (j from k).  ref == 0: LU with partial pivoting,
 // multipliers stored below the diagonal and the permutation kept in piv.
-__global__ void k_dense_factor(double* D, int sz, int ref, int* piv)
+// The matrix sits in shared memory (global memory past kDenseSmem), the pivot is
+// one warp's search and the update spreads over rows and columns: 47 unknowns
+// 0.557 -> 0.031 ms (one thread scanning the CTA's candidates and a thread a row).
+__global__ void __launch_bounds__(kThreads) k_dense_factor(double* Dg, int sz, int ref, int* piv)
 {
+    extern __shared__ __align__(16) double dense_sm[];
     __shared__ int s_pk;
-    __shared__ double s_red[kThreads];
-    __shared__ int s_idx[kThreads];
+    const bool in_smem = sz <= kDenseSmem;
+    double* const D = in_smem ? dense_sm : Dg;
+    const int ld = in_smem ? (sz | 1) : sz;
+    const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
+    constexpr int TY = kThreads / 32;
+    if (in_smem)
+        for (int i = ty; i < sz; i += TY)
+            for (int j = tx; j < sz; j += 32) D[i * ld + j] = Dg[(size_t)i * sz + j];
     for (int i = threadIdx.x; i < sz; i += blockDim.x) piv[i] = i;
     __syncthreads();
     for (int k = 0; k < sz; ++k)
     {
         // first row with the largest |D[i][k]|, i >= k (strict > keeps the earliest)
-        double best = -1.0;
-        int bi = k;
-        for (int i = k + threadIdx.x; i < sz; i += blockDim.x)
+        if (ty == 0)
         {
-            const double a = fabs(D[(size_t)i * sz + k]);
-            if (a > best)
+            double best = -1.0;
+            int bi = k;
+            for (int i = k + tx; i < sz; i += 32)
             {
-                best = a;
-                bi = i;
-            }
-        }
-        s_red[threadIdx.x] = best;
-        s_idx[threadIdx.x] = bi;
-        __syncthreads();
-        if (threadIdx.x == 0)
-        {
-            // the earliest row attaining the maximum, as the sequential scan finds it
-            double b = -1.0;
-            int pk = k;
-            for (int t = 0; t < (int)blockDim.x; ++t)
-                if (s_red[t] > b || (s_red[t] == b && s_idx[t] < pk))
+                const double a = fabs(D[(size_t)i * ld + k]);
+                if (a > best)
                 {
-                    b = s_red[t];
-                    pk = s_idx[t];
+                    best = a;
+                    bi = i;
                 }
-            s_pk = pk;
+            }
+#pragma unroll
+            for (int o = 16; o; o >>= 1)
+            {
+                const double b = __shfl_xor_sync(0xffffffffu, best, o);
+                const int i = __shfl_xor_sync(0xffffffffu, bi, o);
+                if (b > best || (b == best && i < bi))
+                {
+                    best = b;
+                    bi = i;
+                }
+            }
+            if (tx == 0) s_pk = bi;
         }
         __syncthreads();
         const int pk = s_pk;
@@ -919,9 +1080,9 @@ __global__ void k_dense_factor(double* D, int sz, int ref, int* piv)
         {
             for (int j = threadIdx.x; j < sz; j += blockDim.x)
             {
-                const double t = D[(size_t)k * sz + j];
-                D[(size_t)k * sz + j] = D[(size_t)pk * sz + j];
-                D[(size_t)pk * sz + j] = t;
+                const double t = D[(size_t)k * ld + j];
+                D[(size_t)k * ld + j] = D[(size_t)pk * ld + j];
+                D[(size_t)pk * ld + j] = t;
             }
             if (threadIdx.x == 0 && !ref)
             {
@@ -931,39 +1092,92 @@ __global__ void k_dense_factor(double* D, int sz, int ref, int* piv)
             }
         }
         __syncthreads();
-        double d = D[(size_t)k * sz + k];
+        const double raw = D[(size_t)k * ld + k];
+        double d = raw;
         if (ref)
         {
             if (fabs(d) < 1e-14) d = (d >= 0 ? 1e-14 : -1e-14);
         }
         else if (fabs(d) < 1e-300)
-        {
             d = 1e-300;
-            if (threadIdx.x == 0) D[(size_t)k * sz + k] = d;
-        }
-        for (int i = k + 1 + threadIdx.x; i < sz; i += blockDim.x)
+        __syncthreads();  // (the pivot is read before it is replaced)
+        if (!ref && d != raw && threadIdx.x == 0) D[(size_t)k * ld + k] = d;
+        // a warp a row: every lane forms the row's multiplier, then takes its columns
+        for (int i = k + 1 + ty; i < sz; i += TY)
         {
-            const double f = D[(size_t)i * sz + k] / d;
+            const double f = D[(size_t)i * ld + k] / d;
+            __syncwarp();
             if (ref)
-                for (int j = k; j < sz; ++j) D[(size_t)i * sz + j] -= f * D[(size_t)k * sz + j];
-            else
             {
-                D[(size_t)i * sz + k] = f;
-                for (int j = k + 1; j < sz; ++j) D[(size_t)i * sz + j] -= f * D[(size_t)k * sz + j];
+                if (tx == 0) D[(size_t)i * ld + k] -= f * raw;
             }
+            else if (tx == 0)
+                D[(size_t)i * ld + k] = f;
+            for (int j = k + 1 + tx; j < sz; j += 32) D[(size_t)i * ld + j] -= f * D[(size_t)k * ld + j];
         }
         __syncthreads();
     }
+    if (in_smem)
+        for (int i = ty; i < sz; i += TY)
+            for (int j = tx; j < sz; j += 32) Dg[(size_t)i * sz + j] = D[i * ld + j];
 }
 
-// coarsest solve, one thread (the row sums are sequential in the reference)
-__global__ void k_dense_solve(const double* __restrict__ D, int sz, int ref, const int* __restrict__ piv,
-                              const double* __restrict__ rhs, double* __restrict__ x, const int* done)
+// Coarsest solve, one CTA.  The reference's row sums are sequential: forward, row i
+// takes column j's term when x_j is known, so a thread a row works through the
+// columns together; backward, row i starts with x_{i+1}'s term, so the row's
+// products are formed side by side and subtracted by one thread in order.  47
+// unknowns 65 -> 17 us (one thread for all of it).
+__global__ void __launch_bounds__(kThreads) k_dense_solve(const double* __restrict__ Dg, int sz, int ref,
+                                                          const int* __restrict__ piv, const double* __restrict__ rhs,
+                                                          double* __restrict__ x, const int* done)
 {
     if (done && *done) return;
-    if (threadIdx.x != 0 || blockIdx.x != 0) return;
+    extern __shared__ __align__(16) double dense_sm[];
+    __shared__ double s_x[kDenseSmem], s_t[kDenseSmem];
+    const int t = threadIdx.x, tx = t & 31;
+    if (sz <= kDenseSmem)
+    {
+        const int ld = sz | 1;
+        for (int i = t >> 5; i < sz; i += kThreads / 32)
+            for (int j = tx; j < sz; j += 32) dense_sm[i * ld + j] = Dg[(size_t)i * sz + j];
+        auto pivot = [&](int i) {
+            const double d = dense_sm[i * ld + i];
+            return ref && fabs(d) < 1e-14 ? (d >= 0 ? 1e-14 : -1e-14) : d;
+        };
+        double xi = t < sz ? rhs[ref ? t : piv[t]] : 0.0;
+        __syncthreads();
+        for (int j = 0; j < sz; ++j)
+        {
+            if (t == j) s_x[j] = xi;
+            __syncthreads();
+            if (t > j && t < sz)
+            {
+                const double f = ref ? dense_sm[t * ld + j] / pivot(j) : dense_sm[t * ld + j];
+                xi -= f * s_x[j];
+            }
+        }
+        __syncthreads();
+        if (t >= 32) return;
+        for (int i = sz - 1; i >= 0; --i)
+        {
+            for (int j = i + 1 + tx; j < sz; j += 32) s_t[j] = dense_sm[i * ld + j] * s_x[j];
+            __syncwarp();
+            if (tx == 0)
+            {
+                double v = s_x[i];
+#pragma unroll 4
+                for (int j = i + 1; j < sz; ++j) v -= s_t[j];
+                s_x[i] = v / pivot(i);
+            }
+            __syncwarp();
+        }
+        for (int i = tx; i < sz; i += 32) x[i] = s_x[i];
+        return;
+    }
+    if (t != 0) return;
     // Each row's running value stays in a register while its terms are
     // subtracted in the same order as an in-place x[i] -= ... loop would.
+    const double* const D = Dg;
     if (ref)
     {
         for (int i = 0; i < sz; ++i) x[i] = rhs[i];
@@ -1132,7 +1346,7 @@ struct PcAMG final : PcImpl
         const unsigned g = stream_grid(ctx, L.nrows);
         if (l == (int)lv.size() - 1)
         {
-            B2S_LAUNCH(ctx, k_dense_solve, 1, 32, 0, dense.p, sz, ref_coarse ? 1 : 0, piv.p, rhs, sol, done);
+            B2S_LAUNCH(ctx, k_dense_solve, 1, kThreads, dense_smem(sz), dense.p, sz, ref_coarse ? 1 : 0, piv.p, rhs, sol, done);
             return;
         }
         // products on FP64 or FP32 values, each with its epilogue
@@ -1254,12 +1468,18 @@ void build_hierarchy(b2s_ctx* ctx, PcAMG& pc, const BaijDev& A0, int max_levels,
         }
         // strength
         DBuf<uint32_t> cnt(n + 1), sp(n + 1);
-        B2S_LAUNCH(ctx, k_strength<BS>, stream_grid(ctx, n), kThreads, 0, n, cur->rp.p, cur->ci.p, cur->v.p,
-                   (const uint32_t*)nullptr, cnt.p, (uint32_t*)nullptr);
+        // lanes a row of the setup kernels that walk rows: a warp where the rows are long
+        const bool long_rows = cur->nnzb >= 16ull * n && n <= 65536u;
+        const unsigned rows_grid = stream_grid(ctx, long_rows ? 32ull * n : n);
+        const auto strength = long_rows ? k_strength<BS, 32> : k_strength<BS, 1>;
+        const auto p_count = long_rows ? k_p_count<32> : k_p_count<1>;
+        const auto p_fill = long_rows ? k_p_fill<BS, 32> : k_p_fill<BS, 1>;
+        B2S_LAUNCH(ctx, strength, rows_grid, kThreads, 0, n, cur->rp.p, cur->ci.p, cur->v.p, (const uint32_t*)nullptr,
+                   cnt.p, (uint32_t*)nullptr);
         const uint32_t ns = exclusive_scan(ctx, cnt.p, sp.p, n);
         DBuf<uint32_t> sc(ns ? ns : 1);
-        B2S_LAUNCH(ctx, k_strength<BS>, stream_grid(ctx, n), kThreads, 0, n, cur->rp.p, cur->ci.p, cur->v.p, sp.p,
-                   (uint32_t*)nullptr, sc.p);
+        B2S_LAUNCH(ctx, strength, rows_grid, kThreads, 0, n, cur->rp.p, cur->ci.p, cur->v.p, sp.p, (uint32_t*)nullptr,
+                   sc.p);
         // aggregation
         L->agg.alloc(n);
         B2S_CUDA(cudaMemsetAsync(L->agg.p, 0xFF, (size_t)n * sizeof(int32_t), ctx->stream));
@@ -1284,12 +1504,12 @@ void build_hierarchy(b2s_ctx* ctx, PcAMG& pc, const BaijDev& A0, int max_levels,
         L->P.bs = BS;
         L->P.nbr = n;
         L->P.nbc = nagg;
-        B2S_LAUNCH(ctx, k_p_count, stream_grid(ctx, n), kThreads, 0, n, cur->rp.p, cur->ci.p, L->agg.p, cnt.p);
+        B2S_LAUNCH(ctx, p_count, rows_grid, kThreads, 0, n, cur->rp.p, cur->ci.p, L->agg.p, cnt.p);
         L->P.rp.alloc(n + 1);
         const uint32_t pn = exclusive_scan(ctx, cnt.p, L->P.rp.p, n);
         L->P.ci.alloc(pn ? pn : 1);
         L->P.v.alloc(pn ? (size_t)pn * BV : 1);
-        B2S_LAUNCH(ctx, k_p_fill<BS>, stream_grid(ctx, n), kThreads, 0, n, cur->rp.p, cur->ci.p, cur->v.p, L->dinv.p,
+        B2S_LAUNCH(ctx, p_fill, rows_grid, kThreads, 0, n, cur->rp.p, cur->ci.p, cur->v.p, L->dinv.p,
                    L->agg.p, L->P.rp.p, L->P.ci.p, L->P.v.p);
         finish_baij(ctx, L->P);
         block_transpose<BS>(ctx, L->P, L->R);
@@ -1325,7 +1545,9 @@ void build_hierarchy(b2s_ctx* ctx, PcAMG& pc, const BaijDev& A0, int max_levels,
     if (C.nrows)
         B2S_LAUNCH(ctx, k_dense_from_baij<BS>, stream_grid(ctx, C.nrows), kThreads, 0, C.nrows, C.A->rp.p, C.A->ci.p,
                    C.A->v.p, pc.dense.p, pc.sz);
-    B2S_LAUNCH(ctx, k_dense_factor, 1, kThreads, 0, pc.dense.p, pc.sz, pc.ref_coarse ? 1 : 0, pc.piv.p);
+    for (const void* kern : {(const void*)k_dense_factor, (const void*)k_dense_solve})
+        B2S_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dense_smem(kDenseSmem)));
+    B2S_LAUNCH(ctx, k_dense_factor, 1, kThreads, dense_smem(pc.sz), pc.dense.p, pc.sz, pc.ref_coarse ? 1 : 0, pc.piv.p);
     // FP32 copies of every operator the V-cycle multiplies by (the coarsest level is the dense LU, kept in FP64)
     if (pc.fp32)
         for (size_t k = 0; k + 1 < pc.lv.size(); ++k)

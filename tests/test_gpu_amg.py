@@ -165,6 +165,23 @@ def test_amg_wide_galerkin_rows(b2s, ctx, orc):
         assert np.array_equal(Arp, lv["Arp"]) and np.array_equal(Aci, lv["Aci"]) and np.array_equal(Av, lv["Av"]), k
 
 
+@pytest.mark.parametrize("n", [1, 2, 31, 33, 159, 160, 161, 300])
+def test_amg_dense_coarse_sizes(b2s, ctx, n):
+    """A hierarchy of one level is its dense factor: sizes around a warp and
+    around the largest one kept in shared memory.  The large entry of each row
+    sits beside the diagonal, so every column but the last pivots."""
+    rng = np.random.default_rng(n)
+    D = rng.uniform(-0.5, 0.5, (n, n)) / n + 0.01 * np.eye(n)
+    D[np.arange(n), (np.arange(n) + 1) % n] += 2.0
+    rp = (np.arange(n + 1) * n).astype(np.uint32)
+    B = b2s.BAIJ(ctx, 1, n, n, rp, np.tile(np.arange(n, dtype=np.uint32), n), D.reshape(-1))
+    M = b2s.Precond(ctx, B, b2s.PC_BSA_AMG, amg_coarse_max=n)
+    r = rng.uniform(-1, 1, n)
+    # off the permuted diagonal a row sums to under 0.6 of its large entry: condition below 5,
+    # growth below 2, so 3 n eps * 10 bounds the solve
+    assert np.linalg.norm(D @ M.apply(r) - r) <= 30 * n * 2.3e-16 * np.linalg.norm(r)
+
+
 @pytest.mark.parametrize("case", ["poisson2d_48", "poisson3d_16", "maxit"])
 def test_stationary_amg(b2s, ctx, orc, case):
     """SMatrix::amg (array.cpp:4534-4563) as B2S_STATIONARY with the SA V-cycle:

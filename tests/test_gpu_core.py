@@ -284,6 +284,34 @@ def test_csr_matmul_transpose(b2s, ctx, orc, ref, case):
     assert rel(C.spmv(x), A.spmv(B.spmv(x))) < 1e-13
 
 
+@pytest.mark.parametrize("mean", [1, 8, 16, 40])
+def test_csr_matmul_row_widths(b2s, ctx, orc, mean):
+    """Product rows on both sides of every size of the symbolic hash table
+    (32, 128, 256 and 512 columns), of one table filled to the last slot, and
+    empty ones, for each group of lanes that walks a row of B."""
+    widths = [0, 1, 31, 32, 33, 127, 128, 129, 255, 256, 257, 511, 512, 513, 700]
+    rng = np.random.default_rng(mean)
+    nb, m = 1500, 1024
+    cols = [np.sort(rng.choice(m, size=int(k), replace=False)) for k in rng.integers(0, 2 * mean + 1, nb)]
+    brp = np.concatenate([[0], np.cumsum([len(c) for c in cols])]).astype(np.uint32)
+    b = (nb, m, brp, np.concatenate(cols).astype(np.uint32), rng.uniform(-1, 1, int(brp[-1])))
+    rows = []
+    for w in widths:  # rows of B until the product row has about w columns
+        seen, row = set(), []
+        for k in rng.permutation(nb):
+            if len(seen | set(cols[k])) <= w and len(row) < 400:
+                seen |= set(cols[k])
+                row.append(k)
+            if len(seen) == w:
+                break
+        rows.append(np.sort(np.array(row, np.int64)))
+    arp = np.concatenate([[0], np.cumsum([len(r) for r in rows])]).astype(np.uint32)
+    a = (len(rows), nb, arp, np.concatenate(rows).astype(np.uint32), rng.uniform(-1, 1, int(arp[-1])))
+    C = b2s.CSR(ctx, *a).matmul(b2s.CSR(ctx, *b))
+    Co = orc.matmul(orc.csr(*a), orc.csr(*b)).export()
+    assert np.array_equal(C.rp, Co[0]) and np.array_equal(C.ci, Co[1]) and np.array_equal(C.v, Co[2])
+
+
 def test_csr_matmul_shape_error(b2s, ctx):
     n, rp, ci, v = P.poisson2d(8)
     A = b2s.CSR(ctx, n, n, rp, ci, v)
