@@ -35,7 +35,7 @@ void baij_partition(b2s_ctx* ctx, BaijDev& M, const uint32_t* h_rp)
     M.nblk = 0;
     if (M.bs != 1 || M.nbr == 0 || M.nnzb < (uint64_t)kBaijStagedMinRow * M.nbr) return;
     std::vector<uint32_t> blk;
-    build_row_blocks(h_rp, M.nbr, 1, kThreads, kBaijStagedCap, blk);
+    build_row_blocks(h_rp, M.nbr, 1, kThreads, baij_staged_cap(ctx, M.nnzb), blk);
     M.nblk = (uint32_t)blk.size() - 1;
     M.blk_row = upload(ctx, blk.data(), blk.size());
 }

@@ -93,61 +93,75 @@ __global__ void __launch_bounds__(kThreads, kBaijCtasPerSm)
 }
 
 
-
-
 // y = A x with the stored values v (A's pattern), every output component
 // handed to the epilogue: epi.put<BS>(I, r, y_Ir, valid, lane).  For BS >= 2
 // all 32 lanes of a warp call put together (valid false on idle lanes), so an
 // epilogue may exchange a block row's components with shuffles; the lanes of
 // block row I are lanes (lane / BS) * BS .. + BS - 1.  For BS = 1 a thread
 // calls put for its own rows only.
+//
 // 1x1 blocks with long rows (the coarse operators and restrictions of a
-// scalar AMG hierarchy, 30 to 100+ entries a row): a CTA stages a contiguous
-// range of entries (the partition in A.blk_row, at most kBaijStagedCap
-// entries) in shared memory and one thread per row sums its row from it.
-constexpr uint32_t kBaijStagedCap = 3072;
+// scalar AMG hierarchy, 30 to 100+ entries a row): a CTA takes a contiguous
+// range of at most kThreads rows (the partition in A.blk_row).  All its
+// threads load entries and gather x, so that the row length does not bound
+// the loads in flight, and leave the products in shared memory; then one
+// thread a row adds its products in column order.  Bound by the stream of
+// values and columns on the large levels and by the chain row pointers,
+// entries, x, sum on the small ones.  On the hierarchy of the 128^3 Poisson
+// grid, against one thread a row that also gathered its x from staged
+// columns: restriction of 7.2M entries 56 -> 33 us, operator of 6.2M entries
+// 46 -> 29, of 0.4M 14 -> 7, restriction of 60k entries 27 -> 8.
+constexpr uint32_t kBaijStagedCap = 2048;   // products a pass
+constexpr uint32_t kBaijStagedMin = 256;    // smallest share of a CTA
 constexpr uint32_t kBaijStagedMinRow = 16;  // mean entries per row from which the staged kernel is used
 
-__device__ __forceinline__ void stage_vals(double* s, const double* g, uint32_t cnt) { stage_f64(s, g, cnt); }
-
-__device__ __forceinline__ void stage_vals(float* s, const float* g, uint32_t cnt)
+// Entries a CTA's range may hold.  A full pass where the matrix gives every
+// SM several CTAs; less on the small levels, whose time is one CTA's chain.
+inline uint32_t baij_staged_cap(const b2s_ctx* ctx, uint64_t nnz)
 {
-    for (uint32_t i = threadIdx.x; i < cnt; i += blockDim.x) s[i] = __ldg(&g[i]);
+    const uint64_t share = nnz / (4ull * ctx->sm_count);
+    return (uint32_t)(share < kBaijStagedMin ? kBaijStagedMin : share > kBaijStagedCap ? kBaijStagedCap : share);
 }
 
 template <typename VT, class Epi>
-__global__ void __launch_bounds__(kThreads) k_baij_staged1(const uint32_t* __restrict__ rp, const uint32_t* __restrict__ ci,
-                                                           const VT* __restrict__ v,
-                                                           const uint32_t* __restrict__ blk_row,
-                                                           const double* __restrict__ x, Epi epi, const int* done)
+__global__ void __launch_bounds__(kThreads, 6)
+    k_baij_staged1(const uint32_t* __restrict__ rp, const uint32_t* __restrict__ ci, const VT* __restrict__ v,
+                   const uint32_t* __restrict__ blk_row, const double* __restrict__ x, Epi epi, const int* done)
 {
     if (done && *done) return;
-    __shared__ VT sv[kBaijStagedCap];
-    __shared__ uint32_t sc[kBaijStagedCap];
-    const uint32_t r0 = blk_row[blockIdx.x], r1 = blk_row[blockIdx.x + 1];
+    constexpr int U = kBaijStagedCap / kThreads;
+    __shared__ double P[kBaijStagedCap];
+    const uint32_t r0 = __ldg(&blk_row[blockIdx.x]), r1 = __ldg(&blk_row[blockIdx.x + 1]);
+    const uint32_t row = r0 + threadIdx.x;
+    const bool own = row < r1;
     const uint32_t p0 = __ldg(&rp[r0]), p1 = __ldg(&rp[r1]);
-    const uint32_t cnt = p1 - p0;
-    if (cnt <= kBaijStagedCap)
+    const uint32_t a = own ? __ldg(&rp[row]) : 0u, b = own ? __ldg(&rp[row + 1]) : 0u;
+    double sum = 0.0;
+    for (uint32_t base = p0, end; base < p1; base = end)  // one pass, unless a single row is longer
     {
-        stage_vals(sv, v + p0, cnt);
-        stage_u32(sc, ci + p0, cnt);
+        end = p1 - base < kBaijStagedCap ? p1 : base + kBaijStagedCap;
+        VT vv[U];
+        uint32_t cc[U];
+#pragma unroll
+        for (int k = 0; k < U; ++k)
+        {
+            const uint32_t q = base + k * kThreads + threadIdx.x;
+            vv[k] = q < end ? ld_stream(v + q) : (VT)0;
+            cc[k] = q < end ? ld_stream(ci + q) : 0u;
+        }
+#pragma unroll
+        for (int k = 0; k < U; ++k)
+        {
+            const uint32_t q = base + k * kThreads + threadIdx.x;
+            if (q < end) P[k * kThreads + threadIdx.x] = (double)vv[k] * __ldg(&x[cc[k]]);
+        }
         __syncthreads();
-        for (uint32_t br = r0 + threadIdx.x; br < r1; br += blockDim.x)
-        {
-            const uint32_t a = __ldg(&rp[br]) - p0, b = __ldg(&rp[br + 1]) - p0;
-            double yr = 0.0;
-            for (uint32_t k = a; k < b; ++k) yr += (double)sv[k] * __ldg(&x[sc[k]]);
-            epi.template put<1>(br, 0, yr, true, 0u);
-        }
+        const uint32_t lo = a > base ? a : base, hi = b < end ? b : end;
+#pragma unroll 8
+        for (uint32_t q = lo; q < hi; ++q) sum += P[q - base];
+        if (end < p1) __syncthreads();
     }
-    else
-        for (uint32_t br = r0 + threadIdx.x; br < r1; br += blockDim.x)
-        {
-            double yr = 0.0;
-            for (uint32_t k = __ldg(&rp[br]); k < __ldg(&rp[br + 1]); ++k)
-                yr += (double)__ldg(&v[k]) * __ldg(&x[__ldg(&ci[k])]);
-            epi.template put<1>(br, 0, yr, true, 0u);
-        }
+    if (own) epi.template put<1>(row, 0, sum, true, 0u);
 }
 
 // 1x1 blocks with short rows (the fine operator and the prolongation) use

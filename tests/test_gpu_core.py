@@ -284,6 +284,23 @@ def test_csr_matmul_transpose(b2s, ctx, orc, ref, case):
     assert rel(C.spmv(x), A.spmv(B.spmv(x))) < 1e-13
 
 
+@pytest.mark.parametrize("n,width", [(1, 1), (3, 40), (255, 16), (257, 17), (1000, 64), (40, 2048), (70, 6000)])
+def test_baij1_long_rows(b2s, ctx, orc, n, width):
+    """Scalar-block matvec with 16 and more entries a row: rows of no entry,
+    of a whole pass of a CTA, of several; one row; CTAs of 256 rows."""
+    rng = np.random.default_rng(n)
+    m = max(n, 2 * width)
+    lens = rng.integers(0, 2 * width, n)
+    lens[-1] = 2 * width - 1
+    lens[: n // 2 : 3] = 0
+    lens[n // 2 :] = np.maximum(lens[n // 2 :], min(width + width // 2, m))
+    cols = [np.sort(rng.choice(m, size=int(k), replace=False)) for k in lens]
+    rp = np.concatenate([[0], np.cumsum(lens)]).astype(np.uint32)
+    ci, v, x = np.concatenate(cols).astype(np.uint32), rng.uniform(-1, 1, int(rp[-1])), rng.uniform(-1, 1, m)
+    y = b2s.BAIJ(ctx, 1, n, m, rp, ci, v).matvec(x)
+    assert np.array_equal(y, orc.spmv(orc.csr(n, m, rp, ci, v), x))
+
+
 @pytest.mark.parametrize("mean", [1, 8, 16, 40])
 def test_csr_matmul_row_widths(b2s, ctx, orc, mean):
     """Product rows on both sides of every size of the symbolic hash table
