@@ -301,6 +301,24 @@ def test_baij1_long_rows(b2s, ctx, orc, n, width):
     assert np.array_equal(y, orc.spmv(orc.csr(n, m, rp, ci, v), x))
 
 
+@pytest.mark.parametrize("n", [1, 33, 1000, 60001])
+def test_spmv_warp_groups(b2s, ctx, orc, n):
+    """CSR product by groups of 32 rows: a last group of one row, empty rows
+    and whole empty groups, rows longer than a warp's chunk, several groups a
+    warp.  One row of 700 entries keeps the matrix off the row kernel."""
+    rng = np.random.default_rng(n)
+    m = max(n, 1024)
+    lens = rng.integers(0, 12, n)
+    lens[32 * 5 : 32 * 9] = 0
+    lens[[0, -1]] = 700
+    lens[n // 2] = 257
+    cols = [np.sort(rng.choice(m, size=int(k), replace=False)) if k > 20 else np.unique(rng.integers(0, m, int(k)))
+            for k in lens]
+    rp = np.concatenate([[0], np.cumsum([len(c) for c in cols])]).astype(np.uint32)
+    ci, v, x = np.concatenate(cols).astype(np.uint32), rng.uniform(-1, 1, int(rp[-1])), rng.uniform(-1, 1, m)
+    assert np.array_equal(b2s.CSR(ctx, n, m, rp, ci, v).spmv(x), orc.spmv(orc.csr(n, m, rp, ci, v), x))
+
+
 @pytest.mark.parametrize("mean", [1, 8, 16, 40])
 def test_csr_matmul_row_widths(b2s, ctx, orc, mean):
     """Product rows on both sides of every size of the symbolic hash table
