@@ -2,96 +2,161 @@
 // an epilogue, shared by the BAIJ operator (baij.cu) and the AMG V-cycle
 // (amg.cu), whose residual and smoothing updates ride on the products.
 //
-// Block matvec (bs >= 2): a warp owns 32/bs consecutive block rows (one lane
-// per output component) and walks their blocks min(32, 256/bs^2) at a time.  The
-// lanes stream the blocks' values into the warp's shared memory (coalesced,
-// no L1 allocation), lane b gathers x_J of block b and forms the block's bs
-// row dots with the reference's association (blk_row_dot), and the lane of
+// Block matvec (bs >= 2): a warp owns a contiguous range of block rows and
+// streams its blocks, 32 (16 of 4x4) a pass, through a two-stage ring in shared
+// memory: cp.async brings the next pass's values and columns while lane b
+// gathers x_J of block b of this one and forms the block's bs row dots with the
+// reference's association (blk_row_dot).  The dots go to a second ring, and
+// whenever the stream has passed the end of a group of 32/bs rows the lane of
 // output component (I, r) adds the dots of row I in block order -- the
 // reference's order, so y is bit-exact.  No CTA-wide barrier.
+//
+// Bound by the stream of values once the warp's chain (columns, x, dots, sums)
+// is covered: the sums are the serial part, 3 to 6 lanes wide when taken every
+// pass and a whole group wide from the ring.  64^3 Q1 elasticity, 3x3 (552 MB,
+// a copy of as many bytes takes 84 us): 127 us with register-staged passes
+// summed one by one at 32 warps an SM; here 99 us at 24 warps (20: 103, 32 with a
+// ring of half the size: 107, 16 with twice: 107; x gathered a pass ahead: 122,
+// three stages at 16 warps: 107).  The coarse products of the block hierarchies
+// gain more, their few rows now spread over all warps: V-cycle of 48^3 elements
+// 466 -> 221 us, of 10^3 172 -> 132.
 #pragma once
 #include "block_ops.cuh"
 #include "spmv_staged.cuh"
 
 namespace b2s {
 
+constexpr int kBaijThreads = 192;
 constexpr int kBaijCtasPerSm = 4;
 
+template <int BS, typename VT>
+struct alignas(16) BaijWarpSmem
+{
+    static constexpr int NB = BS <= 3 ? 32 : 256 / (BS * BS);  // blocks a pass, one lane each
+    static constexpr int RING = 4 * NB;                        // blocks whose dots are kept (a power of two)
+    VT val[2][NB * BS * BS];
+    uint32_t col[2][NB];
+    double dot[RING * BS];
+};
+
 // VT: stored value type (double, or float for the FP32 copies of the AMG
-// hierarchy); products and sums are FP64 either way.
+// hierarchy); products and sums are FP64 either way.  v is 16-byte aligned.
+// per: block rows a warp.
 template <int BS, typename VT, class Epi>
-__global__ void __launch_bounds__(kThreads, kBaijCtasPerSm)
-    k_baij_warp(uint32_t nbr, const uint32_t* __restrict__ rp, const uint32_t* __restrict__ ci,
+__global__ void __launch_bounds__(kBaijThreads, kBaijCtasPerSm)
+    k_baij_warp(uint32_t nbr, uint32_t per, const uint32_t* __restrict__ rp, const uint32_t* __restrict__ ci,
                 const VT* __restrict__ v, const double* __restrict__ x, Epi epi, const int* done)
 {
     if (done && *done) return;
-    constexpr int BV = BS * BS;
-    constexpr int GR = 32 / BS;                        // block rows per warp group
-    constexpr int NB = 256 / BV < 32 ? 256 / BV : 32;  // blocks per pass: one lane per block
-    constexpr int PER = (NB * BV + 31) / 32;           // value loads per lane per pass
-    __shared__ double sval[kThreads / 32][NB * BV];
-    __shared__ double sdot[kThreads / 32][NB * BS];
-    const uint32_t lane = threadIdx.x & 31u, wid = threadIdx.x >> 5;
-    double* V = sval[wid];
-    double* P = sdot[wid];
-    // one pass's operands in registers: its values and this lane's block column
-    auto load_pass = [&](uint32_t base, uint32_t nb, double* tv, uint32_t& J) {
-        const VT* vb = v + (size_t)base * BV;
-#pragma unroll
-        for (int k = 0; k < PER; ++k)
+    using Smem = BaijWarpSmem<BS, VT>;
+    constexpr int BV = BS * BS, NB = Smem::NB, RING = Smem::RING;
+    constexpr uint32_t GR = 32 / BS;                           // block rows a group
+    constexpr int CHUNKS = (NB * BV * (int)sizeof(VT) + 511) / 512;  // 16-byte copies a lane and pass
+    __shared__ Smem smem[kBaijThreads / 32];
+    const uint32_t lane = threadIdx.x & 31u, wid = threadIdx.x >> 5, r = lane % BS;
+    Smem& s = smem[wid];
+    const uint64_t begin = (uint64_t)(blockIdx.x * (kBaijThreads / 32) + wid) * per;
+    if (begin >= nbr) return;
+    const uint32_t R1 = (uint32_t)(begin + per < nbr ? begin + per : nbr);
+    uint32_t I0 = (uint32_t)begin;  // the group's first row
+    const uint32_t p0 = __ldg(&rp[I0]), p1 = __ldg(&rp[R1]);
+    const uint32_t first = p0 & ~3u;  // four blocks of any size and type are whole 16-byte units
+    const uint32_t passes = (p1 - first + NB - 1) / NB;
+    auto copy = [&](uint32_t i) {
+        if (i < passes)
         {
-            const uint32_t q = k * 32 + lane;
-            tv[k] = q < nb * BV ? (double)ld_stream(vb + q) : 0.0;
+            const uint32_t base = first + i * NB, nb = p1 - base < NB ? p1 - base : NB;
+            const uint32_t bytes = nb * BV * (uint32_t)sizeof(VT);
+            const char* src = reinterpret_cast<const char*>(v + (size_t)base * BV);
+            const uint32_t dst = (uint32_t)__cvta_generic_to_shared(s.val[i & 1u]);
+#pragma unroll
+            for (int k = 0; k < CHUNKS; ++k)
+            {
+                const uint32_t c = (k * 32 + lane) * 16u;
+                if (c < bytes)  // (the last unit may be part of one: the copy reads no further)
+                    asm volatile("cp.async.cg.shared.global.L2::128B [%0], [%1], 16, %2;" ::"r"(dst + c), "l"(src + c),
+                                 "r"(bytes - c < 16u ? bytes - c : 16u)
+                                 : "memory");
+            }
+            if (lane < nb)
+                asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(
+                                 (uint32_t)__cvta_generic_to_shared(&s.col[i & 1u][lane])),
+                             "l"(ci + base + lane)
+                             : "memory");
         }
-        J = lane < nb ? ld_stream(ci + base + lane) : 0u;
     };
-    const uint32_t ngroups = (nbr + GR - 1) / GR;
-    for (uint32_t g = blockIdx.x * (kThreads / 32) + wid; g < ngroups; g += gridDim.x * (kThreads / 32))
+    copy(0);
+    // the group: this lane's row [a, b), the group's end, and the next group's row
+    uint32_t a = 0, b = 0, gend = 0, na = 0, nb = 0;
+    bool out = false;
+    double acc = 0.0;
+    auto row_of = [&](uint32_t g0, uint32_t& ra, uint32_t& rb) {
+        const uint32_t I = g0 + lane / BS;
+        const bool on = lane < GR * BS && I < R1;
+        ra = on ? __ldg(&rp[I]) : 0u;
+        rb = on ? __ldg(&rp[I + 1]) : 0u;
+    };
+    row_of(I0, na, nb);
+    auto group = [&] {
+        const uint32_t rows = R1 - I0 < GR ? R1 - I0 : GR;
+        out = lane < rows * BS;
+        a = na;
+        b = nb;
+        gend = __shfl_sync(0xffffffffu, b, (rows - 1) * BS);
+        acc = 0.0;
+        row_of(I0 + GR, na, nb);
+    };
+    group();
+    uint32_t low = p0;  // dots of blocks below are summed
+    for (uint32_t i = 0; i < passes; ++i)
     {
-        const uint32_t I0 = g * GR;
-        const uint32_t rows = min((uint32_t)GR, nbr - I0);
-        const bool out = lane < rows * BS;
-        const uint32_t I = I0 + lane / BS;
-        const uint32_t r = lane % BS;
-        const uint32_t a = out ? __ldg(&rp[I]) : 0u, b = out ? __ldg(&rp[I + 1]) : 0u;
-        const uint32_t p0 = __shfl_sync(0xffffffffu, a, 0);
-        const uint32_t p1 = __shfl_sync(0xffffffffu, b, (rows - 1) * BS);
-        double acc = 0.0;
-        double tv[PER];
-        uint32_t J = 0;
-        if (p0 < p1) load_pass(p0, min((uint32_t)NB, p1 - p0), tv, J);
-        for (uint32_t base = p0; base < p1; base += NB)
+        asm volatile("cp.async.wait_all;" ::: "memory");
+        __syncwarp();
+        const uint32_t base = first + i * NB, end = p1 - base < NB ? p1 : base + NB, q = base + lane;
+        const bool on = lane < NB && q < end && q >= p0;
+        double xv[BS];
+        if (on)
         {
-            const uint32_t nb = min((uint32_t)NB, p1 - base);
+            const double* xj = x + (size_t)s.col[i & 1u][lane] * BS;
 #pragma unroll
-            for (int k = 0; k < PER; ++k)
-            {
-                const uint32_t q = k * 32 + lane;
-                if (q < nb * BV) V[q] = tv[k];
-            }
-            double xv[BS];
-            if (lane < nb)
-#pragma unroll
-                for (int c = 0; c < BS; ++c) xv[c] = __ldg(&x[(size_t)J * BS + c]);
-            // the next pass's operands load while this pass computes
-            const uint32_t nbase = base + NB;
-            if (nbase < p1) load_pass(nbase, min((uint32_t)NB, p1 - nbase), tv, J);
-            __syncwarp();
-            if (lane < nb)
-#pragma unroll
-                for (int r2 = 0; r2 < BS; ++r2) P[lane * BS + r2] = blk_row_dot<BS>(&V[lane * BV + r2 * BS], xv);
-            __syncwarp();
-            if (out)
-            {
-                const uint32_t lo = a > base ? a : base, hi = b < base + nb ? b : base + nb;
-                for (uint32_t k = lo; k < hi; ++k) acc += P[(k - base) * BS + r];
-            }
-            __syncwarp();
+            for (int c = 0; c < BS; ++c) xv[c] = __ldg(&xj[c]);
         }
-        epi.template put<BS>(I, r, acc, out, lane);
+        copy(i + 1);  // into the stage of pass i - 1
+        if (on)
+        {
+            double vv[BV];
+#pragma unroll
+            for (int e = 0; e < BV; ++e) vv[e] = (double)s.val[i & 1u][lane * BV + e];
+#pragma unroll
+            for (int c = 0; c < BS; ++c) s.dot[(q % RING) * BS + c] = blk_row_dot<BS>(&vv[c * BS], xv);
+        }
+        __syncwarp();
+        // sum the groups that end here; part of one when the ring has no room for another pass
+        while (I0 < R1 && (gend <= end || end - low > RING - NB))
+        {
+            const uint32_t to = b < end ? b : end;
+            if (out)
+#pragma unroll 4
+                for (uint32_t k = a > low ? a : low; k < to; ++k) acc += s.dot[(k % RING) * BS + r];
+            if (gend > end)
+            {
+                low = end;
+                break;
+            }
+            low = gend;
+            epi.template put<BS>(I0 + lane / BS, r, acc, out, lane);
+            I0 += GR;
+            if (I0 < R1) group();
+        }
+        __syncwarp();
+    }
+    while (I0 < R1)  // no blocks at all
+    {
+        epi.template put<BS>(I0 + lane / BS, r, acc, out, lane);
+        I0 += GR;
+        if (I0 < R1) group();
     }
 }
-
 
 // y = A x with the stored values v (A's pattern), every output component
 // handed to the epilogue: epi.put<BS>(I, r, y_Ir, valid, lane).  For BS >= 2
@@ -192,12 +257,13 @@ void baij_mv(b2s_ctx* ctx, const BaijDev& A, const VT* v, const double* x, Epi e
     }
     else
     {
-        constexpr int GR = 32 / BS;
-        const uint32_t groups = (A.nbr + GR - 1) / GR;
-        const uint32_t ctas = (groups + kThreads / 32 - 1) / (kThreads / 32);
-        const uint32_t cap = (uint32_t)ctx->sm_count * kBaijCtasPerSm;
-        B2S_LAUNCH(ctx, (k_baij_warp<BS, VT, Epi>), ctas < cap ? ctas : cap, kThreads, 0, A.nbr, A.rp.p, A.ci.p, v,
-                   x, epi, done);
+        // one wave of warps, the rows dealt evenly
+        constexpr uint32_t W = kBaijThreads / 32;
+        const uint32_t warps = (uint32_t)ctx->sm_count * kBaijCtasPerSm * W;
+        const uint32_t per = (A.nbr + warps - 1) / warps;
+        const uint32_t used = (A.nbr + per - 1) / per;
+        B2S_LAUNCH(ctx, (k_baij_warp<BS, VT, Epi>), (used + W - 1) / W, kBaijThreads, 0, A.nbr, per, A.rp.p, A.ci.p,
+                   v, x, epi, done);
     }
 }
 

@@ -96,6 +96,29 @@ def test_baij_matvec_irregular(b2s, ctx, orc, bs):
     assert np.array_equal(B.matvec(x), orc.blk_matvec(Bo, x))
 
 
+@pytest.mark.parametrize("bs", [2, 3, 4])
+@pytest.mark.parametrize("nb", [1, 3553, 60001])
+def test_baij_matvec_streams(b2s, ctx, orc, bs, nb):
+    # a warp's range of several row groups: empty groups and ranges, rows longer
+    # than the ring of dots, ranges that start at any block
+    rng = np.random.default_rng(nb)
+    lens = rng.integers(0, 30, nb)
+    lens[nb // 3:nb // 3 + 50] = 0
+    lens[::1009] = 1 if nb == 1 else 300
+    rp = np.concatenate([[0], np.cumsum(lens)])
+    gaps = rng.integers(1, 4, rp[-1])
+    walk = np.concatenate([[0], np.cumsum(gaps)])
+    start = rng.integers(0, max(1, nb - 1200), nb)
+    row = np.repeat(np.arange(nb), lens)
+    ci = (start[row] + walk[:-1] - walk[rp[row]]).astype(np.uint32)
+    rp = rp.astype(np.uint32)
+    v = rng.uniform(-1, 1, len(ci) * bs * bs)
+    B = b2s.BAIJ(ctx, bs, nb, nb, rp, ci, v)
+    Bo = orc.blk(bs, nb, nb, rp, ci, v)
+    x = rng.uniform(-1, 1, nb * bs)
+    assert np.array_equal(B.matvec(x), orc.blk_matvec(Bo, x))
+
+
 def test_baij_elasticity_matvec(b2s, ctx, orc):
     nbr, rp, ci, v = b2s.gen_elasticity_q1(10)
     B = b2s.BAIJ(ctx, 3, nbr, nbr, rp, ci, v)
