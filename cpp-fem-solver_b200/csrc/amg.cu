@@ -68,13 +68,7 @@ void finish_baij(b2s_ctx* ctx, BaijDev& M)
         B2S_LAUNCH(ctx, k_find_diag, stream_grid(ctx, M.nbr), kThreads, 0, M.nbr, M.rp.p, M.ci.p, M.diag_ptr.p);
     d2h(ctx, &M.nnzb, M.rp.p + M.nbr, sizeof(uint32_t));
     sync(ctx);
-    if (M.bs == 1 && M.nbr && M.nnzb >= (uint64_t)kBaijStagedMinRow * M.nbr)
-    {
-        std::vector<uint32_t> h_rp(M.nbr + 1);
-        d2h(ctx, h_rp.data(), M.rp.p, (M.nbr + 1) * sizeof(uint32_t));
-        sync(ctx);
-        baij_partition(ctx, M, h_rp.data());
-    }
+    baij_partition(ctx, M);
 }
 
 template <int BS>

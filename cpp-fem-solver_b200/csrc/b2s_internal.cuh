@@ -221,8 +221,8 @@ struct BaijDev
 };
 
 // Row partition of a bs = 1 BAIJ with long rows for its staged matvec
-// (nothing for other operators); h_rp: the host row pointers.
-void baij_partition(b2s_ctx* ctx, BaijDev& M, const uint32_t* h_rp);
+// (nothing for other operators), from its device arrays.
+void baij_partition(b2s_ctx* ctx, BaijDev& M);
 
 // Preconditioner implementation.  apply() enqueues z = M^-1 r on ctx->stream
 // (device pointers).  `done` (device, may be null) lets the Krylov drivers

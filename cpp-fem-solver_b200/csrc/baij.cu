@@ -30,14 +30,36 @@ void baij_matvec_f32(b2s_ctx* ctx, const BaijDev& A, const float* v32, const dou
     baij_matvec_t<float>(ctx, A, v32, x, y, done);
 }
 
-void baij_partition(b2s_ctx* ctx, BaijDev& M, const uint32_t* h_rp)
+// Rows of CTA c: those whose weight -- entries before them, and kBaijStagedRow
+// for each row before them -- lies in [c, c + 1) times share.
+static __global__ void k_baij_split(uint32_t nbr, const uint32_t* __restrict__ rp, uint32_t share, uint32_t nblk,
+                                    uint32_t* __restrict__ blk_row)
+{
+    for (uint32_t c = blockIdx.x * blockDim.x + threadIdx.x; c <= nblk; c += gridDim.x * blockDim.x)
+    {
+        const uint64_t target = (uint64_t)c * share;
+        uint32_t lo = 0, hi = nbr;  // the first row of at least that weight
+        while (lo < hi)
+        {
+            const uint32_t mid = lo + (hi - lo) / 2;
+            if (rp[mid] + (uint64_t)kBaijStagedRow * mid < target)
+                lo = mid + 1;
+            else
+                hi = mid;
+        }
+        blk_row[c] = lo;
+    }
+}
+
+void baij_partition(b2s_ctx* ctx, BaijDev& M)
 {
     M.nblk = 0;
     if (M.bs != 1 || M.nbr == 0 || M.nnzb < (uint64_t)kBaijStagedMinRow * M.nbr) return;
-    std::vector<uint32_t> blk;
-    build_row_blocks(h_rp, M.nbr, 1, kThreads, baij_staged_cap(ctx, M.nnzb), blk);
-    M.nblk = (uint32_t)blk.size() - 1;
-    M.blk_row = upload(ctx, blk.data(), blk.size());
+    const uint64_t weight = M.nnzb + (uint64_t)kBaijStagedRow * M.nbr;
+    const uint32_t share = baij_staged_share(ctx, M.nbr, M.nnzb);
+    M.nblk = (uint32_t)((weight + share - 1) / share);
+    M.blk_row.alloc(M.nblk + 1);
+    B2S_LAUNCH(ctx, k_baij_split, stream_grid(ctx, M.nblk + 1), kThreads, 0, M.nbr, M.rp.p, share, M.nblk, M.blk_row.p);
 }
 
 // ------------------------------------------------------------ block Jacobi
@@ -163,7 +185,7 @@ b2s_status b2s_baij_create(b2s_ctx* ctx, int bs, uint32_t nbr, uint32_t nbc, con
         d.ci = upload(ctx, col_idx, nnzb);
         d.v = upload(ctx, values, (size_t)nnzb * bs * bs);
         d.diag_ptr = upload(ctx, diag.data(), nbr);
-        baij_partition(ctx, d, row_ptr);
+        baij_partition(ctx, d);
         sync(ctx);
     });
     if (st != B2S_OK)

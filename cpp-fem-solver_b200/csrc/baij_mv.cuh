@@ -176,16 +176,25 @@ __global__ void __launch_bounds__(kBaijThreads, kBaijCtasPerSm)
 // grid, against one thread a row that also gathered its x from staged
 // columns: restriction of 7.2M entries 56 -> 33 us, operator of 6.2M entries
 // 46 -> 29, of 0.4M 14 -> 7, restriction of 60k entries 27 -> 8.
+//
+// The partition is cut on the device by a weight that grows with entries and
+// rows, so that both are bounded (k_baij_split): greedy blocks needed the row
+// pointers on the host, 0.3 to 0.6 ms for each of the three large operators of
+// that hierarchy (set-up 9.6 -> 8.6 ms).
 constexpr uint32_t kBaijStagedCap = 2048;   // products a pass
-constexpr uint32_t kBaijStagedMin = 256;    // smallest share of a CTA
+constexpr uint32_t kBaijStagedMin = 256;    // entries of the smallest share of a CTA
+constexpr uint32_t kBaijStagedRow = 16;     // weight of a row besides its entries
 constexpr uint32_t kBaijStagedMinRow = 16;  // mean entries per row from which the staged kernel is used
 
-// Entries a CTA's range may hold.  A full pass where the matrix gives every
-// SM several CTAs; less on the small levels, whose time is one CTA's chain.
-inline uint32_t baij_staged_cap(const b2s_ctx* ctx, uint64_t nnz)
+// The weight of a CTA's rows.  About a full pass of mean rows, and no more rows
+// than threads, where the matrix gives every SM several CTAs; less on the small
+// levels, whose time is one CTA's chain.
+inline uint32_t baij_staged_share(const b2s_ctx* ctx, uint64_t rows, uint64_t nnz)
 {
-    const uint64_t share = nnz / (4ull * ctx->sm_count);
-    return (uint32_t)(share < kBaijStagedMin ? kBaijStagedMin : share > kBaijStagedCap ? kBaijStagedCap : share);
+    const uint64_t mean = (nnz + rows - 1) / rows;
+    const uint64_t full = mean < kBaijStagedCap / 2 ? kBaijStagedCap - mean : kBaijStagedCap / 2;
+    const uint64_t entries = std::min(std::max<uint64_t>(nnz / (4ull * ctx->sm_count), kBaijStagedMin), full);
+    return (uint32_t)std::min(entries * (nnz + kBaijStagedRow * rows) / nnz, (uint64_t)kBaijStagedRow * kThreads);
 }
 
 template <typename VT, class Epi>
