@@ -24,6 +24,28 @@ def test_ssor_colouring_and_apply(b2s, ctx, orc, mat):
         assert np.array_equal(M.apply(r), po.apply(r))
 
 
+@pytest.mark.parametrize("n,links", [(1, 0), (7, 0), (2, 1), (300, 1), (301, 1), (301, 3)])
+def test_ssor_colour_counts(b2s, ctx, orc, n, links):
+    # one colour (no links), two (a path or an even ring), three and more (an odd
+    # ring, longer links), with entries on one side of the diagonal only among them
+    rng = np.random.default_rng(n + links)
+    d = np.zeros((n, n))
+    for k in range(1, links + 1):
+        for i in range(n):
+            d[i, (i + k) % n] = rng.uniform(-1, 1)
+            if i % 3:
+                d[(i + k) % n, i] = rng.uniform(-1, 1)
+    d[np.arange(n), np.arange(n)] = rng.uniform(4, 8, n) * rng.choice([-1, 1], n)
+    row, col = np.nonzero(d)
+    rp = np.concatenate([[0], np.cumsum(np.bincount(row, minlength=n))]).astype(np.uint32)
+    ci, v = col.astype(np.uint32), d[row, col]
+    M = b2s.Precond(ctx, b2s.CSR(ctx, n, n, rp, ci, v), b2s.PC_SSOR)
+    r = rng.uniform(-1, 1, n)
+    r[::5] = -0.0
+    z, want = M.apply(r), orc.pc(orc.csr(n, n, rp, ci, v), "ssor", 1.2).apply(r)
+    assert np.array_equal(z, want) and np.array_equal(np.signbit(z), np.signbit(want))
+
+
 def test_ssor_bad_omega(b2s, ctx):
     n, rp, ci, v = P.poisson2d(5)
     A = b2s.CSR(ctx, n, n, rp, ci, v)
