@@ -180,7 +180,7 @@ struct b2s_ctx
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
     // device error word (B2S_TIMEOUT from a bounded wait); counter[32..]
     int* errword() { return reinterpret_cast<int*>(counter.p + 32); }
-    // bounds of the chunked triangular solves' waits (b2s_ctx_set_wait_limits)
+    // bounds of the device-side waits (b2s_ctx_set_wait_limits)
     unsigned wait_fast_polls = 1u << 20;
     unsigned wait_slow_polls = 1u << 20;
 };
@@ -189,6 +189,15 @@ namespace b2s {
 // Reads the context's device error word (synchronises); a set word is
 // cleared and raised as its status (B2S_TIMEOUT: a bounded wait gave up).
 void check_device_error(b2s_ctx* ctx, const char* where);
+
+// Polls of one wait of the kernels that never sleep (grid schedules, level-order
+// traversal, sums over a persistent kernel's grid) before it gives up
+// (B2S_TIMEOUT): the context's wait bounds, spin and sleep budgets together.
+inline unsigned grid_polls(const b2s_ctx* ctx)
+{
+    const uint64_t p = (uint64_t)ctx->wait_fast_polls + ctx->wait_slow_polls;
+    return (unsigned)std::min<uint64_t>(std::max<uint64_t>(p, 1), 0xffffffffu);
+}
 }
 
 namespace b2s {

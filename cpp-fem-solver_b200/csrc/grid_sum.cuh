@@ -8,9 +8,9 @@
 // bits.  It is a grid barrier too, but orders no other memory: what the CTAs
 // exchange besides carries the epoch in its own words.  Two sets of lines
 // alternate: a CTA writes a set again only after a sum over the other one, which
-// every CTA took part in after it had read this one.  A wait ends after
-// kGridSumPolls polls: the CTA records B2S_TIMEOUT and leaves, the others give up
-// at their next sum, and the launch ends.
+// every CTA took part in after it had read this one.  A wait ends after polls_max
+// polls (grid_polls: the context's wait limits): the CTA records B2S_TIMEOUT and
+// leaves, the others give up at their next sum, and the launch ends.
 //
 // It costs two trips through L2 and their spread over the SMs, about 2 us on 148
 // CTAs.  A line for every pair of CTAs instead of one polled by all was no faster
@@ -20,7 +20,6 @@
 
 namespace b2s {
 
-constexpr unsigned kGridSumPolls = 1u << 21;  // about a second
 constexpr uint32_t kGridSumMaxCtas = 160;  // pollers: threads 32 .. 32 + CTAs - 1 of at least 256
 constexpr uint32_t kGridSumStride = 16;    // words between two CTAs' lines
 
@@ -76,7 +75,7 @@ __device__ __forceinline__ void grid_sum_post(GridSum<NT, ROOM>& s, unsigned lon
 // The sums; false (in every thread of the CTA) when a wait gave up.
 template <int NT, int ROOM, int NV>
 __device__ __forceinline__ bool grid_sum_wait(GridSum<NT, ROOM>& s, const unsigned long long* lines, uint32_t epoch,
-                                              double (&sum)[NV], int* err)
+                                              double (&sum)[NV], int* err, unsigned polls_max)
 {
     const uint32_t tid = threadIdx.x, lane = tid & 31u, ctas = gridDim.x;
     if (tid - 32u < ctas)  // (the first warp publishes)
@@ -84,7 +83,7 @@ __device__ __forceinline__ bool grid_sum_wait(GridSum<NT, ROOM>& s, const unsign
         const unsigned long long* w = lines + ((size_t)(epoch & 1u) * ctas + (tid - 32u)) * kGridSumStride;
         unsigned long long lo[NV], hi[NV];
         bool seen = false;
-        for (unsigned polls = 0; polls < kGridSumPolls && !seen; ++polls)
+        for (unsigned polls = 0; polls < polls_max && !seen; ++polls)
         {
             seen = true;
 #pragma unroll
@@ -143,7 +142,8 @@ __device__ __forceinline__ double warp_sum_down(double a)
 
 template <int S>
 __device__ __forceinline__ bool block_sum(BlockSum& s, unsigned long long* lines, uint32_t epoch, uint32_t blocks,
-                                          uint32_t vb, const double (&term)[S], double& sum, int* err)
+                                          uint32_t vb, const double (&term)[S], double& sum, int* err,
+                                          unsigned polls_max)
 {
     static_assert(S <= 4, "at most 8 blocks a CTA");
     constexpr uint32_t W = kThreads / 32;
@@ -177,7 +177,7 @@ __device__ __forceinline__ bool block_sum(BlockSum& s, unsigned long long* lines
         const unsigned long long* w = lines + (size_t)kGridSumStride * (b / vb) + 2u * (b % vb);
         unsigned long long lo = 0, hi = 0;
         bool seen = false;
-        for (unsigned polls = 0; polls < kGridSumPolls && !seen; ++polls)
+        for (unsigned polls = 0; polls < polls_max && !seen; ++polls)
         {
             asm volatile("ld.relaxed.gpu.global.v2.u64 {%0, %1}, [%2];" : "=l"(lo), "=l"(hi) : "l"(w) : "memory");
             seen = (uint32_t)(lo >> 32) == epoch && (uint32_t)(hi >> 32) == epoch;

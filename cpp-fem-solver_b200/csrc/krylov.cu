@@ -314,6 +314,7 @@ struct PcgSmallArgs
     unsigned long long* lines;  // two regions of grid_sum_words
     KState* st;
     int* err;
+    unsigned polls_max;  // of one wait
 };
 
 // the largest |i - j| of a pattern
@@ -418,7 +419,7 @@ __global__ void __launch_bounds__(kPcgSmallThreads, 1) k_pcg_small(PcgSmallArgs 
         }
         ++epoch;
         grid_sum_post(gs, a.lines, epoch, one);
-        if (!grid_sum_wait(gs, a.lines, epoch, pAp, a.err)) break;
+        if (!grid_sum_wait(gs, a.lines, epoch, pAp, a.err, a.polls_max)) break;
         if (!(pAp[0] >= kBreak))  // breakdown, not SPD or NaN: the state's own test decides
         {
             __syncthreads();
@@ -463,7 +464,7 @@ __global__ void __launch_bounds__(kPcgSmallThreads, 1) k_pcg_small(PcgSmallArgs 
             {
                 unsigned long long wl = 0, wh = 0;
                 bool seen = false;
-                for (unsigned polls = 0; polls < kGridSumPolls && !seen; ++polls)
+                for (unsigned polls = 0; polls < a.polls_max && !seen; ++polls)
                 {
                     asm volatile("ld.relaxed.gpu.global.v2.u64 {%0, %1}, [%2];"
                                  : "=l"(wl), "=l"(wh)
@@ -478,7 +479,7 @@ __global__ void __launch_bounds__(kPcgSmallThreads, 1) k_pcg_small(PcgSmallArgs 
                 }
                 zh[k] = __longlong_as_double((long long)((wh << 32) | (wl & 0xffffffffull)));
             }
-        if (!grid_sum_wait(gs, a.lines + grid_sum_words(gridDim.x), epoch, tot, a.err)) break;
+        if (!grid_sum_wait(gs, a.lines + grid_sum_words(gridDim.x), epoch, tot, a.err, a.polls_max)) break;
         rr = tot[0];
         if (tot[0] > clear && tot[0] < HUGE_VAL && tot[1] > 0.0 && it + 1 < maxit)
         {
@@ -545,7 +546,7 @@ static bool pcg_small(b2s_ctx* ctx, const CsrDev& A, const double* d, double* x,
     DBuf<unsigned long long> words(2 * grid_sum_words(ctas) + 2 * (size_t)A.n);
     B2S_CUDA(cudaMemsetAsync(words.p, 0, words.bytes(), ctx->stream));
     unsigned long long* zw = words.p + 2 * grid_sum_words(ctas);
-    PcgSmallArgs a{A.n, rows, band, A.rp.p, A.ci.p, A.v.p, d, x, r, z, p, zw, words.p, st, ctx->errword()};
+    PcgSmallArgs a{A.n, rows, band, A.rp.p, A.ci.p, A.v.p, d, x, r, z, p, zw, words.p, st, ctx->errword(), grid_polls(ctx)};
     void* params[] = {&a};
     B2S_CUDA(cudaLaunchCooperativeKernel(kern, dim3(ctas), dim3(NT), params, smem, ctx->stream));
     note_launch(ctx, "k_pcg_small");
@@ -943,6 +944,7 @@ struct GmMgsArgs
     unsigned long long* lines;
     uint32_t epoch;  // the first sum's
     int* err;
+    unsigned polls_max;  // of one wait
 };
 
 // S: blocks a thread belongs to, K: elements it has in each
@@ -979,6 +981,12 @@ __global__ void __launch_bounds__(kMgsThreads, 1) k_gm_mgs(GmMgsArgs a, const in
         const uint64_t e = at(q / K, q % K);
         w[q] = e < a.n ? a.w[e] : 0.0;
     }
+    // a sum that gave up ends the solve, or the host's cycles, which wait for the
+    // column's end to be recorded, would go on for ever
+    auto gave_up = [&] {
+        asm volatile("cp.async.wait_group 0;" ::: "memory");  // V_{i+1} may be on its way
+        if (threadIdx.x == 0) finish(a.st, B2S_TIMEOUT);
+    };
     __syncthreads();
     uint32_t epoch = a.epoch;
     for (int i = 0; i <= a.j; ++i)
@@ -994,7 +1002,7 @@ __global__ void __launch_bounds__(kMgsThreads, 1) k_gm_mgs(GmMgsArgs a, const in
 #pragma unroll
         for (int q = 0; q < S * K; ++q)
             if (at(q / K, q % K) < a.n) acc[q / K] += w[q] * v[q * kMgsThreads];
-        if (!block_sum(bs, a.lines, epoch++, a.blocks, a.vb, acc, h, a.err)) return;
+        if (!block_sum(bs, a.lines, epoch++, a.blocks, a.vb, acc, h, a.err, a.polls_max)) return gave_up();
         if (blockIdx.x == 0 && threadIdx.x == 0) a.sm.H[(size_t)i * a.sm.m + a.j] = h;
 #pragma unroll
         for (int q = 0; q < S * K; ++q)
@@ -1007,7 +1015,7 @@ __global__ void __launch_bounds__(kMgsThreads, 1) k_gm_mgs(GmMgsArgs a, const in
 #pragma unroll
     for (int q = 0; q < S * K; ++q)
         if (at(q / K, q % K) < a.n) acc[q / K] += w[q] * w[q];
-    if (!block_sum(bs, a.lines, epoch, a.blocks, a.vb, acc, ww, a.err)) return;
+    if (!block_sum(bs, a.lines, epoch, a.blocks, a.vb, acc, ww, a.err, a.polls_max)) return gave_up();
     const double hn = sqrt(ww);  // gm_column_tail's H[j+1][j]
     if (hn > kBreak)
     {
@@ -1062,7 +1070,7 @@ struct GmMgs
     void run(b2s_ctx* ctx, uint64_t n, uint64_t pn, const double* w, double* V, KState* st, const GmSmall& sm, int j,
              const int* skip)
     {
-        GmMgsArgs a{n, pn, blocks, vb, w, V, st, sm, j, lines.p, epoch, ctx->errword()};
+        GmMgsArgs a{n, pn, blocks, vb, w, V, st, sm, j, lines.p, epoch, ctx->errword(), grid_polls(ctx)};
         epoch += (uint32_t)j + 2u;
         void* params[] = {&a, &skip};
         B2S_CUDA(cudaLaunchCooperativeKernel(kern, dim3(ctas), dim3(kMgsThreads), params, smem, ctx->stream));
@@ -1861,8 +1869,8 @@ static b2s_status solve_common(b2s_ctx* ctx, const Operator& A, b2s_pc* pc, b2s_
         run_method(S, method, d_b, d_x, stats);
     }
     if (stats && pc) stats->setup_ms = 0.0;
-    // a bounded wait of a triangular solve that gave up fails the solve
-    check_device_error(ctx, "a triangular-solve wait gave up during the solve");
+    // a bounded device-side wait that gave up fails the solve
+    check_device_error(ctx, "a device-side wait gave up during the solve");
     const int st = stats ? stats->status : B2S_OK;
     if (!stats)
     {

@@ -1024,6 +1024,7 @@ struct PcIC0 final : PcImpl
         a.yw = a.zw + n;
         a.st = st;
         a.err = reinterpret_cast<int*>(pcg_ctl.p + 1);
+        a.polls_max = grid_polls(ctx);
         a.stall_window = stall_window;
         bool ok = false;
         switch (tile_Q * 2 + (tile_fused ? 1 : 0))

@@ -27,7 +27,7 @@
 // grid (grid_sum.cuh) is on its way.  No store needs a fence, and a phase starts
 // with its operands in registers.  512^2, 6 sweeps: 20.0 us an iteration with the
 // vectors behind fenced all-reduces, about 15 us this way.  Each wait is bounded
-// (kGridSumPolls polls): a CTA that gives up records B2S_TIMEOUT and leaves, and
+// (polls_max polls): a CTA that gives up records B2S_TIMEOUT and leaves, and
 // the others give up at their next sum, so the launch always ends.
 #pragma once
 
@@ -56,6 +56,7 @@ struct PcgTileArgs
     unsigned long long* lines;      // two regions of grid_sum_words, zero at launch
     KState* st;
     int* err;
+    unsigned polls_max;  // of one wait
     int stall_window;
 };
 
@@ -86,10 +87,11 @@ __device__ __forceinline__ bool tile_get(const unsigned long long* w, uint32_t e
 }
 // another tile's value of this iteration
 template <typename T>
-__device__ __forceinline__ T tile_await(const unsigned long long* w, uint32_t epoch, int* failed, int* err)
+__device__ __forceinline__ T tile_await(const unsigned long long* w, uint32_t epoch, int* failed, int* err,
+                                        unsigned polls_max)
 {
     T v;
-    for (unsigned polls = 0; polls < kGridSumPolls; ++polls)
+    for (unsigned polls = 0; polls < polls_max; ++polls)
         if (tile_get(w, epoch, v)) return v;
     *failed = 1;
     atomicCAS(err, 0, (int)B2S_TIMEOUT);
@@ -289,7 +291,7 @@ __global__ void __launch_bounds__(kTileThreads, 1) k_pcg_tile(PcgTileArgs a)
             }
             for (uint32_t t = tid + NT; t < n_ring; t += NT)
             {
-                const float zt = epoch ? tile_await<float>(&a.zw[ahalo[t]], epoch, &gs.failed, a.err) : (float)a.z[ahalo[t]];
+                const float zt = epoch ? tile_await<float>(&a.zw[ahalo[t]], epoch, &gs.failed, a.err, a.polls_max) : (float)a.z[ahalo[t]];
                 pe[n_own + t] = pl[t] = (double)zt + beta * pl[t];
             }
             ++epoch;
@@ -316,9 +318,9 @@ __global__ void __launch_bounds__(kTileThreads, 1) k_pcg_tile(PcgTileArgs a)
             {
                 const uint32_t t = tid + NT * q;
                 if (t >= n_own && t < n_el)
-                    Apv[q] = tile_await<double>(&a.apw[2 * (size_t)lower_row(t)], epoch, &gs.failed, a.err);
+                    Apv[q] = tile_await<double>(&a.apw[2 * (size_t)lower_row(t)], epoch, &gs.failed, a.err, a.polls_max);
             }
-            if (!grid_sum_wait(gs, lines1, epoch, tot, a.err)) break;
+            if (!grid_sum_wait(gs, lines1, epoch, tot, a.err, a.polls_max)) break;
             if (tid == 0) pcg_alpha(&sst, tot[0]);
             __syncthreads();
             if (sst.done) break;
@@ -375,7 +377,7 @@ __global__ void __launch_bounds__(kTileThreads, 1) k_pcg_tile(PcgTileArgs a)
                     rr[q] = in ? yf[t] : 0.f;
                 else
                     rr[q] = t < n_own ? yf[t]
-                            : in      ? tile_await<float>(&a.yw[uhalo[t - n_own]], epoch, &gs.failed, a.err)
+                            : in      ? tile_await<float>(&a.yw[uhalo[t - n_own]], epoch, &gs.failed, a.err, a.polls_max)
                                       : 0.f;
             }
             const float* yk = tile_sweeps<Q>(a.k, s_ucnt, dep, val, di, rr, y0, y1, dummy);
@@ -392,8 +394,8 @@ __global__ void __launch_bounds__(kTileThreads, 1) k_pcg_tile(PcgTileArgs a)
                 }
             }
             grid_sum_post(gs, lines2, epoch, acc);
-            if (tid < n_ring) zh = tile_await<float>(&a.zw[ahalo[tid]], epoch, &gs.failed, a.err);
-            if (!grid_sum_wait(gs, lines2, epoch, tot, a.err)) break;
+            if (tid < n_ring) zh = tile_await<float>(&a.zw[ahalo[tid]], epoch, &gs.failed, a.err, a.polls_max);
+            if (!grid_sum_wait(gs, lines2, epoch, tot, a.err, a.polls_max)) break;
             if (tid == 0)
             {
                 converge(tot[0]);

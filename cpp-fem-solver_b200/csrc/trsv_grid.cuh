@@ -64,15 +64,6 @@ constexpr uint32_t kGridHandover = 10;  // steps a tile hand-over adds (the shap
 constexpr uint32_t kGridSmem = 100u << 10;
 constexpr uint32_t kGridMbarPolls = 1u << 27;  // the other warps of a CTA always make progress: a backstop
 
-// polls of one group's hand-over words before a grid schedule's warp gives
-// up (B2S_TIMEOUT): the context's wait bounds (b2s_ctx_set_wait_limits), spin
-// and sleep budgets together, as the grid schedules never sleep
-inline unsigned grid_polls(const b2s_ctx* ctx)
-{
-    const uint64_t p = (uint64_t)ctx->wait_fast_polls + ctx->wait_slow_polls;
-    return (unsigned)std::min<uint64_t>(std::max<uint64_t>(p, 1), 0xffffffffu);
-}
-
 // The tiling of a B x ny x nz grid's lines.
 struct GridTiles
 {

@@ -72,18 +72,20 @@ void* b2s_ctx_stream(b2s_ctx* ctx);
 b2s_status b2s_ctx_synchronize(b2s_ctx* ctx);
 /* Number of this library's kernels launched on ctx since creation. */
 uint64_t b2s_ctx_kernel_launches(const b2s_ctx* ctx);
-/* Bounds of the device-side waits of the chunked triangular solves on ctx
- * (IC(0) / ILU(0) / block ILU(0) with B2S_TRSV_CHUNK, the default): a wait
- * polls spin_polls times without sleeping, then sleeps 1 us per poll, drawing
- * on a budget of sleep_polls per thread for the whole launch.  The 5- and
- * 7-point grid schedules and the level-order traversal (B2S_TRSV_SYNCFREE) of
- * the same solves poll a wait's words up to spin_polls + sleep_polls times (at
- * least once) without sleeping.  A
- * wait that runs out, and every later wait of the same launch, gives up at
- * once and the call reports B2S_TIMEOUT (the synchronous calls at their end, the _device
- * ones at the next b2s_ctx_synchronize or solve).  (0, 0) restores the
- * defaults (2^20 and 2^20, about one second).  No counterpart in the
- * reference (its solves are sequential). */
+/* Bounds of the device-side waits on ctx.  Chunked triangular solves (IC(0) /
+ * ILU(0) / block ILU(0) with B2S_TRSV_CHUNK, the default): a wait polls
+ * spin_polls times without sleeping, then sleeps 1 us per poll, drawing on a
+ * budget of sleep_polls per thread for the whole launch.  The 5- and 7-point
+ * grid schedules and the level-order traversal (B2S_TRSV_SYNCFREE) of the same
+ * solves, and the persistent kernels of PCG and GMRES, whose CTAs wait for one
+ * another's sums (b2s_solve_opts.persistent), poll a wait's words up to
+ * spin_polls + sleep_polls times (at least once) without sleeping.  A wait
+ * that runs out ends the launch early: its later waits give up at once or
+ * within 64 polls (a persistent kernel's CTAs at their next sum), and the call
+ * reports B2S_TIMEOUT (the synchronous calls at their end, the _device ones at
+ * the next b2s_ctx_synchronize or solve).  (0, 0) restores the defaults (2^20
+ * and 2^20, about one second).  No counterpart in the reference (its solves
+ * are sequential). */
 b2s_status b2s_ctx_set_wait_limits(b2s_ctx* ctx, uint32_t spin_polls, uint32_t sleep_polls);
 
 /* ---------------------------------------------------------------- matrices */

@@ -421,3 +421,39 @@ def test_pcg_one_launch_sizes(b2s, ctx, orc, pc, nx, ny, nz):
         # iteration counts by the association of the dots alone; solutions of the same relative residual
         assert abs(st["it"] - io) <= max(2, io // 50)
         assert np.linalg.norm(x - xo) <= 1e-5 * np.linalg.norm(xo)
+
+
+@pytest.mark.parametrize("loop", ["pcg", "pcg_diag", "pcg_tiles", "gmres", "fgmres"])
+def test_persistent_wait_timeout_reported(b2s, ctx, loop):
+    """The persistent kernels' CTAs wait for one another's sums a bounded number
+    of polls.  With the bound cut to one poll the first sums of some 30 and more
+    CTAs, which start microseconds apart, cannot all be there: the solve ends with
+    B2S_TIMEOUT, at once (GMRES's host loop too, which goes on until the device
+    says that a column is done), and with the default bounds the same solve gives
+    the same bits as before."""
+    import time
+    N = 200
+    if loop.startswith("pcg"):
+        n, rp, ci, v = P.poisson2d(N)
+    else:
+        n, rp, ci, v = P.convdiff2d(N)
+    A, b, M = b2s.CSR(ctx, n, n, rp, ci, v), b2s.uniform(5, n), None
+    if loop == "pcg_diag":
+        M = b2s.Precond(ctx, A, b2s.PC_DIAG)
+    if loop == "pcg_tiles":
+        M = b2s.Precond(ctx, A, b2s.PC_IC0, precision=b2s.FP32, trsv=b2s.TRSV_JACOBI, trsv_sweeps=6)
+        assert M.sizes("pcg.tiles")[0] > 1
+    method = {"gmres": b2s.GMRES, "fgmres": b2s.FGMRES}.get(loop, b2s.PCG)
+    x0, _ = b2s.solve(ctx, A, b, method, M, tol=1e-3, maxit=2000)
+    ctx.set_wait_limits(1, 0)
+    try:
+        t0 = time.perf_counter()
+        with pytest.raises(RuntimeError) as e:
+            b2s.solve(ctx, A, b, method, M, tol=1e-3, maxit=2000)
+        dt = time.perf_counter() - t0
+    finally:
+        ctx.set_wait_limits(0, 0)
+    assert e.value.status == b2s.TIMEOUT
+    assert dt < 0.5, dt
+    x, _ = b2s.solve(ctx, A, b, method, M, tol=1e-3, maxit=2000)
+    assert np.array_equal(x, x0)
