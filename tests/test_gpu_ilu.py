@@ -758,3 +758,40 @@ def test_grid7_tile_shapes(b2s, ctx, orc, nx, ny, nz):
         assert np.array_equal(M.apply(r), orc.pc(orc.csr(n, n, rp, ci, v), kind).apply(r)), kind
         M32 = b2s.Precond(ctx, A, b2s.PC_NAMES[kind], precision=b2s.FP32)
         assert np.array_equal(M32.apply(r), _f32_want(M32, kind, r)), kind
+
+
+@pytest.mark.parametrize("what", ["fp64", "fp32", "syncfree", "block"])
+def test_wave_wait_timeout_reported(b2s, ctx, what):
+    """The level-order traversal's waits are bounded.  One row a level and 40
+    entries a row (two passes of a warp): the rows in flight wait for thousands
+    of levels, so with bounds of 200 polls some run out, the others leave on the
+    error word and the call reports B2S_TIMEOUT soon; with the default bounds the
+    same apply gives the same bits as before."""
+    import time
+    n, w = 20000, 40
+    i = np.arange(n)
+    cols = i[:, None] + np.arange(-w, w + 1)
+    keep = (cols >= 0) & (cols < n)
+    rp = np.concatenate([[0], np.cumsum(keep.sum(1))]).astype(np.uint32)
+    v = np.where(cols == i[:, None], 2.0 * w + 1.0, -1.0)[keep]
+    ci = cols[keep].astype(np.uint32)
+    if what == "block":
+        A = b2s.BAIJ(ctx, 2, n, n, rp, ci, (v[:, None, None] * np.eye(2)).ravel())
+        M = b2s.Precond(ctx, A, b2s.PC_BILU0)
+    else:
+        A = b2s.CSR(ctx, n, n, rp, ci, v)
+        M = b2s.Precond(ctx, A, b2s.PC_ILU0, precision=b2s.FP32 if what == "fp32" else b2s.FP64,
+                        trsv=b2s.TRSV_SYNCFREE if what == "syncfree" else b2s.TRSV_AUTO)
+    r = b2s.uniform(3, A.n)
+    z0 = M.apply(r)
+    ctx.set_wait_limits(200, 0)
+    try:
+        t0 = time.perf_counter()
+        with pytest.raises(RuntimeError) as e:
+            M.apply(r)
+        dt = time.perf_counter() - t0
+    finally:
+        ctx.set_wait_limits(0, 0)
+    assert e.value.status == b2s.TIMEOUT
+    assert dt < 0.5, dt
+    assert np.array_equal(M.apply(r), z0)
