@@ -117,7 +117,7 @@ __global__ void __launch_bounds__(wave_threads(GL)) k_trsv_wave(WaveArgs a, cons
     [[maybe_unused]] XT rc = XT(1);
     if constexpr (DIAG == WaveDiag::Divide) rc = (XT)(1.0 / (double)dv[0]);
 
-    bool gave_up = false;  // the same in every lane; the row's later passes read once
+    unsigned limit = a.polls_max;
     for (uint32_t p0 = 0; __any_sync(0xffffffffu, pa + p0 < pe); p0 += GL)
     {
         const uint32_t p = pa + p0 + q;
@@ -149,14 +149,13 @@ __global__ void __launch_bounds__(wave_threads(GL)) k_trsv_wave(WaveArgs a, cons
 #pragma unroll
                 for (int c = 0; c < BS; ++c) fresh &= wave_get(w + c * WPV, epoch, xj[c]);
             }
-            if (gave_up || __all_sync(0xffffffffu, fresh)) break;
-            // by a vote, so that the warp leaves as one: a lane's own load of the error
-            // word may come before or after another's
-            gave_up = polls + 1 >= a.polls_max;
-            if ((polls & 63u) == 63u) gave_up |= __any_sync(0xffffffffu, ld_err(a.err) != 0);
-            if (gave_up)
+            if (__all_sync(0xffffffffu, fresh)) break;
+            // the error word by a vote, so that the warp leaves as one: a lane's own
+            // load may come before or after another's
+            if (polls + 1 >= limit || ((polls & 1023u) == 1023u && __any_sync(0xffffffffu, ld_err(a.err) != 0)))
             {
                 if (lane == 0) atomicCAS(a.err, 0, (int)B2S_TIMEOUT);
+                limit = 1;  // the row's later passes read once
                 break;
             }
             next = __reduce_min_sync(0xffffffffu, fresh ? 0xffffffffu : lev);

@@ -81,7 +81,7 @@ uint64_t b2s_ctx_kernel_launches(const b2s_ctx* ctx);
  * another's sums (b2s_solve_opts.persistent), poll a wait's words up to
  * spin_polls + sleep_polls times (at least once) without sleeping.  A wait
  * that runs out ends the launch early: its later waits give up at once or
- * within 64 polls (a persistent kernel's CTAs at their next sum), and the call
+ * within 1,024 polls (a persistent kernel's CTAs at their next sum), and the call
  * reports B2S_TIMEOUT (the synchronous calls at their end, the _device ones at
  * the next b2s_ctx_synchronize or solve).  (0, 0) restores the defaults (2^20
  * and 2^20, about one second).  No counterpart in the reference (its solves

@@ -764,8 +764,8 @@ def test_grid7_tile_shapes(b2s, ctx, orc, nx, ny, nz):
 def test_wave_wait_timeout_reported(b2s, ctx, what):
     """The level-order traversal's waits are bounded.  One row a level and 40
     entries a row (two passes of a warp): the rows in flight wait for thousands
-    of levels, so with bounds of 200 polls some run out, the others leave on the
-    error word and the call reports B2S_TIMEOUT soon; with the default bounds the
+    of levels, so with bounds of 3,000 polls (1.5 to 2 ms) some run out, the others
+    leave on the error word and the call reports B2S_TIMEOUT soon; with the default bounds the
     same apply gives the same bits as before."""
     import time
     n, w = 20000, 40
@@ -784,7 +784,7 @@ def test_wave_wait_timeout_reported(b2s, ctx, what):
                         trsv=b2s.TRSV_SYNCFREE if what == "syncfree" else b2s.TRSV_AUTO)
     r = b2s.uniform(3, A.n)
     z0 = M.apply(r)
-    ctx.set_wait_limits(200, 0)
+    ctx.set_wait_limits(3000, 0)
     try:
         t0 = time.perf_counter()
         with pytest.raises(RuntimeError) as e:
