@@ -592,6 +592,9 @@ struct Tri
         else
         {
             need(wave.n == n, B2S_UNSUPPORTED, "triangular solve: no schedule was prepared");
+            if constexpr (!UNIT && sizeof(XT) == 4)
+                if (wave.quotient)
+                    return wave.run<1, LOWER, WaveDiag::Quotient>(ctx, m->rp.p, m->ci.p, v, d, rhs, x, out64, done);
             wave.run<1, LOWER, UNIT ? WaveDiag::Unit : WaveDiag::Divide>(ctx, m->rp.p, m->ci.p, v, d, rhs, x, out64,
                                                                          done);
         }
@@ -634,17 +637,20 @@ struct Tri
 
     // The exact solves' schedule: a host chunk plan, the level-by-level one, or
     // the level-order traversal (where it pays, wave_pays, and where no chunk
-    // plan is usable).  rp: the triangle's rows (host); grid: a grid schedule
-    // takes the solves.
-    void load_exact(b2s_ctx* ctx, int mode, const ChunkPlan* plan, uint32_t vs, const uint32_t* rp, bool grid)
+    // plan is usable).  fits: the rows fit chunks (rows_fit_chunks); rp: the
+    // triangle's rows (host); grid: a grid schedule takes the solves.
+    void load_exact(b2s_ctx* ctx, int mode, const ChunkPlan* plan, bool fits, uint32_t vs, const uint32_t* rp, bool grid)
     {
         if (mode == B2S_TRSV_JACOBI || grid || !n) return;
         has_chunks = mode == B2S_TRSV_CHUNK && plan && cs.load(ctx, *plan, vs);
         if (has_chunks) return;
         if (mode == B2S_TRSV_LEVEL)
+        {
             ensure_sched(ctx);
-        else
-            wave.build(ctx, h_level, rp, 1);
+            return;
+        }
+        wave.build(ctx, h_level, rp, 1);
+        wave.quotient = !fits;
     }
 
     // lay the final factor values out for the chunk schedule (no-op otherwise)
@@ -675,6 +681,7 @@ struct HostAnalysis
     bool tiles_grid5 = false;        // a 5-point grid: the index blobs are built on the device
     std::vector<TileGeom> tile_geom;
     bool chunked = false;
+    bool lo_fits = true, up_fits = true;  // asked of chunked triangles only
     std::exception_ptr error;
     std::thread th;
     ~HostAnalysis()
@@ -1336,12 +1343,14 @@ std::unique_ptr<PcImpl> make_pc_ic0_ex(b2s_ctx* ctx, const CsrDev& A, const b2s_
             plan_parallel(2, 2, [&](uint32_t side, unsigned) {
                 if (side == 0)
                 {
+                    if (ha.chunked) ha.lo_fits = rows_fit_chunks(n, hrp.data(), hci.data(), true, 1, vs, vs, 8);
                     if (ha.chunked && !wave_pays(pc->fwd.h_level, hrp.data(), hci.data(), true))
                         ha.lo_plan = plan_chunks(n, hrp.data(), hci.data(), true, 1, vs, vs, 8, kChunkSmemBudget, 1,
                                                  &pc->fwd.h_level);
                     return;
                 }
                 compute_levels(n, ha.up_rp.data(), ha.up_ci.data(), false, ha.up_level);
+                if (ha.chunked) ha.up_fits = rows_fit_chunks(n, ha.up_rp.data(), ha.up_ci.data(), false, 1, vs, vs, 8);
                 if (ha.chunked && !wave_pays(ha.up_level, ha.up_rp.data(), ha.up_ci.data(), false))
                     ha.up_plan = plan_chunks(n, ha.up_rp.data(), ha.up_ci.data(), false, 1, vs, vs, 8,
                                              kChunkSmemBudget, 1, &ha.up_level);
@@ -1381,8 +1390,8 @@ std::unique_ptr<PcImpl> make_pc_ic0_ex(b2s_ctx* ctx, const CsrDev& A, const b2s_
     ha.wait();
     pc->bwd.init(pc->LT, false, false);
     pc->bwd.h_level = std::move(ha.up_level);
-    pc->fwd.load_exact(ctx, pc->mode, ha.chunked ? &ha.lo_plan : nullptr, vs, hrp.data(), gs.any());
-    pc->bwd.load_exact(ctx, pc->mode, ha.chunked ? &ha.up_plan : nullptr, vs, ha.up_rp.data(), gs.any());
+    pc->fwd.load_exact(ctx, pc->mode, ha.chunked ? &ha.lo_plan : nullptr, ha.lo_fits, vs, hrp.data(), gs.any());
+    pc->bwd.load_exact(ctx, pc->mode, ha.chunked ? &ha.up_plan : nullptr, ha.up_fits, vs, ha.up_rp.data(), gs.any());
     enable_grid(ctx, pc->fwd, pc->bwd, gs, n);
     if (sweeps)
     {
@@ -1504,6 +1513,7 @@ std::unique_ptr<PcImpl> make_pc_ilu0(b2s_ctx* ctx, const CsrDev& A, const b2s_pc
                     return;
                 }
                 compute_levels(n, urp.data(), uci.data(), false, ha.up_level);
+                if (ha.chunked) ha.up_fits = rows_fit_chunks(n, urp.data(), uci.data(), false, 1, vs, vs, 8);
                 if (ha.chunked && !wave_pays(ha.up_level, urp.data(), uci.data(), false))
                     ha.up_plan = plan_chunks(n, urp.data(), uci.data(), false, 1, vs, vs, 8, kChunkSmemBudget, 1,
                                              &ha.up_level);
@@ -1536,8 +1546,8 @@ std::unique_ptr<PcImpl> make_pc_ilu0(b2s_ctx* ctx, const CsrDev& A, const b2s_pc
     ha.wait();
     pc->bwd.init(pc->U, false, false);
     pc->bwd.h_level = std::move(ha.up_level);
-    pc->fwd.load_exact(ctx, pc->mode, ha.chunked ? &ha.lo_plan : nullptr, vs, lrp.data(), gs.any());
-    pc->bwd.load_exact(ctx, pc->mode, ha.chunked ? &ha.up_plan : nullptr, vs, urp.data(), gs.any());
+    pc->fwd.load_exact(ctx, pc->mode, ha.chunked ? &ha.lo_plan : nullptr, ha.lo_fits, vs, lrp.data(), gs.any());
+    pc->bwd.load_exact(ctx, pc->mode, ha.chunked ? &ha.up_plan : nullptr, ha.up_fits, vs, urp.data(), gs.any());
     enable_grid(ctx, pc->fwd, pc->bwd, gs, n);
     if (pc->mode == B2S_TRSV_JACOBI)
     {

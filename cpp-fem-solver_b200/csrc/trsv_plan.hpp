@@ -304,6 +304,24 @@ inline bool plan_grow(uint32_t n, const uint32_t* rp, const uint32_t* ci, uint32
     return true;
 }
 
+// Whether each row fits a chunk by itself; a triangle with one that does not has
+// no chunk plan (plan_grow's test for the first row of a chunk, all of whose
+// dependencies lie outside it).  Scalar rows; arguments as plan_chunks'.
+inline bool rows_fit_chunks(uint32_t n, const uint32_t* rp, const uint32_t* ci, bool lower, uint32_t dv, uint32_t vs,
+                            uint32_t xs, uint32_t rs, uint32_t budget = kChunkSmemBudget)
+{
+    const uint64_t fixed = 16 * 10 + (uint64_t)vs * dv + 10 + xs + rs, per = (uint64_t)vs + 2 + xs + 4;
+    const uint64_t most = std::min<uint64_t>({budget > fixed ? (budget - fixed) / per : 0, kChunkMaxDeps, kChunkMaxSlots});
+    for (uint32_t i = 0; i < n; ++i)
+    {
+        if (rp[i + 1] - rp[i] <= most) continue;
+        uint64_t deps = 0;
+        for (uint32_t p = rp[i]; p < rp[i + 1]; ++p) deps += lower ? ci[p] < i : ci[p] > i;
+        if (deps > most) return false;
+    }
+    return true;
+}
+
 // Plan the chunks of a triangle with (block) CSR pattern rp/ci (dependency
 // entries are j < i for lower, j > i for upper; other entries are ignored).
 // vs, xs, rs: element sizes of values, solution and right-hand side the chunks

@@ -34,13 +34,16 @@ namespace b2s {
 constexpr int wave_threads(int gl) { return gl <= 8 ? 512 : 256; }
 constexpr uint32_t kWaveNone = 0xffffffffu;
 
-// What a row does with its sum: nothing (unit diagonal), divide by d[row], or
-// multiply by the inverse diagonal block d[row].  BLOCK: the block kernels'
-// products (each block component summed from zero, then subtracted).
+// What a row does with its sum: nothing (unit diagonal), divide by d[row] (FP32
+// Divide multiplies by the reciprocal, Quotient divides, with one rounding less:
+// the triangles no chunk plan could take), or multiply by the inverse diagonal
+// block d[row].  BLOCK: the block kernels' products (each block component summed
+// from zero, then subtracted).
 enum class WaveDiag
 {
     Unit,
     Divide,
+    Quotient,
     BlockUnit,
     BlockInverse
 };
@@ -105,15 +108,16 @@ __global__ void __launch_bounds__(wave_threads(GL)) k_trsv_wave(WaveArgs a, cons
     if (on && q < BS)
     {
         sum = (XT)rhs[(size_t)row * BS + q];
-        if constexpr (DIAG == WaveDiag::Divide) dv[0] = (XT)__ldg(&d[row]);
+        if constexpr (DIAG == WaveDiag::Divide || DIAG == WaveDiag::Quotient) dv[0] = (XT)__ldg(&d[row]);
         if constexpr (DIAG == WaveDiag::BlockInverse)
 #pragma unroll
             for (int c = 0; c < BS; ++c) dv[c] = (XT)__ldg(&d[((size_t)row * BS + q) * BS + c]);
     }
     else
         for (XT& e : dv) e = XT(1);
-    // FP32 multiplies by the reciprocal rounded once from FP64, FP64 forms the
-    // quotient from the reciprocal (grid_quotient): both before the wait
+    // FP32 multiplies by the reciprocal rounded once from FP64, as the chunks do,
+    // FP64 forms the quotient from the reciprocal (grid_quotient): both before the
+    // wait
     [[maybe_unused]] XT rc = XT(1);
     if constexpr (DIAG == WaveDiag::Divide) rc = (XT)(1.0 / (double)dv[0]);
 
@@ -188,6 +192,7 @@ __global__ void __launch_bounds__(wave_threads(GL)) k_trsv_wave(WaveArgs a, cons
     }
 
     XT r = sum;
+    if constexpr (DIAG == WaveDiag::Quotient) r = sum / dv[0];
     if constexpr (DIAG == WaveDiag::Divide)
     {
         if constexpr (sizeof(XT) == 4)
@@ -263,6 +268,7 @@ inline bool wave_pays(const std::vector<uint32_t>& level, const uint32_t* rp, co
 struct WaveSchedule
 {
     uint32_t n = 0, bs = 1, gl = 32, npos = 0;
+    bool quotient = false;  // FP32 divisors: Quotient, not Divide
     DBuf<uint32_t> order, lev, ctl;
     DBuf<unsigned long long> xch;
 

@@ -211,7 +211,10 @@ typedef enum b2s_trsv
 {
     B2S_TRSV_AUTO = 0,
     B2S_TRSV_LEVEL = 1,    /* one launch per level of the dependency DAG */
-    B2S_TRSV_SYNCFREE = 2, /* one launch; rows in level order, each waiting (bounded) for its operands */
+    B2S_TRSV_SYNCFREE = 2, /* one launch; rows in level order, each waiting (bounded) for its operands.
+                              FP32 pivots: LEVEL divides by them, the one-launch schedules multiply by the
+                              reciprocal, rounded once from FP64 (and AUTO divides in a triangle with a row
+                              too long for a chunk, 15,000 entries and more); FP64 is the same in all */
     B2S_TRSV_CHUNK = 3,    /* one launch (the AUTO choice): row chunks staged in shared memory, local
                               levels split by barriers, bounded flags between chunks; triangles with
                               wide rows or many rows a level take SYNCFREE's traversal instead, and

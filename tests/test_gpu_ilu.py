@@ -795,3 +795,49 @@ def test_wave_wait_timeout_reported(b2s, ctx, what):
     assert e.value.status == b2s.TIMEOUT
     assert dt < 0.5, dt
     assert np.array_equal(M.apply(r), z0)
+
+
+@pytest.mark.parametrize("chain", [True, False])
+@pytest.mark.parametrize("kind", ["ic0", "ilu0"])
+def test_fp32_long_row_divides(b2s, ctx, chain, kind):
+    """FP32 factors with a row too long for a chunk (more than 15,782 entries of
+    14 bytes in 216 KB), the last of L or the first of U, in a chain of n levels
+    and in an arrow of two: its triangle has no chunk plan and divides by the
+    pivots, one rounding each, as the level-by-level solve does; the other's
+    rows are short and multiply by the rounded reciprocal (a unit triangle does
+    neither)."""
+    n, f32 = 16500, np.float32
+    hub = n - 1 if kind == "ic0" else 0
+    i = np.delete(np.arange(n), hub)
+    R = [np.arange(n), np.full(n - 1, hub), i]
+    C_ = [np.arange(n), i, np.full(n - 1, hub)]
+    V = [3.0 + b2s.uniform(1, n)] + [np.full(n - 1, -1e-4)] * 2
+    if chain:
+        R, C_, V = R + [i[1:], i[:-1]], C_ + [i[:-1], i[1:]], V + [np.full(n - 2, -1.0)] * 2
+    n, rp, ci, v = (n,) + P.coo_to_csr(n, n, np.concatenate(R), np.concatenate(C_), np.concatenate(V))
+    A = b2s.CSR(ctx, n, n, rp, ci, v)
+    r = b2s.uniform(27, n)
+    M = b2s.Precond(ctx, A, b2s.PC_NAMES[kind], precision=b2s.FP32)
+
+    def solve(T, rhs, lower, pivot):
+        x = np.zeros(n, f32)
+        for k in range(n) if lower else range(n - 1, -1, -1):
+            c, w = T[1][T[0][k]:T[0][k + 1]], T[2][T[0][k]:T[0][k + 1]].astype(f32)
+            dep = c < k if lower else c > k
+            s = f32(rhs[k])
+            for p in w[dep] * x[c[dep]]:
+                s = f32(s - p)
+            x[k] = pivot(s, k)
+        return x
+
+    if kind == "ic0":
+        L, U = M.export("ic0.L"), M.export("ic0.LT")
+        d = L[2][L[0][1:].astype(np.int64) - 1].astype(f32)
+    else:
+        L, U = M.export("ilu0.L"), M.export("ilu0.U")
+        d = U[2][U[0][:-1].astype(np.int64)].astype(f32)
+    divide = lambda s, k: f32(s / d[k])
+    times = lambda s, k: f32(s * f32(1.0 / np.float64(d[k])))
+    y = solve(L, r, True, divide if kind == "ic0" else lambda s, k: s)
+    z = solve(U, y, False, times if kind == "ic0" else divide)
+    assert np.array_equal(M.apply(r), z.astype(np.float64))
