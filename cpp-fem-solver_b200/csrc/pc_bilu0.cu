@@ -304,6 +304,13 @@ struct PcBILU0 final : PcImpl
     void export_data(b2s_ctx* ctx, const std::string& what, uint64_t* sizes, uint32_t* rp, uint32_t* ci,
                      double* v) override
     {
+        if (what == "trsv.route")  // as for the scalar factors: 1, 2 or 3
+        {
+            sizes[0] = mode == B2S_TRSV_CHUNK && !chunk_l ? B2S_TRSV_SYNCFREE : mode;
+            sizes[1] = mode == B2S_TRSV_CHUNK && !chunk_u ? B2S_TRSV_SYNCFREE : mode;
+            sizes[2] = 0;
+            return;
+        }
         const size_t bv = (size_t)bs * bs;
         const BCsr* m = what == "bilu0.L" ? &L : what == "bilu0.U" ? &U : nullptr;
         if (m)
@@ -400,13 +407,13 @@ std::unique_ptr<PcImpl> make_pc_bilu0(b2s_ctx* ctx, const BaijDev& A, const b2s_
             plan_parallel(2, 2, [&](uint32_t side, unsigned) {
                 if (side == 0)
                 {
-                    if (chunked && !wave_pays(llev, lrp.data(), lci.data(), true))
+                    if (chunked && !wave_pays(llev, lrp.data(), lci.data(), true, (uint32_t)bs))
                         lplan = plan_chunks(nb, lrp.data(), lci.data(), true, 0, vs, vs, 8, kChunkSmemBudget,
                                             (uint32_t)bs, &llev);
                     return;
                 }
                 compute_levels(nb, urp.data(), uci.data(), false, ulev);
-                if (chunked && !wave_pays(ulev, urp.data(), uci.data(), false))
+                if (chunked && !wave_pays(ulev, urp.data(), uci.data(), false, (uint32_t)bs))
                     uplan = plan_chunks(nb, urp.data(), uci.data(), false, (uint32_t)bv, vs, vs, 8, kChunkSmemBudget,
                                         (uint32_t)bs, &ulev);
             });

@@ -600,6 +600,13 @@ struct Tri
         }
     }
 
+    // what run_t takes: 1 level by level, 2 the level-order traversal, 3 chunks, 4 sweeps, 5 a grid schedule
+    uint64_t route(int mode) const
+    {
+        if (mode != B2S_TRSV_CHUNK) return (uint64_t)mode;
+        return grid.on && grid.packed_v ? 5u : has_chunks ? 3u : 2u;
+    }
+
     // x = T^-1 rhs; precision per the type parameters.  With out64 the results
     // also go there in FP64, and the grid schedules then leave x unwritten
     // (an FP32 x is scratch for every caller that passes out64)
@@ -1156,6 +1163,13 @@ struct PcIC0 final : PcImpl
         }
         if (what == "levels.L") return export_levels(ctx, fwd, sizes, ci);
         if (what == "levels.U") return export_levels(ctx, bwd, sizes, ci);
+        if (what == "trsv.route")
+        {
+            sizes[0] = fwd.route(mode);
+            sizes[1] = bwd.route(mode);
+            sizes[2] = 0;
+            return;
+        }
         if (what == "trsv.grid5") return export_grid5(fwd, bwd, sizes);
         if (what == "trsv.grid7") return export_grid7(fwd, bwd, sizes);
         if (what == "pcg.tiles")  // the tiled persistent PCG kernel: tiles (0: not planned), rows per thread, smem
@@ -1453,6 +1467,13 @@ struct PcILU0 final : PcImpl
     {
         if (what == "ilu0.L") return export_csr(ctx, L, sizes, rp, ci, v);
         if (what == "ilu0.U") return export_csr(ctx, U, sizes, rp, ci, v);
+        if (what == "trsv.route")
+        {
+            sizes[0] = fwd.route(mode);
+            sizes[1] = bwd.route(mode);
+            sizes[2] = 0;
+            return;
+        }
         if (what == "trsv.grid5") return export_grid5(fwd, bwd, sizes);
         if (what == "trsv.grid7") return export_grid7(fwd, bwd, sizes);
         if (what == "levels.L") return export_levels(ctx, fwd, sizes, ci);

@@ -304,6 +304,51 @@ inline bool plan_grow(uint32_t n, const uint32_t* rp, const uint32_t* ci, uint32
     return true;
 }
 
+// Whether a triangle's exact solves take the level-order traversal
+// (trsv_wave.cuh) rather than the chunked schedule (trsv_chunk.cuh).  A level
+// costs 0.6-0.85 us in the traversal, one trip through L2 whatever its rows, and
+// another for every 32 entries of a row.  In a chunk it costs what its widest row
+// does: scalar rows of up to 4 entries are straight-line code, 0.25 us FP64 and
+// 0.2 FP32, wider ones 0.25 + 0.126 w (0.2 + 0.085 w); blocks 0.3 + 0.093 w (2x2)
+// and 0.34 + 0.1 w (3x3); and it grows with the rows of a level.  So the widths of
+// all levels are weighed, in 48ths of a traversal's level; wide levels always pay,
+// and a triangle of short rows alone keeps the chunks.
+//
+// Measured, an apply in FP64, traversal / chunked: bands of half-width w, one row
+// a level, 20,000 rows, ms: w 1-4 27 / 10, 5 26 / 35, 8 27 / 50, 16 29 / 91; w 3
+// with n/40, n/4, n and 2 n random links 29 / 11, 29 / 13, 30 / 21, 30 / 31 (here
+// the weights say chunked and, at 2 n, near even); tridiagonal with one row of
+// 500 entries 18 / 10.  13-point 2-D grid 256^2 (6 entries a row) 1.3 / 1.9, 25-point
+// 1.7 / 4.7; Q1 scalar rows of 13 entries 12^3 .. 64^3 elements 0.14 / 0.46 ..
+// 0.85 / 2.23, 3x3 blocks 0.14 / 0.54 .. 0.91 / 5.62.  Short rows: 7-point 64^3 in
+// level-order numbering (1,380 rows a level) 0.28 / 2.09; 5-point in level-order
+// numbering 512^2 (256 rows a level) 1.35 / 1.49 and numbered in 8x8 tiles 1.71 /
+// 0.90; 128^2 (64 a level) 0.36 / 0.20; 3 x 5000 (3 a level) 5.7 / 2.5.
+inline bool wave_pays(const std::vector<uint32_t>& level, const uint32_t* rp, const uint32_t* ci, bool lower,
+                      uint32_t bs = 1)
+{
+    const uint32_t n = (uint32_t)level.size();
+    std::vector<uint32_t> width;  // strict entries of each level's widest row
+    uint32_t widest = 0;
+    for (uint32_t i = 0; i < n; ++i)
+    {
+        uint32_t m = 0;
+        for (uint32_t p = rp[i]; p < rp[i + 1]; ++p) m += lower ? ci[p] < i : ci[p] > i;
+        if (level[i] >= width.size()) width.resize((size_t)level[i] + 1, 0);
+        width[level[i]] = std::max(width[level[i]], m);
+        widest = std::max(widest, m);
+    }
+    if ((uint64_t)n >= 512ull * width.size()) return true;
+    if (widest <= 4) return false;
+    uint64_t chunked = 0, wave = 0;
+    for (uint64_t w : width)
+    {
+        chunked += bs > 1 ? 23 + 7 * w : w <= 4 ? 18 : 16 + 8 * w;
+        wave += 48 * std::max<uint64_t>((w + 31) / 32, 1);
+    }
+    return chunked > wave;
+}
+
 // Whether each row fits a chunk by itself; a triangle with one that does not has
 // no chunk plan (plan_grow's test for the first row of a chunk, all of whose
 // dependencies lie outside it).  Scalar rows; arguments as plan_chunks'.

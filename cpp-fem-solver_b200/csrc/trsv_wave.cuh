@@ -234,36 +234,6 @@ __global__ void __launch_bounds__(wave_threads(GL)) k_trsv_wave(WaveArgs a, cons
     }
 }
 
-// Whether a triangle's solves take the level-order traversal rather than the
-// chunked schedule (trsv_chunk.cuh).  A level costs about 0.6-0.9 us here
-// whatever its width, one trip through L2; in a chunk it costs 0.25-0.45 us
-// when its rows are short (up to 4 entries are straight-line code) and few, and
-// grows with both.  Measured (apply, FP64, this / chunked): Q1 scalar rows of
-// 13 entries 12^3 .. 64^3 elements 0.14 / 0.46 .. 0.85 / 2.23 ms, 3x3 blocks
-// 0.14 / 0.54 .. 0.91 / 5.62; 7-point 64^3 in level-order numbering (1,380 rows
-// a level) 0.28 / 2.09; 5-point in level-order numbering 512^2 (256 rows a
-// level) 1.35 / 1.49 and numbered in 8x8 tiles 1.71 / 0.90; 128^2 (64 a level)
-// 0.36 / 0.20; 3 x 5000 (3 a level) 5.7 / 2.5.
-inline bool wave_pays(uint32_t n, uint32_t levels, uint32_t widest)
-{
-    return widest > 4 || (uint64_t)n >= 512ull * levels;
-}
-
-// the same from a triangle's pattern and levels (host); strict entries only
-inline bool wave_pays(const std::vector<uint32_t>& level, const uint32_t* rp, const uint32_t* ci, bool lower)
-{
-    const uint32_t n = (uint32_t)level.size();
-    uint32_t widest = 0, top = 0;
-    for (uint32_t i = 0; i < n; ++i)
-    {
-        uint32_t m = 0;
-        for (uint32_t p = rp[i]; p < rp[i + 1]; ++p) m += lower ? ci[p] < i : ci[p] > i;
-        widest = std::max(widest, m);
-        top = std::max(top, level[i]);
-    }
-    return wave_pays(n, top + 1, widest);
-}
-
 // One triangle's level-order schedule.
 struct WaveSchedule
 {

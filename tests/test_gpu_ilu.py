@@ -841,3 +841,44 @@ def test_fp32_long_row_divides(b2s, ctx, chain, kind):
     y = solve(L, r, True, divide if kind == "ic0" else lambda s, k: s)
     z = solve(U, y, False, times if kind == "ic0" else divide)
     assert np.array_equal(M.apply(r), z.astype(np.float64))
+
+
+@pytest.mark.parametrize("pattern,route,block_route", [("band4", 3, 3), ("band5", 2, 2), ("band3+long", 3, 3),
+                                                       ("band3+few", 3, 3), ("5pt+long", 3, 2)])
+def test_schedule_of_mixed_rows(b2s, ctx, orc, pattern, route, block_route):
+    """Triangles of short rows with few wide ones keep the chunked schedule, wide
+    ones take the level-order traversal (a long row of blocks weighs more against
+    few levels); either way the FP64 applies equal the
+    restatement bit for bit, block ones (2x2) those solved level by level, and the
+    FP32 ones their emulation."""
+    rng = np.random.default_rng(len(pattern))
+    n = 48 * 45 if pattern == "5pt+long" else 2000
+    i = np.arange(n)
+    pairs = set()
+    if pattern == "5pt+long":
+        pairs |= {(int(k), int(k) - 1) for k in i if k % 48} | {(int(k), int(k) - 48) for k in i if k >= 48}
+    else:
+        pairs |= {(int(k), int(k) - d) for d in range(1, int(pattern[4]) + 1) for k in i if k >= d}
+    if pattern.endswith("long"):
+        pairs |= {(n - 1, int(j)) for j in range(0, n - 60, 7)}
+    if pattern.endswith("few"):
+        pairs |= {(int(k), int(j)) for k in range(100, n, 25) for j in rng.integers(0, k - 5, 4)}
+    lo = np.array(sorted(pairs))
+    a = -rng.uniform(0.1, 1.0, len(lo))
+    deg = np.bincount(lo.ravel(), minlength=n)
+    rp, ci, v = P.coo_to_csr(n, n, np.concatenate([lo[:, 0], lo[:, 1], i]), np.concatenate([lo[:, 1], lo[:, 0], i]),
+                             np.concatenate([a, a, deg + 1.0]))
+    A = b2s.CSR(ctx, n, n, rp, ci, v)
+    r = b2s.uniform(n, n)
+    for kind in ("ic0", "ilu0"):
+        M = b2s.Precond(ctx, A, b2s.PC_NAMES[kind])
+        assert M.sizes("trsv.route")[0] == route, kind
+        assert np.array_equal(M.apply(r), orc.pc(orc.csr(n, n, rp, ci, v), kind).apply(r)), kind
+        M32 = b2s.Precond(ctx, A, b2s.PC_NAMES[kind], precision=b2s.FP32)
+        assert M32.sizes("trsv.route")[0] == route
+        assert np.array_equal(M32.apply(r), _f32_want(M32, kind, r)), kind
+    B = b2s.BAIJ(ctx, 2, n, n, rp, ci, (v[:, None, None] * np.array([[1.0, 0.1], [-0.2, 1.1]])).ravel())
+    M = b2s.Precond(ctx, B, b2s.PC_BILU0)
+    assert M.sizes("trsv.route")[0] == block_route
+    r = b2s.uniform(n, B.n)
+    assert np.array_equal(M.apply(r), b2s.Precond(ctx, B, b2s.PC_BILU0, trsv=b2s.TRSV_LEVEL).apply(r))
