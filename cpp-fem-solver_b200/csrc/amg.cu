@@ -41,13 +41,21 @@ constexpr double kTheta = 0.25, kOmega = 2.0 / 3.0;
 
 // ------------------------------------------------------------ BAIJ helpers
 
-__global__ void k_find_diag(uint32_t nb, const uint32_t* __restrict__ rp, const uint32_t* __restrict__ ci,
-                            uint32_t* __restrict__ dptr)
+// dptr: each row's diagonal block; after them the most blocks in a range of
+// `per` rows (zero before; per 0: left) and the number of blocks
+__global__ void k_find_diag(uint32_t nb, uint32_t per, const uint32_t* __restrict__ rp,
+                            const uint32_t* __restrict__ ci, uint32_t* dptr)
 {
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < nb; i += gridDim.x * blockDim.x)
     {
         uint32_t lo = rp[i];
         const uint32_t end = rp[i + 1];
+        if (per && i % per == 0)
+        {
+            const uint32_t blocks = rp[nb - i < per ? nb : i + per] - lo;
+            if (blocks > *(volatile uint32_t*)&dptr[nb]) atomicMax(&dptr[nb], blocks);
+        }
+        if (i + 1 == nb) dptr[nb + 1] = end;
         for (uint32_t hi = end; lo < hi;)  // columns ascend
         {
             const uint32_t mid = lo + (hi - lo) / 2;
@@ -60,15 +68,20 @@ __global__ void k_find_diag(uint32_t nb, const uint32_t* __restrict__ rp, const 
     }
 }
 
-// finalise a device-built BAIJ: diagonal pointers and the block count
+// finalise a device-built BAIJ: diagonal pointers, the block count, the
+// matvec's row partition
 void finish_baij(b2s_ctx* ctx, BaijDev& M)
 {
-    M.diag_ptr.alloc(M.nbr ? M.nbr : 1);
+    M.diag_ptr.alloc((size_t)M.nbr + 2);
+    B2S_CUDA(cudaMemsetAsync(M.diag_ptr.p + M.nbr, 0, 2 * sizeof(uint32_t), ctx->stream));
     if (M.nbr)
-        B2S_LAUNCH(ctx, k_find_diag, stream_grid(ctx, M.nbr), kThreads, 0, M.nbr, M.rp.p, M.ci.p, M.diag_ptr.p);
-    d2h(ctx, &M.nnzb, M.rp.p + M.nbr, sizeof(uint32_t));
+        B2S_LAUNCH(ctx, k_find_diag, stream_grid(ctx, M.nbr), kThreads, 0, M.nbr,
+                   M.bs > 1 ? baij_even_rows(ctx, M.nbr) : 0u, M.rp.p, M.ci.p, M.diag_ptr.p);
+    uint32_t h[2];
+    d2h(ctx, h, M.diag_ptr.p + M.nbr, sizeof(h));
     sync(ctx);
-    baij_partition(ctx, M);
+    M.nnzb = h[1];
+    baij_partition(ctx, M, h[0]);
 }
 
 template <int BS>

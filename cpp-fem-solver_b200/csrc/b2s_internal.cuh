@@ -225,13 +225,15 @@ struct BaijDev
     DBuf<uint32_t> rp, ci;
     DBuf<double> v;
     DBuf<uint32_t> diag_ptr;    // UINT32_MAX when missing
-    DBuf<uint32_t> blk_row;     // bs = 1 with long rows: staged-matvec row partition (nblk + 1)
+    DBuf<uint32_t> blk_row;     // row partition of the matvec (nblk + 1): its CTAs' (bs = 1) or its warps'
     uint32_t nblk = 0;          // 0: the matvec needs no partition
 };
 
-// Row partition of a bs = 1 BAIJ with long rows for its staged matvec
-// (nothing for other operators), from its device arrays.
-void baij_partition(b2s_ctx* ctx, BaijDev& M);
+// Row partition of a BAIJ for its matvec, from its device arrays: bs = 1 with
+// long rows, and bs > 1 where rows dealt evenly to the warps would not share the
+// blocks.  most: blocks of the fullest of the ranges of baij_even_rows rows.
+void baij_partition(b2s_ctx* ctx, BaijDev& M, uint32_t most);
+uint32_t baij_even_rows(const b2s_ctx* ctx, uint32_t nbr);
 
 // Preconditioner implementation.  apply() enqueues z = M^-1 r on ctx->stream
 // (device pointers).  `done` (device, may be null) lets the Krylov drivers

@@ -30,10 +30,10 @@ void baij_matvec_f32(b2s_ctx* ctx, const BaijDev& A, const float* v32, const dou
     baij_matvec_t<float>(ctx, A, v32, x, y, done);
 }
 
-// Rows of CTA c: those whose weight -- entries before them, and kBaijStagedRow
+// Rows of share c: those whose weight -- entries before them, and row_weight
 // for each row before them -- lies in [c, c + 1) times share.
-static __global__ void k_baij_split(uint32_t nbr, const uint32_t* __restrict__ rp, uint32_t share, uint32_t nblk,
-                                    uint32_t* __restrict__ blk_row)
+static __global__ void k_baij_split(uint32_t nbr, const uint32_t* __restrict__ rp, uint32_t row_weight, uint32_t share,
+                                    uint32_t nblk, uint32_t* __restrict__ blk_row)
 {
     for (uint32_t c = blockIdx.x * blockDim.x + threadIdx.x; c <= nblk; c += gridDim.x * blockDim.x)
     {
@@ -42,7 +42,7 @@ static __global__ void k_baij_split(uint32_t nbr, const uint32_t* __restrict__ r
         while (lo < hi)
         {
             const uint32_t mid = lo + (hi - lo) / 2;
-            if (rp[mid] + (uint64_t)kBaijStagedRow * mid < target)
+            if (rp[mid] + (uint64_t)row_weight * mid < target)
                 lo = mid + 1;
             else
                 hi = mid;
@@ -51,15 +51,35 @@ static __global__ void k_baij_split(uint32_t nbr, const uint32_t* __restrict__ r
     }
 }
 
-void baij_partition(b2s_ctx* ctx, BaijDev& M)
+uint32_t baij_even_rows(const b2s_ctx* ctx, uint32_t nbr)
+{
+    const uint32_t warps = baij_warps(ctx);
+    return std::max((nbr + warps - 1) / warps, 1u);
+}
+
+void baij_partition(b2s_ctx* ctx, BaijDev& M, uint32_t most)
 {
     M.nblk = 0;
-    if (M.bs != 1 || M.nbr == 0 || M.nnzb < (uint64_t)kBaijStagedMinRow * M.nbr) return;
-    const uint64_t weight = M.nnzb + (uint64_t)kBaijStagedRow * M.nbr;
-    const uint32_t share = baij_staged_share(ctx, M.nbr, M.nnzb);
-    M.nblk = (uint32_t)((weight + share - 1) / share);
-    M.blk_row.alloc(M.nblk + 1);
-    B2S_LAUNCH(ctx, k_baij_split, stream_grid(ctx, M.nblk + 1), kThreads, 0, M.nbr, M.rp.p, share, M.nblk, M.blk_row.p);
+    if (!M.nbr) return;
+    uint32_t row_weight, share;
+    if (M.bs == 1)
+    {
+        if (M.nnzb < (uint64_t)kBaijStagedMinRow * M.nbr) return;
+        row_weight = kBaijStagedRow;
+        share = baij_staged_share(ctx, M.nbr, M.nnzb);
+    }
+    else
+    {
+        const uint32_t per = baij_even_rows(ctx, M.nbr);
+        if (per == 1 || (uint64_t)most * M.nbr <= kBaijUneven * (uint64_t)per * M.nnzb) return;
+        row_weight = kBaijWarpRow;
+        const uint32_t shares = std::min(baij_warps(ctx), M.nbr);
+        share = (uint32_t)((M.nnzb + (uint64_t)row_weight * M.nbr + shares - 1) / shares);
+    }
+    M.nblk = (uint32_t)((M.nnzb + (uint64_t)row_weight * M.nbr + share - 1) / share);
+    M.blk_row.alloc((size_t)M.nblk + 1);
+    B2S_LAUNCH(ctx, k_baij_split, stream_grid(ctx, M.nblk + 1ull), kThreads, 0, M.nbr, M.rp.p, row_weight, share, M.nblk,
+               M.blk_row.p);
 }
 
 // ------------------------------------------------------------ block Jacobi
@@ -172,6 +192,10 @@ b2s_status b2s_baij_create(b2s_ctx* ctx, int bs, uint32_t nbr, uint32_t nbc, con
         d.nbr = nbr;
         d.nbc = nbc;
         d.nnzb = nnzb;
+        const uint32_t per = baij_even_rows(ctx, nbr);
+        uint32_t most = 0;
+        for (uint64_t i = 0; i < nbr; i += per)
+            most = std::max(most, row_ptr[std::min<uint64_t>(i + per, nbr)] - row_ptr[i]);
         std::vector<uint32_t> diag(nbr, 0xFFFFFFFFu);
         for (uint32_t i = 0; i < nbr; ++i)
             for (uint32_t k = row_ptr[i]; k < row_ptr[i + 1]; ++k)
@@ -185,7 +209,7 @@ b2s_status b2s_baij_create(b2s_ctx* ctx, int bs, uint32_t nbr, uint32_t nbc, con
         d.ci = upload(ctx, col_idx, nnzb);
         d.v = upload(ctx, values, (size_t)nnzb * bs * bs);
         d.diag_ptr = upload(ctx, diag.data(), nbr);
-        baij_partition(ctx, d);
+        baij_partition(ctx, d, most);
         sync(ctx);
     });
     if (st != B2S_OK)

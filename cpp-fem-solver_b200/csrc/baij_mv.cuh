@@ -28,6 +28,15 @@ namespace b2s {
 
 constexpr int kBaijThreads = 192;
 constexpr int kBaijCtasPerSm = 4;
+inline uint32_t baij_warps(const b2s_ctx* ctx) { return (uint32_t)ctx->sm_count * kBaijCtasPerSm * (kBaijThreads / 32); }
+
+// Rows are dealt evenly, or, where that gives a warp more than kBaijUneven times
+// the mean blocks, by weight, a row kBaijWarpRow besides its blocks (k_baij_split).
+// 3x3, 120,000 rows of 9 blocks with 200 adjacent rows of 2,500: 97 us by weight,
+// 2,700 evenly.  Up to twice the mean an even deal, which reads no partition, is as
+// good: half the rows of 27 blocks, half of 3 (1.8 times): 39 us.
+constexpr uint32_t kBaijUneven = 2;
+constexpr uint32_t kBaijWarpRow = 2;
 
 template <int BS, typename VT>
 struct alignas(16) BaijWarpSmem
@@ -41,11 +50,12 @@ struct alignas(16) BaijWarpSmem
 
 // VT: stored value type (double, or float for the FP32 copies of the AMG
 // hierarchy); products and sums are FP64 either way.  v is 16-byte aligned.
-// per: block rows a warp.
+// per: block rows a warp, or part: the warps' first rows (warps + 1 of them).
 template <int BS, typename VT, class Epi>
 __global__ void __launch_bounds__(kBaijThreads, kBaijCtasPerSm)
-    k_baij_warp(uint32_t nbr, uint32_t per, const uint32_t* __restrict__ rp, const uint32_t* __restrict__ ci,
-                const VT* __restrict__ v, const double* __restrict__ x, Epi epi, const int* done)
+    k_baij_warp(uint32_t nbr, uint32_t per, const uint32_t* __restrict__ part, uint32_t warps,
+                const uint32_t* __restrict__ rp, const uint32_t* __restrict__ ci, const VT* __restrict__ v,
+                const double* __restrict__ x, Epi epi, const int* done)
 {
     if (done && *done) return;
     using Smem = BaijWarpSmem<BS, VT>;
@@ -55,10 +65,12 @@ __global__ void __launch_bounds__(kBaijThreads, kBaijCtasPerSm)
     __shared__ Smem smem[kBaijThreads / 32];
     const uint32_t lane = threadIdx.x & 31u, wid = threadIdx.x >> 5, r = lane % BS;
     Smem& s = smem[wid];
-    const uint64_t begin = (uint64_t)(blockIdx.x * (kBaijThreads / 32) + wid) * per;
-    if (begin >= nbr) return;
-    const uint32_t R1 = (uint32_t)(begin + per < nbr ? begin + per : nbr);
-    uint32_t I0 = (uint32_t)begin;  // the group's first row
+    const uint32_t w = blockIdx.x * (kBaijThreads / 32) + wid;
+    if (w >= warps) return;
+    // the group's first row, and the end of the warp's
+    uint32_t I0 = part ? __ldg(&part[w]) : w * per;
+    const uint32_t R1 = part ? __ldg(&part[w + 1]) : nbr - I0 < per ? nbr : I0 + per;
+    if (I0 >= R1) return;
     const uint32_t p0 = __ldg(&rp[I0]), p1 = __ldg(&rp[R1]);
     const uint32_t first = p0 & ~3u;  // four blocks of any size and type are whole 16-byte units
     const uint32_t passes = (p1 - first + NB - 1) / NB;
@@ -266,13 +278,12 @@ void baij_mv(b2s_ctx* ctx, const BaijDev& A, const VT* v, const double* x, Epi e
     }
     else
     {
-        // one wave of warps, the rows dealt evenly
+        // one wave of warps
         constexpr uint32_t W = kBaijThreads / 32;
-        const uint32_t warps = (uint32_t)ctx->sm_count * kBaijCtasPerSm * W;
-        const uint32_t per = (A.nbr + warps - 1) / warps;
-        const uint32_t used = (A.nbr + per - 1) / per;
-        B2S_LAUNCH(ctx, (k_baij_warp<BS, VT, Epi>), (used + W - 1) / W, kBaijThreads, 0, A.nbr, per, A.rp.p, A.ci.p,
-                   v, x, epi, done);
+        const uint32_t per = baij_even_rows(ctx, A.nbr);
+        const uint32_t warps = A.nblk ? A.nblk : (A.nbr + per - 1) / per;
+        B2S_LAUNCH(ctx, (k_baij_warp<BS, VT, Epi>), (warps + W - 1) / W, kBaijThreads, 0, A.nbr, per,
+                   A.nblk ? A.blk_row.p : (const uint32_t*)nullptr, warps, A.rp.p, A.ci.p, v, x, epi, done);
     }
 }
 

@@ -457,3 +457,27 @@ def test_persistent_wait_timeout_reported(b2s, ctx, loop):
     assert dt < 0.5, dt
     x, _ = b2s.solve(ctx, A, b, method, M, tol=1e-3, maxit=2000)
     assert np.array_equal(x, x0)
+
+
+@pytest.mark.parametrize("bs", [2, 3, 4])
+@pytest.mark.parametrize("where", ["first", "middle", "last", "hub", "hub_first"])
+def test_baij_matvec_adjacent_long_rows(b2s, ctx, orc, bs, where):
+    """Block matvec where rows dealt evenly would give a few warps most of the
+    blocks, so that they are dealt by their blocks: long rows next to one another
+    among short and empty ones, one row longer than all the rest; shares of no
+    row, of one, of many."""
+    n = 9001  # more rows than warps in a wave
+    rng = np.random.default_rng(bs)
+    lens = rng.integers(0, 4, n)
+    lens[100:400] = 0
+    at = {"first": 0, "middle": 4000, "last": n - 120}.get(where)
+    if at is None:
+        lens[0 if where == "hub_first" else n - 1] = 8000
+    else:
+        lens[at:at + 120] = rng.integers(200, 700, 120)
+    cols = [np.sort(rng.choice(n, size=int(k), replace=False)) for k in lens]
+    rp = np.concatenate([[0], np.cumsum(lens)]).astype(np.uint32)
+    ci, v = np.concatenate(cols).astype(np.uint32), rng.uniform(-1, 1, int(rp[-1]) * bs * bs)
+    x = rng.uniform(-1, 1, n * bs)
+    y = b2s.BAIJ(ctx, bs, n, n, rp, ci, v).matvec(x)
+    assert np.array_equal(y, orc.blk_matvec(orc.blk(bs, n, n, rp, ci, v), x))
