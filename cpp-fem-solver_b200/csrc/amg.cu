@@ -73,13 +73,15 @@ __global__ void k_find_diag(uint32_t nb, uint32_t per, const uint32_t* __restric
 void finish_baij(b2s_ctx* ctx, BaijDev& M)
 {
     M.diag_ptr.alloc((size_t)M.nbr + 2);
-    B2S_CUDA(cudaMemsetAsync(M.diag_ptr.p + M.nbr, 0, 2 * sizeof(uint32_t), ctx->stream));
+    uint32_t h[2] = {0, 0};
     if (M.nbr)
+    {
+        if (M.bs > 1) B2S_CUDA(cudaMemsetAsync(M.diag_ptr.p + M.nbr, 0, sizeof(uint32_t), ctx->stream));
         B2S_LAUNCH(ctx, k_find_diag, stream_grid(ctx, M.nbr), kThreads, 0, M.nbr,
                    M.bs > 1 ? baij_even_rows(ctx, M.nbr) : 0u, M.rp.p, M.ci.p, M.diag_ptr.p);
-    uint32_t h[2];
-    d2h(ctx, h, M.diag_ptr.p + M.nbr, sizeof(h));
-    sync(ctx);
+        d2h(ctx, h, M.diag_ptr.p + M.nbr, sizeof(h));
+        sync(ctx);
+    }
     M.nnzb = h[1];
     baij_partition(ctx, M, h[0]);
 }
@@ -652,8 +654,8 @@ __global__ void k_mm_unique_fill(uint32_t nr, const uint32_t* __restrict__ off, 
 // cci[crp[i]...]; Values (scalars): their sums too, every product added in A's
 // entry order -- the entries of one row of B have distinct columns, so no two
 // lanes add into one slot between two barriers -- which is the reference's order.
-// A row whose columns do not fit the table raises *overflow; the caller takes a
-// larger one.
+// A row whose columns do not fit the table raises *overflow, and the groups stop
+// after the row they are at; the caller takes a larger one.
 //
 // A row of B is as short as 3 or 4 entries (the prolongation), so a warp a row left
 // most lanes idle and cleared and searched a 512-slot table for 8 columns: 128^3,
@@ -697,6 +699,8 @@ __global__ void __launch_bounds__(kThreads) k_mm_row(uint32_t nr, const uint32_t
     for (uint32_t i0 = blockIdx.x * RPC; i0 < nr; i0 += gridDim.x * RPC)
     {
         const uint32_t i = i0 + g;
+        int stop = 0;  // looked at when the row is done
+        if constexpr (MODE == MmMode::Count) stop = *(volatile int*)overflow;
         for (uint32_t s = l; s < (uint32_t)SL; s += GL)
         {
             T.key[s] = kMmEmpty;
@@ -709,6 +713,7 @@ __global__ void __launch_bounds__(kThreads) k_mm_row(uint32_t nr, const uint32_t
         bool full = false;
         // one entry of B into the table (s: the product's term)
         auto take = [&](uint32_t j, double term) {
+            if (MODE == MmMode::Count && full) return;
             uint32_t h = (j * 2654435761u) >> SHIFT;
             for (uint32_t probes = 0;; ++probes)
             {
@@ -767,6 +772,8 @@ __global__ void __launch_bounds__(kThreads) k_mm_row(uint32_t nr, const uint32_t
 #pragma unroll
             for (int o = GL / 2; o; o >>= 1) added += __shfl_xor_sync(0xffffffffu, added, o);
             if (l == 0 && i < nr) cnt[i] = added;
+            // counts of this table size are of no use once a row has not fitted
+            if (__any_sync(0xffffffffu, stop != 0)) return;
         }
         else
         {
@@ -910,7 +917,15 @@ void mm_rows_t(b2s_ctx* ctx, const BaijDev& A, const BaijDev& B, BaijDev& C, uin
                C.v.p, overflow);
 }
 
-// tier: 32, 128, 256 or 512 slots a row; lanes a row by B's mean row length
+// tier: 32, 128, 256 or 512 slots a row; lanes a row by B's mean row length, so
+// that a row of B is about one pass of them.  Whole products, ms, at 4 / 8 / 16
+// lanes and 32 slots for rows of B of 3 entries (P of the 64^3 grid) 3.42 / 3.44 /
+// 3.64; at 8 / 16 / 32 lanes for 25 (27-point, 128 slots) 17.7 / 17.6 / 18.1, for 51
+// (a band, 128) 4.2 / 3.9 / 3.8; at 16 / 32 for 228 (512 slots) 7.8 / 5.7.  Slots
+// beyond the columns cost their clearing: 3.42 with 32 at 3 entries, 3.9 with 512.
+// A table that is too small costs little, as its counts stop at the first row that
+// does not fit: a 64^3 grid whose one long row, and the rows that refer to it, have
+// 900 columns 25 ms (66 when the counts of three sizes ran to their end).
 template <MmMode MODE>
 void mm_rows(b2s_ctx* ctx, int tier, double mean_b, const BaijDev& A, const BaijDev& B, BaijDev& C, uint32_t* cnt,
              int* overflow)

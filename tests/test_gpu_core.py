@@ -481,3 +481,21 @@ def test_baij_matvec_adjacent_long_rows(b2s, ctx, orc, bs, where):
     x = rng.uniform(-1, 1, n * bs)
     y = b2s.BAIJ(ctx, bs, n, n, rp, ci, v).matvec(x)
     assert np.array_equal(y, orc.blk_matvec(orc.blk(bs, n, n, rp, ci, v), x))
+
+
+@pytest.mark.parametrize("where", [0, 1500, 2999])
+@pytest.mark.parametrize("columns", [33, 129, 257, 513])
+def test_csr_matmul_one_wide_row(b2s, ctx, orc, where, columns):
+    """A product of which one row alone does not fit the first table sizes, first,
+    amid and last of 3,000: its counts stop the others' at whatever row they are."""
+    n = 3000
+    cols = [np.unique([i, (7 * i + 1) % n]) for i in range(n)]
+    cols[where] = np.unique(np.concatenate([[where], np.arange(columns) * (n // columns)]))
+    rp = np.concatenate([[0], np.cumsum([len(c) for c in cols])]).astype(np.uint32)
+    a = (n, n, rp, np.concatenate(cols).astype(np.uint32), b2s.uniform(columns, int(rp[-1])))
+    i = np.arange(n)
+    b = (n, n, np.arange(n + 1, dtype=np.uint32), i.astype(np.uint32), 1.0 + b2s.uniform(1, n))
+    for x, y in ((a, b), (a, a)):
+        C = b2s.CSR(ctx, *x).matmul(b2s.CSR(ctx, *y))
+        Co = orc.matmul(orc.csr(*x), orc.csr(*y)).export()
+        assert np.array_equal(C.rp, Co[0]) and np.array_equal(C.ci, Co[1]) and np.array_equal(C.v, Co[2])
