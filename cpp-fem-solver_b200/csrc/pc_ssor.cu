@@ -12,11 +12,12 @@
 // re-sorted).  The apply runs one kernel per colour per sweep, rows of one
 // colour being independent, except that the last colour takes both its sweeps
 // in one (its backward sum is empty); the gather f = P r and the scatter
-// z = P^T z2 are in those kernels.  With two colours the first one's forward value
-// is one quotient, which its readers form themselves: two launches an apply, not
-// four, and w is never stored.  PCG with SSOR to 1e-10 on the 256^2 Poisson matrix,
-// bound by its launches: 15.4 -> 13.9 ms.  An apply: 512^2 18.8 -> 12.5 us, 1400^2
-// 73.6 -> 61.7, 128^3 91 -> 82, 40^3 Q1 elements (8 colours) 108 -> 101.
+// z = P^T z2 are in those kernels.  With two colours, few rows and short ones the
+// first colour's forward value is one quotient that its readers form themselves:
+// two launches an apply, not three, and w is never stored (pays).  Bound by its
+// launches there: PCG with SSOR to 1e-10 on the 256^2 Poisson matrix 13.9 ms, 15.4
+// with a launch a colour and sweep.  An apply: 512^2 11.8 us (18.5), 1400^2 61.6
+// (72.8), 128^3 77.6 (90.9), 40^3 Q1 elements (8 colours) 101 (108).
 #include <algorithm>
 #include <cmath>
 
@@ -220,14 +221,20 @@ struct PcSSOR final : PcImpl
 {
     uint32_t n = 0, ncolor = 0;
     double omega = 1.2;
+    bool pair = false;  // two launches an apply
     std::vector<uint32_t> h_cptr, h_new_id;
     DBuf<uint32_t> perm, new_id, rp2, ci2;
     DBuf<double> v2, d2, w, z2;
 
+    // Whether the readers of the first of two colours form its values.  That saves a
+    // launch, 2 us, and costs two more gathers and a quotient an entry.  Two launches /
+    // three, us: 5-point 512^2 11.8 / 14.5, 7-point 64^3 14.4 / 16.5, 128^3 81.7 / 77.6;
+    // bipartite rows of 41 over 10,000 rows 43 / 30, of 7 over 800,000 70 / 47.
+    static bool pays(uint32_t n, uint32_t nnz) { return n <= 1u << 18 && nnz <= 7ull * n; }
+
     void apply(b2s_ctx* ctx, const double* r, double* z, const int* done) override
     {
         const double fw = omega * (2.0 - omega);
-        const bool pair = ncolor == 2;
         const auto ssor_last = pair ? k_ssor_last<true> : k_ssor_last<false>;
         const auto ssor_bwd = pair ? k_ssor_bwd<true> : k_ssor_bwd<false>;
         for (uint32_t c = 0; c < ncolor; ++c)
@@ -321,6 +328,7 @@ std::unique_ptr<PcImpl> make_pc_ssor(b2s_ctx* ctx, const CsrDev& A, const b2s_pc
     RedBlack rb;
     build_redblack(ctx, A, rb, "SSOR/red-black");
     pc->ncolor = rb.ncolor;
+    pc->pair = rb.ncolor == 2 && PcSSOR::pays(n, A.nnz);
     pc->h_cptr = std::move(rb.h_cptr);
     pc->h_new_id = std::move(rb.h_new_id);
     pc->perm = std::move(rb.perm);

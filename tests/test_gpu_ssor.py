@@ -46,6 +46,25 @@ def test_ssor_colour_counts(b2s, ctx, orc, n, links):
     assert np.array_equal(z, want) and np.array_equal(np.signbit(z), np.signbit(want))
 
 
+@pytest.mark.parametrize("n,entries", [(40, 240), (40, 241), (500, 8000), (600, 300)])
+def test_ssor_two_colours(b2s, ctx, orc, n, entries):
+    # two colours on both sides of the row length (7 n entries with the diagonal)
+    # from which the first one's values are stored and read, not formed by their readers
+    rng = np.random.default_rng(entries)
+    half, d = n // 2, np.zeros((n, n))
+    at = rng.permutation(2 * half * half)[:entries]
+    i, j = at % (half * half) // half, half + at % half
+    d[np.where(at < half * half, i, j), np.where(at < half * half, j, i)] = rng.uniform(-1, 1, entries)
+    d[np.arange(n), np.arange(n)] = rng.uniform(4, 8, n) * rng.choice([-1, 1], n)
+    row, col = np.nonzero(d)
+    assert len(row) == n + entries
+    rp = np.concatenate([[0], np.cumsum(np.bincount(row, minlength=n))]).astype(np.uint32)
+    ci, v = col.astype(np.uint32), d[row, col]
+    M = b2s.Precond(ctx, b2s.CSR(ctx, n, n, rp, ci, v), b2s.PC_SSOR)
+    r = rng.uniform(-1, 1, n)
+    assert np.array_equal(M.apply(r), orc.pc(orc.csr(n, n, rp, ci, v), "ssor", 1.2).apply(r))
+
+
 def test_ssor_bad_omega(b2s, ctx):
     n, rp, ci, v = P.poisson2d(5)
     A = b2s.CSR(ctx, n, n, rp, ci, v)
