@@ -211,6 +211,7 @@ struct CsrDev
     DBuf<uint32_t> blk_row;     // staged-SpMV row partition (nblk+1)
     uint32_t nblk = 0;
     uint32_t max_row = 0;       // longest row (nonzeros); 0 = not known
+    mutable uint32_t band = 0xFFFFFFFFu;  // largest |i - j|; all ones: not known yet
     DBuf<double> diag;          // diagonal entries (0 where missing)
     // host copy of the pattern, made on demand by the setup code that needs it
     mutable std::vector<uint32_t> h_rp, h_ci;

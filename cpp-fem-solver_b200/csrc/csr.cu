@@ -141,7 +141,7 @@ b2s_status b2s_csr_create(b2s_ctx* ctx, uint32_t n, uint32_t m, const uint32_t* 
         const uint32_t nnz = row_ptr[n];
         need(nnz == 0 || (col_idx && values), B2S_INVALID_ARG, "null col_idx / values");
         // one pass: row pointers non-decreasing, columns in range and strictly ascending
-        uint32_t max_row = 0;
+        uint32_t max_row = 0, band = 0;
         bool ok_rp = true, ok_range = true, ok_order = true;
         for (uint32_t i = 0; i < n && ok_rp; ++i)
         {
@@ -152,6 +152,8 @@ b2s_status b2s_csr_create(b2s_ctx* ctx, uint32_t n, uint32_t m, const uint32_t* 
                 break;
             }
             max_row = std::max(max_row, b - a);
+            if (b > a)  // columns ascend, or the matrix is refused
+                band = std::max({band, std::max(i, col_idx[a]) - col_idx[a], std::max(i, col_idx[b - 1]) - i});
             uint32_t prev = 0;
             for (uint32_t k = a; k < b; ++k)
             {
@@ -169,6 +171,7 @@ b2s_status b2s_csr_create(b2s_ctx* ctx, uint32_t n, uint32_t m, const uint32_t* 
         d.m = m;
         d.nnz = nnz;
         d.max_row = max_row;
+        d.band = band;
         d.rp = upload(ctx, row_ptr, (size_t)n + 1);
         // 8 elements of padding: the bulk copies of the SpMV start and end on
         // 16-byte boundaries and may read a few elements past the last nonzero

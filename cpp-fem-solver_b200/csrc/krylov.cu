@@ -529,12 +529,15 @@ static bool pcg_small(b2s_ctx* ctx, const CsrDev& A, const double* d, double* x,
     // a CTA's entries: every row at its longest
     const size_t base = (size_t)rows * 8 + (size_t)rows * A.max_row * 12 + ((size_t)rows + 1) * 4 + 12288;
     if (!coop || rows > NT * kPcgSmallRows || base > (size_t)optin) return false;
-    DBuf<uint32_t> band_d(1);
-    B2S_CUDA(cudaMemsetAsync(band_d.p, 0, sizeof(uint32_t), ctx->stream));
-    B2S_LAUNCH(ctx, k_csr_band, stream_grid(ctx, A.n), kThreads, 0, A.n, A.rp.p, A.ci.p, band_d.p);
-    uint32_t band = 0;
-    d2h(ctx, &band, band_d.p, sizeof(band));
-    sync(ctx);
+    if (A.band == 0xFFFFFFFFu)  // a device-built operator's first solve
+    {
+        DBuf<uint32_t> band_d(1);
+        B2S_CUDA(cudaMemsetAsync(band_d.p, 0, sizeof(uint32_t), ctx->stream));
+        B2S_LAUNCH(ctx, k_csr_band, stream_grid(ctx, A.n), kThreads, 0, A.n, A.rp.p, A.ci.p, band_d.p);
+        d2h(ctx, &A.band, band_d.p, sizeof(uint32_t));
+        sync(ctx);
+    }
+    const uint32_t band = A.band;
     if (2ull * band > (uint64_t)NT * kPcgSmallHalo || base + 16ull * band > (size_t)optin) return false;
     const size_t smem = base - 12288 + 16 * (size_t)band;
     const uint32_t q = (rows + NT - 1) / NT;

@@ -499,3 +499,32 @@ def test_csr_matmul_one_wide_row(b2s, ctx, orc, where, columns):
         C = b2s.CSR(ctx, *x).matmul(b2s.CSR(ctx, *y))
         Co = orc.matmul(orc.csr(*x), orc.csr(*y)).export()
         assert np.array_equal(C.rp, Co[0]) and np.array_equal(C.ci, Co[1]) and np.array_equal(C.v, Co[2])
+
+
+def test_pcg_wide_band_costs_no_launch(b2s, ctx):
+    """An operator that the one-launch loop refuses for its band (2,500 of 2,048)
+    is refused by what its handle knows: as many launches as with the loop off."""
+    n, rp, ci, v = P.diffusion3d(50, 50, 30, seed=1)
+    A, b = b2s.CSR(ctx, n, n, rp, ci, v), b2s.uniform(1, n)
+    M = b2s.Precond(ctx, A, b2s.PC_DIAG)
+    count = []
+    for k in (b2s.PERSIST_AUTO, b2s.PERSIST_OFF):
+        l0 = ctx.kernel_launches
+        b2s.solve(ctx, A, b, b2s.PCG, M, tol=1e-8, maxit=16, persistent=k)
+        count.append(ctx.kernel_launches - l0)
+    assert count[0] == count[1]
+
+
+def test_pcg_one_launch_on_a_product(b2s, ctx):
+    """A device-built operator, whose band the first solve reads: the one-launch
+    loop runs from the first solve on and gives the host-built operator's bits."""
+    n, rp, ci, v = P.poisson2d(60)
+    A = b2s.CSR(ctx, n, n, rp, ci, v)
+    C = A.matmul(A)
+    H, b = b2s.CSR(ctx, n, n, C.rp, C.ci, C.v), b2s.uniform(1, n)
+    want, _ = b2s.solve(ctx, H, b, b2s.PCG, None, tol=1e-6, maxit=200)
+    for _ in range(2):
+        l0 = ctx.kernel_launches
+        x, _ = b2s.solve(ctx, C, b, b2s.PCG, None, tol=1e-6, maxit=200)
+        assert ctx.kernel_launches - l0 < 20
+        assert np.array_equal(x, want)
