@@ -882,3 +882,52 @@ def test_schedule_of_mixed_rows(b2s, ctx, orc, pattern, route, block_route):
     assert M.sizes("trsv.route")[0] == block_route
     r = b2s.uniform(n, B.n)
     assert np.array_equal(M.apply(r), b2s.Precond(ctx, B, b2s.PC_BILU0, trsv=b2s.TRSV_LEVEL).apply(r))
+
+
+def _off_grid(n, rp, ci, v):
+    """A 2-D 5-point system with one more pair of entries, (0, 2) and (2, 0): off the
+    grid schedules, its rows still short."""
+    rows = np.repeat(np.arange(n), np.diff(rp.astype(np.int64)))
+    return (n,) + P.coo_to_csr(n, n, np.concatenate([rows, [0, 2]]), np.concatenate([ci, [2, 0]]),
+                               np.concatenate([v, [-0.01, -0.01]]))
+
+
+@pytest.mark.parametrize("precision", [0, 1])
+def test_chunk_schedule_timeout_reported(b2s, ctx, precision):
+    """The chunked schedule's waits are bounded: at one poll and no sleeps the
+    ILU(0) apply of a 400^2 system whose triangles both take the chunks gives up
+    and reports B2S_TIMEOUT; with the default bounds the bits are as before."""
+    import time
+    n, rp, ci, v = _off_grid(*b2s.gen_poisson2d(400))
+    A = b2s.CSR(ctx, n, n, rp, ci, v)
+    M = b2s.Precond(ctx, A, b2s.PC_ILU0, precision=b2s.FP32 if precision else b2s.FP64)
+    assert M.sizes("trsv.route")[:2] == (3, 3)
+    r = b2s.uniform(21, n)
+    z0 = M.apply(r)
+    ctx.set_wait_limits(1, 0)
+    try:
+        t0 = time.perf_counter()
+        with pytest.raises(RuntimeError) as e:
+            M.apply(r)
+        dt = time.perf_counter() - t0
+    finally:
+        ctx.set_wait_limits(0, 0)
+    assert e.value.status == b2s.TIMEOUT and dt < 0.5, dt
+    assert np.array_equal(M.apply(r), z0)
+
+
+@pytest.mark.parametrize("spread,rhs_lo", [(60, -40), (500, -700)])
+def test_chunk_schedule_division_bit_exact(b2s, ctx, orc, spread, rhs_lo):
+    """FP64 solves in the chunks across the binary64 range, as
+    test_grid5_division_bit_exact on the grid schedule."""
+    n, rp, ci, v = _off_grid(*P.diffusion2d(48, 70, seed=spread))
+    rng = np.random.default_rng(spread + 1)
+    d = np.exp2(rng.integers(0, spread + 1, n).astype(np.float64))
+    rows = np.repeat(np.arange(n), np.diff(rp.astype(np.int64)))
+    vs = v * d[rows] * d[ci]
+    A = b2s.CSR(ctx, n, n, rp, ci, vs)
+    r = b2s.uniform(37, n) * np.exp2(rng.integers(rhs_lo, 41, n).astype(np.float64))
+    for kind in ("ic0", "ilu0"):
+        M = b2s.Precond(ctx, A, b2s.PC_NAMES[kind])
+        assert M.sizes("trsv.route")[:2] == (3, 3)
+        assert np.array_equal(M.apply(r), orc.pc(orc.csr(n, n, rp, ci, vs), kind).apply(r)), kind
