@@ -1043,9 +1043,9 @@ struct GmMgs
     const void* kern = nullptr;
     size_t smem = 0;
 
-    GmMgs(b2s_ctx* ctx, uint64_t n, int orth)
+    GmMgs(b2s_ctx* ctx, uint64_t n, const b2s_solve_opts& o)
     {
-        if (orth != B2S_ORTH_MGS || !n) return;
+        if (o.orth != B2S_ORTH_MGS || o.persistent == 2 || !n) return;
         int coop = 0, optin = 0;
         B2S_CUDA(cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, ctx->device));
         B2S_CUDA(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, ctx->device));
@@ -1502,7 +1502,7 @@ static void run_gmres(Solve& S, const double* b, double* x, b2s_stats* stats, bo
     auto Vj = [&](int j) { return V + pn * (size_t)j; };
     auto Zj = [&](int j) { return Z + pn * (size_t)j; };
 
-    GmMgs mgs(ctx, n, S.o.orth);
+    GmMgs mgs(ctx, n, S.o);
 
     S.init_state();
     B2S_CUDA(cudaEventRecord(ctx->ev0, ctx->stream));

@@ -395,7 +395,9 @@ typedef struct b2s_solve_opts
                          0 = the whole loop in one launch, over 2-D tiles when they can be planned,
                          else over row strips; 1 = row strips only; 2 = three launches per iteration.
                          PCG without or with the diagonal preconditioner on a CSR operator that the
-                         SMs' shared memory holds: one launch, 2 = three launches per iteration */
+                         SMs' shared memory holds: one launch, 2 = three launches per iteration.
+                         GMRES with B2S_ORTH_MGS on vectors that the SMs' registers hold: a column's
+                         Gram-Schmidt in one launch, 2 = a launch a step (the same bits) */
 } b2s_solve_opts;
 
 void b2s_solve_opts_default(b2s_solve_opts* opts);

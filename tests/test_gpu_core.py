@@ -528,3 +528,25 @@ def test_pcg_one_launch_on_a_product(b2s, ctx):
         x, _ = b2s.solve(ctx, C, b, b2s.PCG, None, tol=1e-6, maxit=200)
         assert ctx.kernel_launches - l0 < 20
         assert np.array_equal(x, want)
+
+
+@pytest.mark.parametrize("n", [1, 256, 257, 37889, 60001, 100003, 151553, 200001, 303105, 700001, 1000003, 1300001,
+                               1700001, 1818624, 1818625])
+def test_gmres_column_launch_bits(b2s, ctx, n):
+    """The one-launch Gram-Schmidt column against a launch a step, bit for bit, over
+    one to eight blocks a CTA (37,888 rows a block count on 148 SMs) and one to six
+    elements a thread of each (303,104 rows), with odd remainders; one row more
+    than the SMs hold keeps the launch a step."""
+    rp = np.concatenate([[0], np.cumsum(np.full(n, 3) - (np.arange(n) == 0) - (np.arange(n) == n - 1))]).astype(np.uint32)
+    i = np.arange(n)
+    cols = i[:, None] + np.array([-1, 0, 1])
+    keep = (cols >= 0) & (cols < n)
+    v = np.where(cols == i[:, None], 2.5 + b2s.uniform(1, n)[:, None], np.array([-1.0, 0.0, -0.5]))[keep]
+    A, b = b2s.CSR(ctx, n, n, rp, cols[keep].astype(np.uint32), v), b2s.uniform(2, n)
+    got = []
+    for k in (b2s.PERSIST_AUTO, b2s.PERSIST_OFF):
+        l0 = ctx.kernel_launches
+        x, st = b2s.solve(ctx, A, b, b2s.GMRES, None, tol=1e-14, maxit=9, restart=6, persistent=k)
+        got.append((x, st["it"], st["relres"], ctx.kernel_launches - l0))
+    assert np.array_equal(got[0][0], got[1][0]) and got[0][1:3] == got[1][1:3]
+    assert got[0][3] < got[1][3] if n < 1818625 else got[0][3] == got[1][3]
