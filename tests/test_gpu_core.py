@@ -550,3 +550,48 @@ def test_gmres_column_launch_bits(b2s, ctx, n):
         got.append((x, st["it"], st["relres"], ctx.kernel_launches - l0))
     assert np.array_equal(got[0][0], got[1][0]) and got[0][1:3] == got[1][1:3]
     assert got[0][3] < got[1][3] if n < 1818625 else got[0][3] == got[1][3]
+
+
+@pytest.mark.parametrize("pc", ["none", "diag"])
+@pytest.mark.parametrize("nx,ny,one", [(300, 300, True), (400, 333, True), (512, 512, True), (551, 550, True),
+                                       (2048, 61, True), (2049, 61, False), (552, 552, False)])
+def test_pcg_one_launch_rows_and_band(b2s, ctx, pc, nx, ny, one):
+    """The one-launch PCG loop against the launch-by-launch one with two and four
+    rows a thread (609 to 2,048 rows a CTA) and at both sides of its limits, a
+    band of 2,048 and 2,048 rows a CTA.  The two differ by the association of the
+    dots, some 1e-15 of them an iteration, which 40 iterations of these operators
+    (conditions of 1e5 and below) cannot raise past 1e-9 of the iterate."""
+    i = np.arange(nx * ny)
+    n, rng = nx * ny, np.random.default_rng(nx)
+    x_, y_ = i % nx, i // nx
+    cx, cy = rng.uniform(0.5, 2.0, n), rng.uniform(0.5, 2.0, n)  # of (i, i + 1) and (i, i + nx)
+    w, e = np.where(x_ > 0, np.roll(cx, 1), 0.0), np.where(x_ < nx - 1, cx, 0.0)
+    s, t = np.where(y_ > 0, np.roll(cy, nx), 0.0), np.where(y_ < ny - 1, cy, 0.0)
+    cols = i[:, None] + np.array([-nx, -1, 0, 1, nx])
+    vals = np.stack([-s, -w, w + e + s + t + 0.1, -e, -t], 1)
+    keep = vals != 0
+    rp = np.concatenate([[0], np.cumsum(keep.sum(1))]).astype(np.uint32)
+    A, b = b2s.CSR(ctx, n, n, rp, cols[keep].astype(np.uint32), vals[keep]), b2s.uniform(nx, n)
+    M = b2s.Precond(ctx, A, b2s.PC_DIAG) if pc == "diag" else None
+    got = []
+    for k in (b2s.PERSIST_AUTO, b2s.PERSIST_OFF):
+        l0 = ctx.kernel_launches
+        x, st = b2s.solve(ctx, A, b, b2s.PCG, M, tol=1e-12, maxit=40, persistent=k)
+        got.append((x, st, ctx.kernel_launches - l0))
+    (x, st, l), (xr, sr, lr) = got
+    assert (l < 20 < lr) if one else l == lr
+    assert st["iterations"] == sr["iterations"] == 40
+    assert np.linalg.norm(x - xr) <= 1e-9 * np.linalg.norm(xr)
+
+
+@pytest.mark.parametrize("method", [0, 1])
+def test_graph_replay_matches_eager(b2s, ctx, method):
+    """Iterations captured and replayed against launched ones, for PCG with its
+    one-launch loop off and for BiCGSTAB: the same bits."""
+    n, rp, ci, v = P.poisson2d(40)
+    A, b = b2s.CSR(ctx, n, n, rp, ci, v), b2s.uniform(9, n)
+    M = b2s.Precond(ctx, A, b2s.PC_DIAG)
+    o = dict(tol=1e-8, persistent=b2s.PERSIST_OFF)
+    x1, s1 = b2s.solve(ctx, A, b, method, M, use_graphs=1, check_every=8, **o)
+    x2, s2 = b2s.solve(ctx, A, b, method, M, use_graphs=0, check_every=3, **o)
+    assert s1["it"] > 8 and s1["it"] == s2["it"] and np.array_equal(x1, x2)
