@@ -223,7 +223,8 @@ __global__ void __launch_bounds__(kThreads, 6)
     const uint32_t p0 = __ldg(&rp[r0]), p1 = __ldg(&rp[r1]);
     const uint32_t a = own ? __ldg(&rp[row]) : 0u, b = own ? __ldg(&rp[row + 1]) : 0u;
     double sum = 0.0;
-    for (uint32_t base = p0, end; base < p1; base = end)  // one pass, unless a single row is longer
+    // one pass of a CTA whose rows are of about the mean length, more where they are longer
+    for (uint32_t base = p0, end; base < p1; base = end)
     {
         end = p1 - base < kBaijStagedCap ? p1 : base + kBaijStagedCap;
         VT vv[U];

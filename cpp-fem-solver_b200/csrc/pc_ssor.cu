@@ -171,6 +171,15 @@ __device__ __forceinline__ double ssor_first(uint32_t j, const double* __restric
     return fw * r[perm[j]] / d2[j];
 }
 
+// the first colour's forward values, where they are stored
+__global__ void k_ssor_first(uint32_t hi, const double* __restrict__ d2, const uint32_t* __restrict__ perm,
+                             const double* __restrict__ r, double* __restrict__ w, double fw, const int* done)
+{
+    if (done && *done) return;
+    for (uint32_t ii = blockIdx.x * blockDim.x + threadIdx.x; ii < hi; ii += gridDim.x * blockDim.x)
+        w[ii] = ssor_first(ii, d2, perm, r, fw);
+}
+
 // the last colour: forward, then backward with no later row.  PAIR: of two
 // colours, so that the rows before are all of the first one.
 template <bool PAIR>
@@ -243,6 +252,8 @@ struct PcSSOR final : PcImpl
             if (c + 1 == ncolor)
                 B2S_LAUNCH(ctx, ssor_last, stream_grid(ctx, hi - lo), kThreads, 0, lo, hi,
                            rp2.p, ci2.p, v2.p, d2.p, perm.p, r, w.p, z2.p, z, omega, fw, done);
+            else if (c == 0 && !pair)
+                B2S_LAUNCH(ctx, k_ssor_first, stream_grid(ctx, hi), kThreads, 0, hi, d2.p, perm.p, r, w.p, fw, done);
             else if (!pair)
                 B2S_LAUNCH(ctx, k_ssor_fwd, stream_grid(ctx, hi - lo), kThreads, 0, lo, hi, rp2.p, ci2.p, v2.p, d2.p,
                            perm.p, r, w.p, omega, fw, done);

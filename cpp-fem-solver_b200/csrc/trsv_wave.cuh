@@ -121,7 +121,6 @@ __global__ void __launch_bounds__(wave_threads(GL)) k_trsv_wave(WaveArgs a, cons
     [[maybe_unused]] XT rc = XT(1);
     if constexpr (DIAG == WaveDiag::Divide) rc = (XT)(1.0 / (double)dv[0]);
 
-    unsigned limit = a.polls_max;
     for (uint32_t p0 = 0; __any_sync(0xffffffffu, pa + p0 < pe); p0 += GL)
     {
         const uint32_t p = pa + p0 + q;
@@ -156,10 +155,9 @@ __global__ void __launch_bounds__(wave_threads(GL)) k_trsv_wave(WaveArgs a, cons
             if (__all_sync(0xffffffffu, fresh)) break;
             // the error word by a vote, so that the warp leaves as one: a lane's own
             // load may come before or after another's
-            if (polls + 1 >= limit || ((polls & 1023u) == 1023u && __any_sync(0xffffffffu, ld_err(a.err) != 0)))
+            if (polls + 1 >= a.polls_max || ((polls & 1023u) == 1023u && __any_sync(0xffffffffu, ld_err(a.err) != 0)))
             {
                 if (lane == 0) atomicCAS(a.err, 0, (int)B2S_TIMEOUT);
-                limit = 1;  // the row's later passes read once
                 break;
             }
             next = __reduce_min_sync(0xffffffffu, fresh ? 0xffffffffu : lev);
