@@ -193,6 +193,7 @@ void check_device_error(b2s_ctx* ctx, const char* where);
 // Polls of one wait of the kernels that never sleep (grid schedules, level-order
 // traversal, sums over a persistent kernel's grid) before it gives up
 // (B2S_TIMEOUT): the context's wait bounds, spin and sleep budgets together.
+constexpr unsigned kGridPolls = 1u << 21;  // by the default bounds
 inline unsigned grid_polls(const b2s_ctx* ctx)
 {
     const uint64_t p = (uint64_t)ctx->wait_fast_polls + ctx->wait_slow_polls;

@@ -10,7 +10,9 @@
 // alternate: a CTA writes a set again only after a sum over the other one, which
 // every CTA took part in after it had read this one.  A wait ends after polls_max
 // polls (grid_polls: the context's wait limits): the CTA records B2S_TIMEOUT and
-// leaves, the others give up at their next sum, and the launch ends.
+// leaves, the others give up at their next sum, and the launch ends.  A kernel
+// that sums all the time has an instance of its own for the default bound: one
+// that is not a constant cost the tiled PCG 8 % and the one-launch PCG 1 %.
 //
 // It costs two trips through L2 and their spread over the SMs, about 2 us on 148
 // CTAs.  A line for every pair of CTAs instead of one polled by all was no faster

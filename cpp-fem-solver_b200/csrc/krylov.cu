@@ -331,9 +331,10 @@ __global__ void __launch_bounds__(kThreads) k_csr_band(uint32_t n, const uint32_
     if ((threadIdx.x & 31u) == 0 && b) atomicMax(band, b);
 }
 
-template <int Q>
+template <int Q, bool LIMITED>
 __global__ void __launch_bounds__(kPcgSmallThreads, 1) k_pcg_small(PcgSmallArgs a)
 {
+    const unsigned polls_max = LIMITED ? a.polls_max : kGridPolls;
     constexpr uint32_t NT = kPcgSmallThreads;
     constexpr int HQ = kPcgSmallHalo;
     extern __shared__ __align__(16) double pcg_sm[];
@@ -419,7 +420,7 @@ __global__ void __launch_bounds__(kPcgSmallThreads, 1) k_pcg_small(PcgSmallArgs 
         }
         ++epoch;
         grid_sum_post(gs, a.lines, epoch, one);
-        if (!grid_sum_wait(gs, a.lines, epoch, pAp, a.err, a.polls_max)) break;
+        if (!grid_sum_wait(gs, a.lines, epoch, pAp, a.err, polls_max)) break;
         if (!(pAp[0] >= kBreak))  // breakdown, not SPD or NaN: the state's own test decides
         {
             __syncthreads();
@@ -464,7 +465,7 @@ __global__ void __launch_bounds__(kPcgSmallThreads, 1) k_pcg_small(PcgSmallArgs 
             {
                 unsigned long long wl = 0, wh = 0;
                 bool seen = false;
-                for (unsigned polls = 0; polls < a.polls_max && !seen; ++polls)
+                for (unsigned polls = 0; polls < polls_max && !seen; ++polls)
                 {
                     asm volatile("ld.relaxed.gpu.global.v2.u64 {%0, %1}, [%2];"
                                  : "=l"(wl), "=l"(wh)
@@ -479,7 +480,7 @@ __global__ void __launch_bounds__(kPcgSmallThreads, 1) k_pcg_small(PcgSmallArgs 
                 }
                 zh[k] = __longlong_as_double((long long)((wh << 32) | (wl & 0xffffffffull)));
             }
-        if (!grid_sum_wait(gs, a.lines + grid_sum_words(gridDim.x), epoch, tot, a.err, a.polls_max)) break;
+        if (!grid_sum_wait(gs, a.lines + grid_sum_words(gridDim.x), epoch, tot, a.err, polls_max)) break;
         rr = tot[0];
         if (tot[0] > clear && tot[0] < HUGE_VAL && tot[1] > 0.0 && it + 1 < maxit)
         {
@@ -541,7 +542,11 @@ static bool pcg_small(b2s_ctx* ctx, const CsrDev& A, const double* d, double* x,
     if (2ull * band > (uint64_t)NT * kPcgSmallHalo || base + 16ull * band > (size_t)optin) return false;
     const size_t smem = base - 12288 + 16 * (size_t)band;
     const uint32_t q = (rows + NT - 1) / NT;
-    const void* kern = q <= 1 ? (const void*)k_pcg_small<1> : q == 2 ? (const void*)k_pcg_small<2> : (const void*)k_pcg_small<4>;
+    const bool limited = grid_polls(ctx) != kGridPolls;
+    const void* const kerns[3][2] = {{(const void*)k_pcg_small<1, false>, (const void*)k_pcg_small<1, true>},
+                                     {(const void*)k_pcg_small<2, false>, (const void*)k_pcg_small<2, true>},
+                                     {(const void*)k_pcg_small<4, false>, (const void*)k_pcg_small<4, true>}};
+    const void* kern = kerns[q <= 1 ? 0 : q == 2 ? 1 : 2][limited];
     B2S_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     int occ = 0;
     B2S_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kern, NT, smem));
@@ -947,12 +952,13 @@ struct GmMgsArgs
     unsigned long long* lines;
     uint32_t epoch;  // the first sum's
     int* err;
-    unsigned polls_max;  // of one wait
 };
 
-// S: blocks a thread belongs to, K: elements it has in each
+// S: blocks a thread belongs to, K: elements it has in each.  polls_max, of one
+// wait, is no member of a: with one more the compiler keeps the elements' places
+// in fewer registers and forms them again (96^3 GMRES(30) 6.65 ms for 6.5).
 template <int S, int K>
-__global__ void __launch_bounds__(kMgsThreads, 1) k_gm_mgs(GmMgsArgs a, const int* skip)
+__global__ void __launch_bounds__(kMgsThreads, 1) k_gm_mgs(GmMgsArgs a, const int* skip, unsigned polls_max)
 {
     if (*skip) return;
     extern __shared__ __align__(16) double mgs_sm[];  // two sets of V's elements
@@ -1005,7 +1011,7 @@ __global__ void __launch_bounds__(kMgsThreads, 1) k_gm_mgs(GmMgsArgs a, const in
 #pragma unroll
         for (int q = 0; q < S * K; ++q)
             if (at(q / K, q % K) < a.n) acc[q / K] += w[q] * v[q * kMgsThreads];
-        if (!block_sum(bs, a.lines, epoch++, a.blocks, a.vb, acc, h, a.err, a.polls_max)) return gave_up();
+        if (!block_sum(bs, a.lines, epoch++, a.blocks, a.vb, acc, h, a.err, polls_max)) return gave_up();
         if (blockIdx.x == 0 && threadIdx.x == 0) a.sm.H[(size_t)i * a.sm.m + a.j] = h;
 #pragma unroll
         for (int q = 0; q < S * K; ++q)
@@ -1018,7 +1024,7 @@ __global__ void __launch_bounds__(kMgsThreads, 1) k_gm_mgs(GmMgsArgs a, const in
 #pragma unroll
     for (int q = 0; q < S * K; ++q)
         if (at(q / K, q % K) < a.n) acc[q / K] += w[q] * w[q];
-    if (!block_sum(bs, a.lines, epoch, a.blocks, a.vb, acc, ww, a.err, a.polls_max)) return gave_up();
+    if (!block_sum(bs, a.lines, epoch, a.blocks, a.vb, acc, ww, a.err, polls_max)) return gave_up();
     const double hn = sqrt(ww);  // gm_column_tail's H[j+1][j]
     if (hn > kBreak)
     {
@@ -1073,9 +1079,10 @@ struct GmMgs
     void run(b2s_ctx* ctx, uint64_t n, uint64_t pn, const double* w, double* V, KState* st, const GmSmall& sm, int j,
              const int* skip)
     {
-        GmMgsArgs a{n, pn, blocks, vb, w, V, st, sm, j, lines.p, epoch, ctx->errword(), grid_polls(ctx)};
+        GmMgsArgs a{n, pn, blocks, vb, w, V, st, sm, j, lines.p, epoch, ctx->errword()};
+        unsigned polls = grid_polls(ctx);
         epoch += (uint32_t)j + 2u;
-        void* params[] = {&a, &skip};
+        void* params[] = {&a, &skip, &polls};
         B2S_CUDA(cudaLaunchCooperativeKernel(kern, dim3(ctas), dim3(kMgsThreads), params, smem, ctx->stream));
         note_launch(ctx, "k_gm_mgs");
     }

@@ -993,11 +993,12 @@ struct PcIC0 final : PcImpl
     template <uint32_t Q, bool FUSED>
     bool launch_tiles(b2s_ctx* ctx, PcgTileArgs& a)
     {
-        B2S_CUDA(cudaFuncSetAttribute(k_pcg_tile<Q, FUSED>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                      (int)tile_smem));
+        const void* kern = a.polls_max == kGridPolls ? (const void*)k_pcg_tile<Q, FUSED, false>
+                                                     : (const void*)k_pcg_tile<Q, FUSED, true>;
+        B2S_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tile_smem));
         void* params[] = {&a};
-        const cudaError_t e = cudaLaunchCooperativeKernel((const void*)k_pcg_tile<Q, FUSED>, dim3(tile_count),
-                                                          dim3(kTileThreads), params, tile_smem, ctx->stream);
+        const cudaError_t e =
+            cudaLaunchCooperativeKernel(kern, dim3(tile_count), dim3(kTileThreads), params, tile_smem, ctx->stream);
         if (e == cudaErrorCooperativeLaunchTooLarge || e == cudaErrorNotSupported)
         {
             cudaGetLastError();

@@ -56,7 +56,7 @@ struct PcgTileArgs
     unsigned long long* lines;      // two regions of grid_sum_words, zero at launch
     KState* st;
     int* err;
-    unsigned polls_max;  // of one wait
+    unsigned polls_max;  // of one wait, where the context's bounds are not the default
     int stall_window;
 };
 
@@ -163,9 +163,11 @@ __device__ __forceinline__ uint32_t tile_dep_slots(uint32_t w, uint32_t dummy)
     return (d0 == kTileNoDep ? dummy : d0) | ((d1 == kTileNoDep ? dummy : d1) << 16);
 }
 
-template <uint32_t Q, bool FUSED>
+// LIMITED: waits of a.polls_max polls, not of the default number
+template <uint32_t Q, bool FUSED, bool LIMITED>
 __global__ void __launch_bounds__(kTileThreads, 1) k_pcg_tile(PcgTileArgs a)
 {
+    const unsigned polls_max = LIMITED ? a.polls_max : kGridPolls;
     constexpr uint32_t NT = kTileThreads;
     extern __shared__ __align__(16) unsigned char smem[];
     __shared__ KState sst;
@@ -291,7 +293,7 @@ __global__ void __launch_bounds__(kTileThreads, 1) k_pcg_tile(PcgTileArgs a)
             }
             for (uint32_t t = tid + NT; t < n_ring; t += NT)
             {
-                const float zt = epoch ? tile_await<float>(&a.zw[ahalo[t]], epoch, &gs.failed, a.err, a.polls_max) : (float)a.z[ahalo[t]];
+                const float zt = epoch ? tile_await<float>(&a.zw[ahalo[t]], epoch, &gs.failed, a.err, polls_max) : (float)a.z[ahalo[t]];
                 pe[n_own + t] = pl[t] = (double)zt + beta * pl[t];
             }
             ++epoch;
@@ -318,9 +320,9 @@ __global__ void __launch_bounds__(kTileThreads, 1) k_pcg_tile(PcgTileArgs a)
             {
                 const uint32_t t = tid + NT * q;
                 if (t >= n_own && t < n_el)
-                    Apv[q] = tile_await<double>(&a.apw[2 * (size_t)lower_row(t)], epoch, &gs.failed, a.err, a.polls_max);
+                    Apv[q] = tile_await<double>(&a.apw[2 * (size_t)lower_row(t)], epoch, &gs.failed, a.err, polls_max);
             }
-            if (!grid_sum_wait(gs, lines1, epoch, tot, a.err, a.polls_max)) break;
+            if (!grid_sum_wait(gs, lines1, epoch, tot, a.err, polls_max)) break;
             if (tid == 0) pcg_alpha(&sst, tot[0]);
             __syncthreads();
             if (sst.done) break;
@@ -377,7 +379,7 @@ __global__ void __launch_bounds__(kTileThreads, 1) k_pcg_tile(PcgTileArgs a)
                     rr[q] = in ? yf[t] : 0.f;
                 else
                     rr[q] = t < n_own ? yf[t]
-                            : in      ? tile_await<float>(&a.yw[uhalo[t - n_own]], epoch, &gs.failed, a.err, a.polls_max)
+                            : in      ? tile_await<float>(&a.yw[uhalo[t - n_own]], epoch, &gs.failed, a.err, polls_max)
                                       : 0.f;
             }
             const float* yk = tile_sweeps<Q>(a.k, s_ucnt, dep, val, di, rr, y0, y1, dummy);
@@ -394,8 +396,8 @@ __global__ void __launch_bounds__(kTileThreads, 1) k_pcg_tile(PcgTileArgs a)
                 }
             }
             grid_sum_post(gs, lines2, epoch, acc);
-            if (tid < n_ring) zh = tile_await<float>(&a.zw[ahalo[tid]], epoch, &gs.failed, a.err, a.polls_max);
-            if (!grid_sum_wait(gs, lines2, epoch, tot, a.err, a.polls_max)) break;
+            if (tid < n_ring) zh = tile_await<float>(&a.zw[ahalo[tid]], epoch, &gs.failed, a.err, polls_max);
+            if (!grid_sum_wait(gs, lines2, epoch, tot, a.err, polls_max)) break;
             if (tid == 0)
             {
                 converge(tot[0]);
