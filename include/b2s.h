@@ -216,9 +216,9 @@ typedef enum b2s_trsv
                               reciprocal, rounded once from FP64 (and AUTO divides in a triangle with a row
                               too long for a chunk, 15,000 entries and more); FP64 is the same in all */
     B2S_TRSV_CHUNK = 3,    /* one launch (the AUTO choice): row chunks staged in shared memory, local
-                              levels split by barriers, bounded flags between chunks; triangles with
-                              wide rows or many rows a level take SYNCFREE's traversal instead, and
-                              5- / 7-point grid factors their grid schedules */
+                              levels split by barriers, bounded flags between chunks; triangles mostly
+                              of wide rows, or with many rows a level, take SYNCFREE's traversal
+                              instead, and 5- / 7-point grid factors their grid schedules */
     B2S_TRSV_JACOBI = 4    /* inexact: rows grouped into segments of trsv_segment consecutive rows;
                               each segment solved on its own, then trsv_sweeps block-Jacobi sweeps
                               (Gauss-Seidel inside a segment, the previous sweep's values outside);
