@@ -2,9 +2,8 @@
 // ILU(0)): every row of the factor in level order, each waiting for the values
 // it reads.
 //
-// Rows are dealt to lane groups in (level, index) order: GL lanes (4, 8, 16 or 32:
-// the smallest that holds the widest row, longer rows take several passes) own
-// one row, lane q its q-th entry.  A group loads everything that is fixed --
+// Rows are dealt to lane groups in (level, index) order: GL lanes (4, 8, 16 or 32,
+// wave_lanes; longer rows take several passes) own one row, lane q its q-th entry.  A group loads everything that is fixed --
 // its entry's column, coefficients, right-hand side, divisor -- and then polls
 // the rows it depends on in the exchange array, where a finished row leaves its
 // value as 64-bit words {epoch, 32 value bits}: one word per FP32 component, two
@@ -232,6 +231,29 @@ __global__ void __launch_bounds__(wave_threads(GL)) k_trsv_wave(WaveArgs a, cons
     }
 }
 
+// Lanes a row.  More of them take a level's widest row in fewer passes, 0.7 us
+// each, but every row has as many, and 20,000 lanes cost as much as a pass (FP64,
+// rows of 3 entries, an apply's wider triangle: 262,144 rows at 4 / 8 / 16 / 32
+// lanes 41 / 66 / 149 / 283 us).  By the widest row alone, one row of 40 entries in a
+// red-black 1,000^2 system had all rows take 32 lanes: 1,248 us an apply, 214 now
+// (chunked 369); one of 2,000 in a 512^2 one 364 and 251 (354).
+inline uint32_t wave_lanes(uint32_t n, const std::vector<uint32_t>& width)
+{
+    uint32_t best = 4;
+    uint64_t cost = ~0ull;
+    for (uint32_t gl = 4; gl <= 32; gl *= 2)
+    {
+        uint64_t c = (uint64_t)n * gl / 20000;
+        for (uint32_t w : width) c += std::max(1u, (w + gl - 1) / gl);
+        if (c < cost)
+        {
+            cost = c;
+            best = gl;
+        }
+    }
+    return best;
+}
+
 // One triangle's level-order schedule.
 struct WaveSchedule
 {
@@ -246,13 +268,11 @@ struct WaveSchedule
         n = (uint32_t)level.size();
         bs = block;
         if (!n) return;
-        uint32_t widest = 0, top = 0;
-        for (uint32_t i = 0; i < n; ++i)
-        {
-            widest = std::max(widest, rp[i + 1] - rp[i]);
-            top = std::max(top, level[i]);
-        }
-        gl = widest <= 4 ? 4 : widest <= 8 ? 8 : widest <= 16 ? 16 : 32;
+        uint32_t top = 0;
+        for (uint32_t l : level) top = std::max(top, l);
+        std::vector<uint32_t> width(top + 1, 0);  // each level's widest row
+        for (uint32_t i = 0; i < n; ++i) width[level[i]] = std::max(width[level[i]], rp[i + 1] - rp[i]);
+        gl = wave_lanes(n, width);
         const uint32_t rw = 32 / gl;
         std::vector<uint32_t> at(top + 2, 0);
         for (uint32_t l : level) ++at[l + 1];

@@ -931,3 +931,40 @@ def test_chunk_schedule_division_bit_exact(b2s, ctx, orc, spread, rhs_lo):
         M = b2s.Precond(ctx, A, b2s.PC_NAMES[kind])
         assert M.sizes("trsv.route")[:2] == (3, 3)
         assert np.array_equal(M.apply(r), orc.pc(orc.csr(n, n, rp, ci, vs), kind).apply(r)), kind
+
+
+@pytest.mark.parametrize("entries", [40, 200, 2000])
+def test_level_order_traversal_long_rows(b2s, ctx, orc, entries):
+    """Two or three levels of very many short rows, and rows of 40, 200 or 2,000
+    entries among the last: the traversal takes 4, 8 or 16 lanes a row, so the long
+    rows take many passes.  Red-black 300^2 system; the FP64 applies equal the
+    restatement bit for bit, the FP32 ones are within 1e-5 of them, the block ones
+    (2x2) equal those of the level-by-level solve bit for bit."""
+    N, rng = 300, np.random.default_rng(entries)
+    n, i = N * N, np.arange(N * N)
+    x, y = i % N, i // N
+    order = np.argsort((x + y) % 2, kind="stable")
+    new = np.empty(n, np.int64)
+    new[order] = i
+    lo = np.concatenate([np.stack([i[x > 0], i[x > 0] - 1], 1), np.stack([i[y > 0], i[y > 0] - N], 1)])
+    lo = np.sort(new[lo], 1)[:, ::-1]
+    hubs = np.concatenate([np.stack([np.full(entries, n - 1 - 7 * k),
+                                     rng.choice(n // 4, size=entries, replace=False)], 1) for k in range(3)])
+    lo = np.unique(np.concatenate([lo, hubs]), axis=0)
+    a = -rng.uniform(0.1, 1.0, len(lo))
+    deg = np.bincount(lo.ravel(), minlength=n)
+    rp, ci, v = P.coo_to_csr(n, n, np.concatenate([lo[:, 0], lo[:, 1], i]), np.concatenate([lo[:, 1], lo[:, 0], i]),
+                             np.concatenate([a, a, deg + 1.0]))
+    A, r = b2s.CSR(ctx, n, n, rp, ci, v), b2s.uniform(n, n)
+    for kind in ("ic0", "ilu0"):
+        k = b2s.PC_NAMES[kind]
+        M = b2s.Precond(ctx, A, k)
+        assert M.sizes("trsv.route")[0] == 2
+        z = M.apply(r)
+        assert np.array_equal(z, orc.pc(orc.csr(n, n, rp, ci, v), kind).apply(r)), kind
+        assert rel(b2s.Precond(ctx, A, k, precision=b2s.FP32).apply(r), z) < 1e-5
+    B = b2s.BAIJ(ctx, 2, n, n, rp, ci, (v[:, None, None] * np.array([[1.0, 0.1], [-0.2, 1.1]])).ravel())
+    r = b2s.uniform(n, B.n)
+    M = b2s.Precond(ctx, B, b2s.PC_BILU0)
+    assert M.sizes("trsv.route")[0] == 2
+    assert np.array_equal(M.apply(r), b2s.Precond(ctx, B, b2s.PC_BILU0, trsv=b2s.TRSV_LEVEL).apply(r))
